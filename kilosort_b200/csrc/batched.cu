@@ -3,7 +3,7 @@
 // Per call:
 //   per recording   template energy nm, {nm, 1/nm} pairs, U reordered to
 //                   [Kpad][Q] (bf16 hi/lo, or f32)
-//   per batch       Xres <- X; temporal projection into the recording's
+//   per batch       temporal projection into the recording's
 //                   stacked Y (split-BF16) or a shared Y buffer (FP32)
 //   contraction     split-BF16: ONE grouped tcgen05 launch over the tiles of
 //                   every batch of every recording (tensor maps per recording,
@@ -15,7 +15,7 @@
 //                   longest-first order with team-wide barriers; every loop ends
 //                   on the device (no host round trip between iterations or
 //                   batches)
-//   residual        ONE launch over (batch, block, 32 channels)
+//                   and writes each batch's residual from X after its peel
 // Nothing is copied from host memory and nothing synchronises the host, so the
 // sequence can be captured in a CUDA graph and replayed.
 #include "peel_core.cuh"
@@ -41,6 +41,7 @@ struct MultiRec {
   const int* rperm;             // group order of the grouped update
   const float* mg;              // its product bounds [K][ng]
   const float2* nmip;           // {nm, 1/nm} in group order
+  const unsigned long long* sup;  // support masks
   int C, K, P, nt;
   float th2;
   int max_peels;
@@ -49,6 +50,7 @@ struct MultiRec {
 
 struct MultiBatch {
   float* Bt;
+  const float* X;
   float* Xres;
   long long* st;
   float* amps;
@@ -77,6 +79,7 @@ __device__ void fill_args(const MultiParams& p, int b, char* team, PeelArgs& a) 
   const MultiRec& r = p.recs[mb.rec];
   a = PeelArgs{};
   a.Bt = mb.Bt;
+  a.X = mb.X;
   a.Xres = mb.Xres;
   a.U = r.U;
   a.W = r.W;
@@ -99,6 +102,7 @@ __device__ void fill_args(const MultiParams& p, int b, char* team, PeelArgs& a) 
   a.rperm = r.rperm;
   a.mg = r.mg;
   a.nmip = r.nmip;
+  a.sup = r.sup;
   a.limit_ns = p.limit_ns;
   a.upstream_err = p.upstream_err;
 #ifdef KS_PEEL_TRACE
@@ -110,8 +114,8 @@ __device__ void fill_args(const MultiParams& p, int b, char* team, PeelArgs& a) 
 // team's barrier count carries over from batch to batch.  After a batch's
 // peel the same team applies its residual pass (record order per element, as
 // ks_residual_kernel does), so one team's residual work fills the barrier
-// waits of the others.  A team stops at its first error (info of its later
-// batches keeps the "not run" value).
+// waits of the others.  A team peels nothing after its first error (info of
+// its later batches keeps the "not run" value, their Xres is X).
 template <int kRows, bool kLean>
 __device__ __forceinline__ void peel_multi_body(const MultiParams& p, char* smem_raw,
                                                 PeelArgs& sa);
@@ -155,32 +159,25 @@ __device__ __forceinline__ void peel_multi_body(const MultiParams& p, char* smem
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   char* tbase = p.teams + (size_t)team * p.team_bytes;
   unsigned epoch = 0;
+  bool failed = false;
   for (int i = team; i < p.n_batches; i += n_teams) {
     __syncthreads();
     if (threadIdx.x == 0) fill_args(p, p.order[i], tbase, sa);
     __syncthreads();
     const Smem s = carve_smem(sa, smem_raw, true);
-    const PeelOutcome o = run_peel<kRows, true, kLean>(sa, s, rank, (unsigned)p.team_size, epoch);
-    if (o.status != KS_OK) {
-      if (o.status == KS_ERR_OVERFLOW) continue;   // that batch only
-      break;
+    PeelOutcome o{0, 0, KS_OK};
+    if (!failed) {
+      o = run_peel<kRows, true, kLean>(sa, s, rank, (unsigned)p.team_size, epoch);
+      failed = o.status != KS_OK && o.status != KS_ERR_OVERFLOW;   // overflow: that batch only
     }
-    if (o.n_out > 0) {
-      // the residual's per-warp lists and transpose tiles use the update's
-      // stage tiles, which the peel of this batch no longer needs
-      int* xl = reinterpret_cast<int*>(s.stage);
-      ResSmem rs;
-      rs.W = s.W;
-      rs.xl_tau = xl;
-      rs.xl_k = xl + kWarps * kXList;
-      rs.xl_amp = reinterpret_cast<float*>(xl + 2 * kWarps * kXList);
-      rs.xt = reinterpret_cast<float*>(xl + 3 * kWarps * kXList);
-      const int xg = (sa.C + 31) / 32;
-      const long long n_items = (long long)sa.nblk * xg;
-      for (long long w = (long long)rank * kWarps + warp; w < n_items;
-           w += (long long)p.team_size * kWarps)
-        residual_item<true>(sa, rs, o.iters, o.n_out, (int)(w / xg), (int)(w % xg), lane, warp);
-    }
+    const bool good = !failed && o.status == KS_OK;
+    if (sa.X == sa.Xres && (!good || o.n_out == 0)) continue;
+    // the residual's scratch uses the update's stage tiles, which the peel of
+    // this batch no longer needs; a batch without a result gets Xres = X
+    __syncthreads();
+    const ResSmem rs = residual_smem(s.W, s.stage, warp);
+    residual_items(sa, rs, o.iters, good ? o.n_out : 0, (long long)rank * kWarps + warp,
+                   (long long)p.team_size * kWarps, lane);
   }
 }
 
@@ -394,7 +391,7 @@ extern "C" KS_API int ks_match_batches(const ks_rec_desc* recs, int64_t n_recs,
     m.ctcT = d.ctcT;
     m.nm = reinterpret_cast<const float*>(base + pl.rec[r].nm);
     m.nmi = reinterpret_cast<const float2*>(base + pl.rec[r].nmi);
-    group_tables(base + pl.rec[r].groups, d.K, &m.rperm, &m.mg, &m.nmip);
+    group_tables(base + pl.rec[r].groups, d.K, &m.rperm, &m.mg, &m.nmip, &m.sup);
     m.C = (int)d.C;
     m.K = (int)d.K;
     m.P = (int)d.P;
@@ -409,6 +406,7 @@ extern "C" KS_API int ks_match_batches(const ks_rec_desc* recs, int64_t n_recs,
     const ks_rec_desc& r = recs[d.rec];
     MultiBatch& m = mp.batches[b];
     m.Bt = reinterpret_cast<float*>(base + pl.bat[b].bt);
+    m.X = d.X;
     m.Xres = d.Xres;
     m.st = reinterpret_cast<long long*>(d.st);
     m.amps = d.amps;
@@ -467,8 +465,6 @@ extern "C" KS_API int ks_match_batches(const ks_rec_desc* recs, int64_t n_recs,
       const ks_rec_desc& r = recs[d.rec];
       const RecPlan& rp = pl.rec[d.rec];
       const BatchPlan& bp = pl.bat[b];
-      if (d.Xres != d.X)
-        KS_CUDA(cudaMemcpyAsync(d.Xres, d.X, sizeof(float) * r.C * d.L, cudaMemcpyDeviceToDevice, ps));
       KS_CUDA(cudaMemsetAsync(d.info, 0xff, 4 * sizeof(int64_t), ps));   // "not run" until the peel writes it
       float* Bt = reinterpret_cast<float*>(base + bp.bt);
       if (precision == KS_PROJ_BF16X3) {

@@ -6,10 +6,11 @@ namespace ks {
 
 // Scratch of one single-batch peel: [team region] [lists] [nmi 8K], and for
 // the grouped update its tables (group_tables_bytes).
-// Tables of the grouped update: [rperm 4K] [key 4K] [mg 4*K*ng] [nmip 8K].
+// Tables of the grouped update: [rperm 4K] [key 4K] [mg 4*K*ng] [nmip 8K]
+// [sup 8K].
 static size_t group_setup_bytes(int64_t K) {
   return al256(4 * (size_t)K) + al256(4 * (size_t)K) + al256(4 * (size_t)K * n_groups(K)) +
-         al256(8 * (size_t)K);
+         2 * al256(8 * (size_t)K);
 }
 
 size_t peel_scratch_size(int64_t L, int64_t K, bool grouped) {
@@ -24,6 +25,7 @@ struct GroupTables {
   float* key;
   float* mg;
   float2* nmip;
+  unsigned long long* sup;
 };
 
 static GroupTables group_tables_at(void* tables, int64_t K) {
@@ -33,7 +35,9 @@ static GroupTables group_tables_at(void* tables, int64_t K) {
   t.rperm = reinterpret_cast<int*>(base);
   t.key = reinterpret_cast<float*>(base + k4);
   t.mg = reinterpret_cast<float*>(base + 2 * k4);
-  t.nmip = reinterpret_cast<float2*>(base + 2 * k4 + al256(4 * (size_t)K * n_groups(K)));
+  char* tail = base + 2 * k4 + al256(4 * (size_t)K * n_groups(K));
+  t.nmip = reinterpret_cast<float2*>(tail);
+  t.sup = reinterpret_cast<unsigned long long*>(tail + al256(8 * (size_t)K));
   return t;
 }
 
@@ -45,7 +49,7 @@ int launch_group_setup(const float* U, const float* ctcT, const float2* nmi, int
   const GroupTables t = group_tables_at(tables, K);
   const int ng = n_groups(K);
   ks_template_key_kernel<<<(unsigned)((K * 32 + 255) / 256), 256, 0, stream>>>(U, (int)K, (int)P,
-                                                                              (int)C, t.key);
+                                                                              (int)C, t.key, t.sup);
   KS_CUDA(cudaGetLastError());
   ks_group_order_kernel<<<(unsigned)((K + 255) / 256), 256, 0, stream>>>(t.key, (int)K, t.rperm);
   KS_CUDA(cudaGetLastError());
@@ -60,11 +64,12 @@ int launch_group_setup(const float* U, const float* ctcT, const float2* nmi, int
 }
 
 void group_tables(void* tables, int64_t K, const int** rperm, const float** mg,
-                  const float2** nmip) {
+                  const float2** nmip, const unsigned long long** sup) {
   const GroupTables t = group_tables_at(tables, K);
   *rperm = t.rperm;
   *mg = t.mg;
   *nmip = t.nmip;
+  *sup = t.sup;
 }
 
 int64_t tiled_rows_floats(int64_t L, int64_t K) { return ((L + kCol - 1) / kCol) * K * kCol; }
@@ -132,13 +137,13 @@ int peel_occupancy(const DeviceInfo& dev, size_t smem, const void* kernel, int* 
   return KS_OK;
 }
 
-int launch_peel_tiled(float* Bt, float* Xres, const float* U, const float* W,
+int launch_peel_tiled(float* Bt, const float* X, float* Xres, const float* U, const float* W,
                       const float* ctcT, const float* nm, int64_t C, int64_t L, int64_t K,
                       int64_t P, int64_t nt, float th2, int64_t max_peels,
                       int64_t capacity, int64_t* st, float* amps, float* th_amps,
                       int64_t* info, void* ws, size_t ws_bytes, cudaStream_t stream,
                       unsigned long long limit_ns, const int* upstream_err, bool grouped) {
-  if (!Bt || !Xres || !U || !W || !ctcT || !nm || !st || !amps || !th_amps || !info)
+  if (!Bt || !X || !Xres || !U || !W || !ctcT || !nm || !st || !amps || !th_amps || !info)
     return fail(KS_ERR_ARG, "ks_peel: null pointer");
   int rc = check_peel_shape(C, L, K, P, nt, th2, max_peels, capacity);
   if (rc) return rc;
@@ -150,7 +155,7 @@ int launch_peel_tiled(float* Bt, float* Xres, const float* U, const float* W,
   if (rc) return rc;
 
   PeelArgs a{};
-  a.Bt = Bt; a.Xres = Xres; a.U = U; a.W = W; a.ctcT = ctcT; a.nm = nm;
+  a.Bt = Bt; a.X = X; a.Xres = Xres; a.U = U; a.W = W; a.ctcT = ctcT; a.nm = nm;
   a.C = (int)C; a.L = (int)L; a.K = (int)K; a.P = (int)P; a.nt = (int)nt;
   a.th2 = th2;
   a.max_peels = (int)max_peels;
@@ -164,7 +169,7 @@ int launch_peel_tiled(float* Bt, float* Xres, const float* U, const float* W,
   float2* nmi = reinterpret_cast<float2*>(base + team_bytes + list_bytes);
   a.nmi = nmi;
   void* tables = base + team_bytes + list_bytes + al256(8 * (size_t)K);
-  if (grouped) group_tables(tables, K, &a.rperm, &a.mg, &a.nmip);
+  if (grouped) group_tables(tables, K, &a.rperm, &a.mg, &a.nmip, &a.sup);
   a.limit_ns = limit_ns;
   a.upstream_err = upstream_err;
 #ifdef KS_PEEL_TRACE
@@ -201,7 +206,7 @@ int launch_peel_tiled(float* Bt, float* Xres, const float* U, const float* W,
   // residual updates of all recorded spikes
   const long long n_res = (long long)a.nblk * ((C + 31) / 32);
   const unsigned rgrid = (unsigned)((n_res + kResWarps - 1) / kResWarps);
-  ks_residual_kernel<<<rgrid, kResThreads, residual_smem_bytes(a.P, a.nt), stream>>>(a);
+  ks_residual_kernel<<<rgrid, kResThreads, residual_smem_bytes(a.nt), stream>>>(a);
   KS_CUDA(cudaGetLastError());
   trace_mark(4, stream);
   return KS_OK;

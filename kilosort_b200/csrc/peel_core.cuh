@@ -11,7 +11,7 @@
 //   ctcT   [K][K][2nt+1] f32   ctcT[k][j][l] = ctc[j][k][l]: the cross-
 //                              correlations a peak of template k subtracts are
 //                              one contiguous slab
-//   Xres   [C][L] f32          residual, updated in place
+//   Xres   [C][L] f32          residual, written once after the loop from X
 //   cfmax [L] f32 / imax [L] i32  settled best score relu(B)^2/nm over
 //                              templates, and its template, per column
 //   pack   [2][L] u64          rescoring of dirty columns per iteration:
@@ -104,11 +104,14 @@ struct Touch {
 
 struct PeelArgs {
   float* Bt;
+  const float* X;             // the batch; Xres = X - residual updates (may be Xres)
   float* Xres;
   const float* U;
   const float* W;
   const float* ctcT;
   const float* nm;
+  const unsigned long long* sup;  // [K] channel groups where a template is not all zero
+                                  //     (support_width; null: taken as everywhere)
   const float2* nmi;          // {nm[j], 1/nm[j]} (1/nm NaN when nm is not a positive normal)
   int C, L, K, P, nt;
   float th2;
@@ -158,7 +161,7 @@ struct PeelArgs {
 };
 
 struct Smem {
-  float* W;        // Wt[nt][8] (the fused residual's basis)
+  float* W;        // [8][nt] (the fused residual's basis)
   int* prefix;     // nchunks+1   exclusive prefix of chunk peak counts
   int* wprefix;    // nwords+1    exclusive prefix of dirty-bitmap popcounts
   float* win;      // kChunk + 2*nt   column scores around the chunk
@@ -176,14 +179,10 @@ struct Smem {
                       //   of the rows of the group a warp processes
 };
 
-// Wt[t][p] = W[p][t] for p < P, 0 for P <= p < 8: each tap's components are
-// two aligned float4 in shared memory.
-__device__ __forceinline__ void stage_basis_t8(const float* W, int P, int nt, float* sWt,
-                                               int nthreads) {
-  for (int i = threadIdx.x; i < 8 * nt; i += nthreads) {
-    const int t = i >> 3, p = i & 7;
-    sWt[i] = p < P ? W[p * nt + t] : 0.f;
-  }
+// The basis [P][nt] in shared memory with rows P .. 7 zero.
+__device__ __forceinline__ void stage_basis(const float* W, int P, int nt, float* sW,
+                                            int nthreads) {
+  for (int i = threadIdx.x; i < 8 * nt; i += nthreads) sW[i] = i < P * nt ? W[i] : 0.f;
 }
 
 __device__ __forceinline__ Smem carve_smem(const PeelArgs& a, char* base, bool grouped) {
@@ -1101,7 +1100,7 @@ __device__ PeelOutcome run_peel(const PeelArgs& a, const Smem& s, int rank, unsi
   const int lane = tid & 31, warp = tid >> 5;
   const long long gwarp = (long long)rank * kWarps + warp;
   const long long nwarps = (long long)G * kWarps;
-  stage_basis_t8(a.W, a.P, a.nt, s.W, kThreads);
+  stage_basis(a.W, a.P, a.nt, s.W, kThreads);
   // a failed producer of the score matrix fails the peel
   if (rank == 0 && tid == 0 && a.upstream_err) {
     const int ue = ks_ld_volatile(a.upstream_err);
@@ -1316,17 +1315,34 @@ __global__ void __launch_bounds__(kThreads, 2) peel_kernel(PeelArgs a) {
   run_peel<kRowsPerWarp, kGrouped>(a, s, blockIdx.x, gridDim.x, epoch);
 }
 
-constexpr int kXTile = kCol * (kCol + 1);   // floats of one warp's transpose tile
-// the batched peel's residual lists and transpose tiles fit in the stage tiles
-static_assert(3 * kXList * 4 + kXTile * 4 <= 2 * kGroup * 32 * 4, "residual scratch exceeds a stage tile");
+// Per-warp scratch of the residual pass: the spike list (time, template,
+// amplitude) and one spike's loadings of 16 channels.
+constexpr int kXStride = 20;                // floats of a channel pair's loadings, padded
+                                            // so that the stores spread over the banks
+constexpr int kXU = 8 * kXStride;           // floats of one spike's loadings of 16 channels
+constexpr int kXWarp = 3 * kXList + kXU;    // 4-byte words per warp
+// the batched peel's residual scratch fits in the stage tiles
+static_assert(kXWarp <= 2 * kGroup * 32 && (3 * kXList) % 4 == 0,
+              "residual scratch exceeds a stage tile");
 
 struct ResSmem {
-  const float* W;  // Wt[t][8]: the basis transposed, components padded to 8
-  int* xl_tau;     // warps*kXList
+  const float* W;  // [8][nt]: the basis, rows past P zero
+  int* xl_tau;     // this warp's list, kXList entries
   int* xl_k;
   float* xl_amp;
-  float* xt;       // warps*kXTile (tiled form only): 32 channels x 33 floats per warp
+  float* xu;       // this warp's loadings, [8 channel pairs][kXStride]: [8 components][2]
 };
+
+__device__ __forceinline__ ResSmem residual_smem(const float* W, void* scratch, int warp) {
+  int* base = reinterpret_cast<int*>(scratch) + warp * kXWarp;
+  ResSmem r;
+  r.W = W;
+  r.xl_tau = base;
+  r.xl_k = base + kXList;
+  r.xl_amp = reinterpret_cast<float*>(base + 2 * kXList);
+  r.xu = reinterpret_cast<float*>(base + 3 * kXList);
+  return r;
+}
 
 // ---------------------------------------------------------------- RESIDUAL
 // After the loop: Xres[c, col] -= amp_s * sum_p U[k_s,p,c] W[p, col-tau_s+nt/2]
@@ -1339,13 +1355,13 @@ struct ResSmem {
 // lanes binary-search the time-sorted run of one iteration each.  Returns the
 // total number of such spikes.
 __device__ int gather_residual(const PeelArgs& a, const ResSmem& s, int n_iter,
-                               long long n_out, int c0, int skip, int lane, int warp) {
+                               long long n_out, int c0, int skip, int lane) {
   __syncwarp();   // earlier readers of the warp's list are done
   const int half = a.nt / 2;
   const long long wlo = (long long)c0 - half, whi = (long long)c0 + kCol - 1 + half;
-  int* ltau = s.xl_tau + warp * kXList;
-  int* lk = s.xl_k + warp * kXList;
-  float* lamp = s.xl_amp + warp * kXList;
+  int* ltau = s.xl_tau;
+  int* lk = s.xl_k;
+  float* lamp = s.xl_amp;
   int total = 0;
   for (int i0 = 0; i0 < n_iter; i0 += 32) {
     const int i = i0 + lane;
@@ -1387,8 +1403,7 @@ __device__ int gather_residual(const PeelArgs& a, const ResSmem& s, int n_iter,
 // Load into the warp's list the spikes whose residual window meets block blk,
 // in record order.  Returns their number; when it exceeds kXCap the per-block
 // record list overflowed and the caller gathers with gather_residual instead.
-__device__ int load_residual_list(const PeelArgs& a, const ResSmem& s, int blk, int lane,
-                                  int warp) {
+__device__ int load_residual_list(const PeelArgs& a, const ResSmem& s, int blk, int lane) {
   __syncwarp();
   const int n = a.xcount[blk];
   if (n > kXCap) return n;
@@ -1399,97 +1414,177 @@ __device__ int load_residual_list(const PeelArgs& a, const ResSmem& s, int blk, 
     rank += (oj < o) ? 1 : 0;
   }
   if (lane < n) {
-    s.xl_tau[warp * kXList + rank] = (int)a.st[2 * (long long)o];
-    s.xl_k[warp * kXList + rank] = (int)a.st[2 * (long long)o + 1];
-    s.xl_amp[warp * kXList + rank] = a.amps[o];
+    s.xl_tau[rank] = (int)a.st[2 * (long long)o];
+    s.xl_k[rank] = (int)a.st[2 * (long long)o + 1];
+    s.xl_amp[rank] = a.amps[o];
   }
   __syncwarp();
   return n;
 }
 
-// Residual of block blk for channels [32*cg, 32*cg + 32): lanes run over
-// channels, each lane keeps its 32 residual values in registers while the
-// listed spikes are subtracted in record order.  kTiled: the 32 x 32 tile
-// moves a channel row at a time (lanes over columns, one coalesced access
-// each) through a transpose in shared memory, instead of each lane touching
-// its own row 32 times; the batched peel, whose update phase gains more from
-// the L1 that this shared memory would take, uses the direct form.
-template <bool kTiled>
-__device__ void residual_item(const PeelArgs& a, const ResSmem& s, int n_iter, long long n_out,
-                              int blk, int cg, int lane, int warp) {
-  const int c0 = blk * kCol;
+// Two packed FP32 operations per instruction (each half rounds as the scalar
+// operation does).
+__device__ __forceinline__ unsigned long long f2_pack(float lo, float hi) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void f2_unpack(unsigned long long v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ unsigned long long f2_fma(unsigned long long a, unsigned long long b,
+                                                     unsigned long long c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ unsigned long long f2_mul(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ unsigned long long f2_add(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
+// Channels of one residual tile, and tiles per bit of a template's support
+// mask: the tiles 0 .. ceil(C/16)-1 are spread over 64 bits.
+constexpr int kXCh = 16;
+__host__ __device__ inline int support_width(int C) { return ((C + kXCh - 1) / kXCh + 63) / 64; }
+
+// Subtract the n listed spikes, in record order, from the tile of block blk
+// and channels [cbase, cbase + 16): lanes run over the block's columns and a
+// lane keeps its column's channel values in registers (x2, channel pairs).
+// Per spike a lane loads its tap's PP basis components (conflict-free rows of
+// W); the spike's loadings of the tile's channels come from the warp's shared
+// buffer, loaded from U one spike ahead; channels are processed two at a time
+// with packed FP32 operations: per element the reference's products in the
+// same order, each rounded as the scalar operation.  Spikes whose template is
+// exactly zero on the tile (a.sup) would subtract +0 and are passed over.
+//
+// What bounds it: instruction issue (about 5.5 warp instructions per channel
+// row and spike) next to the 8CL bytes of X and Xres (185 MB, 28 us).  The
+// form with lanes over channels, which applied every listed spike to an Xres
+// copied from X beforehand, took 493 us + 38 us for the copy on a C=384, K=600
+// batch of 60122 samples; this one takes 159 us without a copy, and the
+// batched launch of 16 such batches 29.1 -> 21.6 ms.  Tiles of 32 channels
+// spilled at the peel's 80 registers and pass over fewer spikes.
+template <int PP>
+__device__ void residual_apply(const PeelArgs& a, const ResSmem& s, int n, int c0, int cbase,
+                               int bit, int lane, unsigned long long* x2) {
   const int half = a.nt / 2, nt = a.nt, P = a.P;
-  const int c = cg * 32 + lane;
-  const bool chok = c < a.C;
-  int total = load_residual_list(a, s, blk, lane, warp);
-  const bool overflow = total > kXCap;
-  if (overflow) total = gather_residual(a, s, n_iter, n_out, c0, 0, lane, warp);
-  if (total == 0) return;
-  const int ncol = min(kCol, a.L - c0);
-  float* xrow = a.Xres + (long long)c * a.L + c0;
-  float* xt = kTiled ? s.xt + warp * kXTile : nullptr;
-  const int cbase = cg * 32;
-  const bool colok = lane < ncol;
-  float x[kCol];
-  if (kTiled) {
-    {
-      float v[kCol];
+  const int ch = cbase + (lane & (kXCh - 1));
+  const int p0 = (lane / kXCh) * (PP / 2);     // this lane loads components p0 .. p0 + PP/2 - 1
+  const bool chok = ch < a.C;
+  for (int e0 = 0; e0 < n; e0 += 32) {
+    bool hit = e0 + lane < n;
+    if (hit && a.sup) hit = (a.sup[s.xl_k[e0 + lane]] >> bit) & 1ull;
+    unsigned todo = __ballot_sync(0xffffffffu, hit);
+    if (!todo) continue;
+    float u[PP / 2];
+    auto fetch = [&](int e) {
+      const float* up = a.U + ((long long)s.xl_k[e0 + e] * P + p0) * a.C + ch;
 #pragma unroll
-      for (int r = 0; r < kCol; ++r)
-        v[r] = (colok && cbase + r < a.C) ? a.Xres[(long long)(cbase + r) * a.L + c0 + lane] : 0.f;
+      for (int j = 0; j < PP / 2; ++j)
+        u[j] = (chok && p0 + j < P) ? __ldg(up + (long long)j * a.C) : 0.f;
+    };
+    fetch(__ffs(todo) - 1);
+    while (todo) {
+      const int e = __ffs(todo) - 1;
+      todo &= todo - 1u;
+      __syncwarp();                    // the previous spike's loadings are read
+      {
+        float* dst = s.xu + ((lane & (kXCh - 1)) >> 1) * kXStride + (lane & 1) + 2 * p0;
 #pragma unroll
-      for (int r = 0; r < kCol; ++r) xt[r * (kCol + 1) + lane] = v[r];
-    }
-    __syncwarp();
+        for (int j = 0; j < PP / 2; ++j) dst[2 * j] = u[j];
+      }
+      __syncwarp();
+      if (todo) fetch(__ffs(todo) - 1);
+      const int t = c0 + lane - s.xl_tau[e0 + e] + half;
+      const bool in = t >= 0 && t < nt;
+      const float namp = -s.xl_amp[e0 + e];
+      const unsigned long long amp2 = f2_pack(namp, namp);
+      unsigned long long w2[PP];
 #pragma unroll
-    for (int j = 0; j < kCol; ++j) x[j] = xt[lane * (kCol + 1) + j];
-  } else {
+      for (int p = 0; p < PP; ++p) {
+        const float wv = in ? s.W[p * nt + t] : 0.f;
+        w2[p] = f2_pack(wv, wv);
+      }
 #pragma unroll
-    for (int j = 0; j < kCol; ++j) x[j] = (chok && j < ncol) ? xrow[j] : 0.f;
-  }
-  const int epochs = (total + kXList - 1) / kXList;
-  for (int ep = 0; ep < epochs; ++ep) {
-    if (ep > 0) gather_residual(a, s, n_iter, n_out, c0, ep * kXList, lane, warp);
-    const int n = min(kXList, total - ep * kXList);
-    for (int e = 0; e < n; ++e) {
-      const int tau = s.xl_tau[warp * kXList + e];
-      const int k = s.xl_k[warp * kXList + e];
-      const float amp = s.xl_amp[warp * kXList + e];
-      const int t0 = c0 - tau + half;   // tap of column c0
-      float u[8];
+      for (int i = 0; i < kXCh / 2; ++i) {
+        const ulonglong2* u4 = reinterpret_cast<const ulonglong2*>(s.xu + i * kXStride);
+        unsigned long long v = 0ull;
 #pragma unroll
-      for (int pp = 0; pp < 8; ++pp)
-        u[pp] = (chok && pp < P) ? __ldg(a.U + ((long long)k * P + pp) * a.C + c) : 0.f;
-      const float4* W4 = reinterpret_cast<const float4*>(s.W);
-#pragma unroll
-      for (int j = 0; j < kCol; ++j) {
-        const int t = t0 + j;
-        if (t >= 0 && t < nt) {
-          // the tap's P components: two broadcast 16-byte loads
-          const float4 wa = W4[2 * t], wb = W4[2 * t + 1];
-          const float wt[8] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
-          float wv = 0.f;
-#pragma unroll
-          for (int pp = 0; pp < 8; ++pp)
-            if (pp < P) wv = fmaf(u[pp], wt[pp], wv);
-          x[j] = __fsub_rn(x[j], __fmul_rn(amp, wv));
+        for (int p = 0; p < PP; p += 2) {
+          const ulonglong2 uu = u4[p >> 1];
+          v = f2_fma(uu.x, w2[p], v);
+          v = f2_fma(uu.y, w2[p + 1], v);
         }
+        // x - fl(amp v) = x + fl(-amp v), on the columns inside the window
+        const unsigned long long d = f2_mul(amp2, v);
+        if (in) x2[i] = f2_add(x2[i], d);
       }
     }
   }
-  if (kTiled) {
-    __syncwarp();
+}
+
+// Residual of block blk for channels [32*cg, 32*cg + 32), two tiles: X is
+// read, the block's spikes are subtracted and Xres is written (Xres may be X).
+template <int PP>
+__device__ void residual_item(const PeelArgs& a, const ResSmem& s, int n_iter, long long n_out,
+                              int blk, int cg, int lane) {
+  const int c0 = blk * kCol;
+  const long long col = c0 + lane;
+  const bool colok = col < a.L;
+  const bool copy = a.X != a.Xres;
+  int total = n_out > 0 ? load_residual_list(a, s, blk, lane) : 0;
+  const bool gathered = total > kXCap;
+  if (gathered) total = gather_residual(a, s, n_iter, n_out, c0, 0, lane);
+  if (!copy && total == 0) return;
+  const int width = support_width(a.C);
+#pragma unroll 1
+  for (int h = 0; h < 2; ++h) {
+    const int cbase = cg * 32 + h * kXCh;
+    if (cbase >= a.C) break;
+    const float* src = a.X + (long long)cbase * a.L + col;
+    float* out = a.Xres + (long long)cbase * a.L + col;
+    unsigned long long x2[kXCh / 2];
 #pragma unroll
-    for (int j = 0; j < kCol; ++j) xt[lane * (kCol + 1) + j] = x[j];
-    __syncwarp();
+    for (int i = 0; i < kXCh / 2; ++i) {
+      const float lo = (colok && cbase + 2 * i < a.C) ? src[(long long)(2 * i) * a.L] : 0.f;
+      const float hi = (colok && cbase + 2 * i + 1 < a.C) ? src[(long long)(2 * i + 1) * a.L] : 0.f;
+      x2[i] = f2_pack(lo, hi);
+    }
+    // more spikes than the warp's list holds: gathered kXList at a time
+    for (int done = 0; done < total; done += kXList) {
+      if (gathered && total > kXList)
+        gather_residual(a, s, n_iter, n_out, c0, done, lane);
+      residual_apply<PP>(a, s, min(kXList, total - done), c0, cbase, cbase / kXCh / width, lane,
+                         x2);
+    }
 #pragma unroll
-    for (int r = 0; r < kCol; ++r)
-      if (colok && cbase + r < a.C)
-        a.Xres[(long long)(cbase + r) * a.L + c0 + lane] = xt[r * (kCol + 1) + lane];
-  } else {
-#pragma unroll
-    for (int j = 0; j < kCol; ++j)
-      if (chok && j < ncol) xrow[j] = x[j];
+    for (int i = 0; i < kXCh / 2; ++i) {
+      float lo, hi;
+      f2_unpack(x2[i], lo, hi);
+      if (colok && cbase + 2 * i < a.C) out[(long long)(2 * i) * a.L] = lo;
+      if (colok && cbase + 2 * i + 1 < a.C) out[(long long)(2 * i + 1) * a.L] = hi;
+    }
+  }
+}
+
+// The residual of every (block, channel group) w, w + step, ... below the
+// batch's count.
+__device__ __forceinline__ void residual_items(const PeelArgs& a, const ResSmem& s, int n_iter,
+                                               long long n_out, long long w, long long step,
+                                               int lane) {
+  const int xg = (a.C + 31) / 32;
+  const long long n_items = (long long)a.nblk * xg;
+  for (; w < n_items; w += step) {
+    const int blk = (int)(w / xg), cg = (int)(w % xg);
+    if (a.P <= 6) residual_item<6>(a, s, n_iter, n_out, blk, cg, lane);
+    else residual_item<8>(a, s, n_iter, n_out, blk, cg, lane);
   }
 }
 
@@ -1497,36 +1592,24 @@ constexpr int kResThreads = 256;
 constexpr int kResWarps = kResThreads / 32;
 
 // One warp per (32-column block, 32 channels) of the residual; runs after the
-// peel kernel on the same stream and reads its outcome from info.
+// peel kernel on the same stream and reads its outcome from info (a failed
+// peel leaves Xres = X).
 __global__ void __launch_bounds__(kResThreads)
 ks_residual_kernel(PeelArgs a) {
   extern __shared__ __align__(16) char smem_raw[];
   float* sW = reinterpret_cast<float*>(smem_raw);
-  ResSmem s;
-  s.W = sW;
-  s.xl_tau = reinterpret_cast<int*>(sW + 8 * a.nt);
-  s.xl_k = s.xl_tau + kResWarps * kXList;
-  s.xl_amp = reinterpret_cast<float*>(s.xl_k + kResWarps * kXList);
-  s.xt = s.xl_amp + kResWarps * kXList;
-  stage_basis_t8(a.W, a.P, a.nt, sW, kResThreads);
+  stage_basis(a.W, a.P, a.nt, sW, kResThreads);
   __syncthreads();
-  const long long n_out = a.info[0];
-  const int status = (int)a.info[1];
+  const long long n_out = (int)a.info[1] == KS_OK ? a.info[0] : 0;
   const int n_iter = (int)a.info[2];
-  if (status != KS_OK || n_out <= 0) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int xg = (a.C + 31) / 32;
-  const long long n_items = (long long)a.nblk * xg;
-  const long long w = (long long)blockIdx.x * kResWarps + warp;
-  if (w >= n_items) return;
-  residual_item<true>(a, s, n_iter, n_out, (int)(w / xg), (int)(w % xg), lane, warp);
+  const ResSmem s = residual_smem(sW, sW + 8 * a.nt, warp);
+  residual_items(a, s, n_iter, n_out, (long long)blockIdx.x * kResWarps + warp,
+                 (long long)gridDim.x * kResWarps, lane);
 }
 
-size_t residual_smem_bytes(int P, int nt) {
-  (void)P;
-  return sizeof(float) * 8 * (size_t)nt +
-         (size_t)kResWarps * kXList * (2 * sizeof(int) + sizeof(float)) +
-         sizeof(float) * (size_t)kResWarps * kXTile;
+size_t residual_smem_bytes(int nt) {
+  return sizeof(float) * (8 * (size_t)nt + (size_t)kResWarps * kXWarp);
 }
 
 __global__ void ks_nm_pair_kernel(const float* __restrict__ nm, int K, float2* __restrict__ nmi) {
@@ -1581,28 +1664,43 @@ __global__ void ks_ctc_transpose_kernel(const float* __restrict__ ctc, int K, in
 // results.
 //
 // Spatial key of each template: the channel centroid sum_c c*e_c / sum_c e_c
-// of its energy e_c = sum_p U[k,p,c]^2 (0 for a template without energy).
-// One warp per template, fixed summation order.
+// of its energy e_c = sum_p U[k,p,c]^2 (0 for a template without energy), and
+// its support mask: bit (c/16)/support_width(C) is set where some U[k,p,c] is
+// not zero.  One warp per template, fixed summation order.
 __global__ void ks_template_key_kernel(const float* __restrict__ U, int K, int P, int C,
-                                       float* __restrict__ key) {
+                                       float* __restrict__ key,
+                                       unsigned long long* __restrict__ sup) {
   const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (w >= K) return;
+  const int width = support_width(C);
   double se = 0.0, sc = 0.0;
-  for (int c = lane; c < C; c += 32) {
+  unsigned long long mask = 0ull;
+  for (int c0 = 0; c0 < C; c0 += 32) {
+    const int c = c0 + lane;
     float e = 0.f;
-    for (int p = 0; p < P; ++p) {
-      const float u = U[((size_t)w * P + p) * C + c];
-      e = fmaf(u, u, e);
+    bool nz = false;
+    if (c < C) {
+      for (int p = 0; p < P; ++p) {
+        const float u = U[((size_t)w * P + p) * C + c];
+        e = fmaf(u, u, e);
+        nz |= u != 0.f;
+      }
+      se += e;
+      sc += (double)c * e;
     }
-    se += e;
-    sc += (double)c * e;
+    const unsigned b = __ballot_sync(0xffffffffu, nz);
+    if (b & 0xffffu) mask |= 1ull << (c0 / kXCh / width);
+    if (b >> 16) mask |= 1ull << ((c0 / kXCh + 1) / width);
   }
   for (int o = 16; o; o >>= 1) {
     se += __shfl_xor_sync(0xffffffffu, se, o);
     sc += __shfl_xor_sync(0xffffffffu, sc, o);
   }
-  if (lane == 0) key[w] = se > 0.0 ? (float)(sc / se) : 0.f;
+  if (lane == 0) {
+    key[w] = se > 0.0 ? (float)(sc / se) : 0.f;
+    sup[w] = mask;
+  }
 }
 
 __device__ __forceinline__ unsigned sortable_key(float f) {

@@ -102,7 +102,7 @@ size_t group_tables_bytes(int64_t K);
 int launch_group_setup(const float* U, const float* ctcT, const float2* nmi, int64_t K,
                        int64_t P, int64_t C, int64_t nt, void* tables, cudaStream_t stream);
 void group_tables(void* tables, int64_t K, const int** rperm, const float** mg,
-                  const float2** nmip);
+                  const float2** nmip, const unsigned long long** sup);
 int64_t tiled_rows_floats(int64_t L, int64_t K);
 int launch_tile_rows(const float* B, int64_t ldb, int64_t K, int64_t L, float* Bt,
                      cudaStream_t stream);
@@ -113,7 +113,8 @@ int launch_ctc_transpose(const float* ctc, int64_t K, int64_t nt, float* ctcT,
 int check_peel_shape(int64_t C, int64_t L, int64_t K, int64_t P, int64_t nt, float th2,
                      int64_t max_peels, int64_t capacity);
 int launch_nm_pairs(const float* nm, int64_t K, float2* nmi, cudaStream_t stream);
-int launch_peel_tiled(float* Bt, float* Xres, const float* U, const float* W,
+// Xres is written from X (they may be the same array).
+int launch_peel_tiled(float* Bt, const float* X, float* Xres, const float* U, const float* W,
                       const float* ctcT, const float* nm, int64_t C, int64_t L, int64_t K,
                       int64_t P, int64_t nt, float th2, int64_t max_peels,
                       int64_t capacity, int64_t* st, float* amps, float* th_amps,
