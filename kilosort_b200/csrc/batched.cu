@@ -40,7 +40,7 @@ struct MultiRec {
   const float2* nmi;
   const int* rperm;             // group order of the grouped update
   const float* mg;              // its product bounds [K][ng]
-  const float2* nmip;           // {nm, 1/nm} in group order
+  const float2* nmip;           // {nm, 1/sqrt(nm)} in group order
   const unsigned long long* sup;  // support masks
   int C, K, P, nt;
   float th2;
@@ -72,6 +72,7 @@ struct MultiParams {
   unsigned long long limit_ns;
   const int* upstream_err;
   size_t peel_smem;             // dynamic shared bytes of the peel
+  float one;                    // 1 (PeelArgs::one)
 };
 
 __device__ void fill_args(const MultiParams& p, int b, char* team, PeelArgs& a) {
@@ -92,6 +93,7 @@ __device__ void fill_args(const MultiParams& p, int b, char* team, PeelArgs& a) 
   a.P = r.P;
   a.nt = r.nt;
   a.th2 = r.th2;
+  a.one = p.one;
   a.max_peels = r.max_peels;
   a.capacity = r.capacity;
   a.st = mb.st;
@@ -116,43 +118,9 @@ __device__ void fill_args(const MultiParams& p, int b, char* team, PeelArgs& a) 
 // ks_residual_kernel does), so one team's residual work fills the barrier
 // waits of the others.  A team peels nothing after its first error (info of
 // its later batches keeps the "not run" value, their Xres is X).
-template <int kRows, bool kLean>
-__device__ __forceinline__ void peel_multi_body(const MultiParams& p, char* smem_raw,
-                                                PeelArgs& sa);
-
-// Alone on the device: 2 blocks per SM (64 registers per thread).
-__global__ void __launch_bounds__(kThreads, 2) peel_multi_kernel(const __grid_constant__ MultiParams p) {
+__global__ void __launch_bounds__(kThreads, kTeamBlocksPerSm) peel_multi_kernel(const __grid_constant__ MultiParams p) {
   extern __shared__ __align__(16) char smem_raw[];
   __shared__ PeelArgs sa;
-  peel_multi_body<kRowsPerWarp, false>(p, smem_raw, sa);
-}
-
-// The same with the lean group fold (group_tile<true>), for small teams: a
-// team of at most kLeanTeamBlocks blocks works through tens of tiles per warp
-// and phase, where fewer instructions per row pay; larger teams (few tiles
-// per warp, phases bound by their barriers) measured faster with the other
-// fold.  Results are identical.
-constexpr int kLeanTeamBlocks = 16;
-__global__ void __launch_bounds__(kThreads, 2)
-peel_multi_kernel_lean(const __grid_constant__ MultiParams p) {
-  extern __shared__ __align__(16) char smem_raw[];
-  __shared__ PeelArgs sa;
-  peel_multi_body<kRowsPerWarp, true>(p, smem_raw, sa);
-}
-
-// Beside the projection kernels of the next group: 1 block per SM capped at
-// 80 registers per thread (40960 of the SM's 65536), which leaves room for a
-// tensor-core contraction CTA (192 x 64) or a temporal-projection block
-// (256 x 80) on the same SM.
-__global__ void __maxnreg__(80) peel_multi_kernel_shared(const __grid_constant__ MultiParams p) {
-  extern __shared__ __align__(16) char smem_raw[];
-  __shared__ PeelArgs sa;
-  peel_multi_body<kRowsPerWarp, false>(p, smem_raw, sa);
-}
-
-template <int kRows, bool kLean>
-__device__ __forceinline__ void peel_multi_body(const MultiParams& p, char* smem_raw,
-                                                PeelArgs& sa) {
   const int team = blockIdx.x / p.team_size;
   const int rank = blockIdx.x % p.team_size;
   const int n_teams = gridDim.x / p.team_size;
@@ -167,7 +135,7 @@ __device__ __forceinline__ void peel_multi_body(const MultiParams& p, char* smem
     const Smem s = carve_smem(sa, smem_raw, true);
     PeelOutcome o{0, 0, KS_OK};
     if (!failed) {
-      o = run_peel<kRows, true, kLean>(sa, s, rank, (unsigned)p.team_size, epoch);
+      o = run_peel<kRowsPerWarp, true>(sa, s, rank, (unsigned)p.team_size, epoch);
       failed = o.status != KS_OK && o.status != KS_ERR_OVERFLOW;   // overflow: that batch only
     }
     const bool good = !failed && o.status == KS_OK;
@@ -305,18 +273,10 @@ cudaEvent_t pipeline_event(int i) {
   return ev[i];
 }
 
-// Kernel and resident blocks per SM of the peel: alone on the device 2 blocks
-// per SM; pipelined 1 block per SM, which leaves room on every SM for a block
-// of the projection kernels of the next group.
-struct PeelVariant {
-  void (*kernel)(MultiParams);
-  int blocks_per_sm;
-};
-
-PeelVariant peel_variant(bool pipelined) {
-  if (pipelined) return PeelVariant{peel_multi_kernel_shared, 1};
-  return PeelVariant{peel_multi_kernel, 2};
-}
+// Resident blocks per SM of the peel: alone on the device kTeamBlocksPerSm;
+// pipelined 1, which leaves room on every SM for a block of the projection
+// kernels of the next group.
+int peel_blocks_per_sm(bool pipelined) { return pipelined ? 1 : kTeamBlocksPerSm; }
 
 }  // namespace
 
@@ -426,16 +386,16 @@ extern "C" KS_API int ks_match_batches(const ks_rec_desc* recs, int64_t n_recs,
   mp.upstream_err = precision == KS_PROJ_BF16X3 ? gemm_err : nullptr;
   smem = (smem + 15) & ~size_t(15);
   mp.peel_smem = smem;
-  const PeelVariant pv = peel_variant(pipelined);
+  mp.one = 1.f;
   cudaFuncAttributes fa;
-  KS_CUDA(cudaFuncGetAttributes(&fa, pv.kernel));
+  KS_CUDA(cudaFuncGetAttributes(&fa, peel_multi_kernel));
   if (smem + fa.sharedSizeBytes > dev.smem_optin)
     return fail(KS_ERR_UNSUPPORTED, "ks_match_batches: batch too long for shared memory");
-  KS_CUDA(cudaFuncSetAttribute(pv.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  KS_CUDA(cudaFuncSetAttribute(peel_multi_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int occ = 0;
-  KS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, pv.kernel, kThreads, smem));
+  KS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, peel_multi_kernel, kThreads, smem));
   if (occ < 1) return fail(KS_ERR_UNSUPPORTED, "ks_match_batches: peel does not fit on an SM");
-  const int max_blocks = dev.sm_count * std::min(occ, pv.blocks_per_sm);
+  const int max_blocks = dev.sm_count * std::min(occ, peel_blocks_per_sm(pipelined));
 
   static thread_local GemmGroup g;      // about 14 KB: kept off the stack
   if (precision == KS_PROJ_BF16X3) {
@@ -530,18 +490,7 @@ extern "C" KS_API int ks_match_batches(const ks_rec_desc* recs, int64_t n_recs,
     cfg.stream = s;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    void (*kernel)(MultiParams) = pv.kernel;
-    if (pv.kernel == peel_multi_kernel && mp.team_size <= kLeanTeamBlocks) {
-      // small teams: the lean fold, if it is as resident as the other form
-      KS_CUDA(cudaFuncSetAttribute(peel_multi_kernel_lean,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      int occ_lean = 0;
-      KS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_lean, peel_multi_kernel_lean,
-                                                            kThreads, smem));
-      if (dev.sm_count * std::min(occ_lean, pv.blocks_per_sm) >= max_blocks)
-        kernel = peel_multi_kernel_lean;
-    }
-    KS_CUDA(cudaLaunchKernelEx(&cfg, kernel, mp));
+    KS_CUDA(cudaLaunchKernelEx(&cfg, peel_multi_kernel, mp));
   }
   // the residual passes ran inside the peel launches
   trace_mark(3, s);

@@ -6,11 +6,13 @@ namespace ks {
 
 // Scratch of one single-batch peel: [team region] [lists] [nmi 8K], and for
 // the grouped update its tables (group_tables_bytes).
-// Tables of the grouped update: [rperm 4K] [key 4K] [mg 4*K*ng] [nmip 8K]
-// [sup 8K].
+// Tables of the grouped update: [rperm 4Kg] [key 4K] [mg 4*K*ng] [nmip 8Kg]
+// [sup 8K], Kg = K padded to whole groups.
+static int64_t group_rows_padded(int64_t K) { return (int64_t)n_groups(K) * kGroup; }
 static size_t group_setup_bytes(int64_t K) {
-  return al256(4 * (size_t)K) + al256(4 * (size_t)K) + al256(4 * (size_t)K * n_groups(K)) +
-         2 * al256(8 * (size_t)K);
+  const size_t Kg = (size_t)group_rows_padded(K);
+  return al256(4 * Kg) + al256(4 * (size_t)K) + al256(4 * (size_t)K * n_groups(K)) +
+         al256(8 * Kg) + al256(8 * (size_t)K);
 }
 
 size_t peel_scratch_size(int64_t L, int64_t K, bool grouped) {
@@ -30,14 +32,17 @@ struct GroupTables {
 
 static GroupTables group_tables_at(void* tables, int64_t K) {
   char* base = static_cast<char*>(tables);
-  const size_t k4 = al256(4 * (size_t)K);
+  const size_t Kg = (size_t)group_rows_padded(K);
   GroupTables t;
   t.rperm = reinterpret_cast<int*>(base);
-  t.key = reinterpret_cast<float*>(base + k4);
-  t.mg = reinterpret_cast<float*>(base + 2 * k4);
-  char* tail = base + 2 * k4 + al256(4 * (size_t)K * n_groups(K));
-  t.nmip = reinterpret_cast<float2*>(tail);
-  t.sup = reinterpret_cast<unsigned long long*>(tail + al256(8 * (size_t)K));
+  base += al256(4 * Kg);
+  t.key = reinterpret_cast<float*>(base);
+  base += al256(4 * (size_t)K);
+  t.mg = reinterpret_cast<float*>(base);
+  base += al256(4 * (size_t)K * n_groups(K));
+  t.nmip = reinterpret_cast<float2*>(base);
+  base += al256(8 * Kg);
+  t.sup = reinterpret_cast<unsigned long long*>(base);
   return t;
 }
 
@@ -57,7 +62,7 @@ int launch_group_setup(const float* U, const float* ctcT, const float2* nmi, int
   ks_group_bound_kernel<<<(unsigned)std::min<long long>(items, 1 << 20), 256, 0, stream>>>(
       ctcT, t.rperm, (int)K, (int)(2 * nt + 1), ng, t.mg);
   KS_CUDA(cudaGetLastError());
-  ks_group_nmi_kernel<<<(unsigned)((K + 255) / 256), 256, 0, stream>>>(nmi, t.rperm, (int)K,
+  ks_group_nmi_kernel<<<(unsigned)((K + 31 + 255) / 256), 256, 0, stream>>>(nmi, t.rperm, (int)K,
                                                                       t.nmip);
   KS_CUDA(cudaGetLastError());
   return KS_OK;
@@ -158,6 +163,7 @@ int launch_peel_tiled(float* Bt, const float* X, float* Xres, const float* U, co
   a.Bt = Bt; a.X = X; a.Xres = Xres; a.U = U; a.W = W; a.ctcT = ctcT; a.nm = nm;
   a.C = (int)C; a.L = (int)L; a.K = (int)K; a.P = (int)P; a.nt = (int)nt;
   a.th2 = th2;
+  a.one = 1.f;
   a.max_peels = (int)max_peels;
   a.capacity = capacity;
   a.st = reinterpret_cast<long long*>(st); a.amps = amps; a.th_amps = th_amps;

@@ -33,10 +33,11 @@
 //           and clears its pack[p] entries.
 //   UPDATE  every block computes the exclusive prefix of the chunk counts (a
 //           peak's global index in the iteration) and of the dirty bitmap.
-//           Records are written in (iteration, tau) order.  Warps take work
-//           items (dirty block in column order, row range) from a counter
-//           (large teams: round-robin, the last round from the counter):
-//           B[j,c] -= amp*ctc[j,k,c-tau+nt] for the peaks touching column c,
+//           Records are written in (iteration, tau) order.  Warps scan the dirty
+//           blocks and work through the units found (grouped update), or take
+//           work items (dirty block in column order, row range) from a counter
+//           (ungrouped; large teams: round-robin, the last round from the
+//           counter): B[j,c] -= amp*ctc[j,k,c-tau+nt] for the peaks touching column c,
 //           even-indexed peaks first, then odd-indexed -- the order of the
 //           reference's two interleaved groups (:235-238) -- product and
 //           difference rounded separately; rescored rows fold into pack[p].
@@ -54,7 +55,14 @@
 
 namespace {
 
-constexpr int kThreads = 384;
+constexpr int kThreads = 256;
+// Resident blocks per SM.  The single-batch launch (its phases end at
+// barriers of the whole device, so fewer, faster blocks pay): 1.53 ms with 2,
+// 1.63 ms with 3 for the iterations of a C=384, K=600 batch.  Teams work
+// through many units per phase: 11.0 ms with 3, 11.5 with 2, 13.2 with 4 for 16
+// such batches by 16 teams.
+constexpr int kBlocksPerSm = 2;
+constexpr int kTeamBlocksPerSm = 3;
 constexpr int kWarps = kThreads / 32;
 constexpr int kChunk = 256;          // detection chunk, one column per thread
 constexpr int kCol = 32;             // update block, one column per lane
@@ -70,7 +78,15 @@ constexpr int kMaxTemplates = 65536; // templates of one batch
 constexpr int kXList = 64;           // residual list entries per warp and epoch
 constexpr int kXCap = 32;            // spikes recorded per block for the residual
 constexpr int kGroup = 32;           // template rows of one group (grouped update)
-constexpr int kInitGroups = 2;       // groups per item of the initial scoring
+constexpr long long kStaticUnits = 4; // units per warp up to which they are dealt round-robin
+__host__ __device__ inline int n_groups(long long K) { return (int)((K + kGroup - 1) / kGroup); }
+constexpr int kTileBytes = 4096;     // a warp's tile: a unit's ctc rows (4 KB), a scan's
+                                     // metadata, a detection chunk's windows; larger tiles
+                                     // leave L1 too few lines for the loads in flight (units
+                                     // 6.7 ms of the 16-batch launch, 8.1 with 6 KB)
+constexpr int kScanGroups = 14;      // groups whose metadata a scan stages at once
+static_assert(kScanGroups * 32 * 9 <= kTileBytes && kScanGroups <= 32 &&
+              kGroup * 32 * 4 <= kTileBytes, "a warp's tile is too small");
 
 // Phase timeline for profiling builds (-DKS_PEEL_TRACE): block 0 writes
 // %globaltimer stamps to info[8 + 8*it + slot]; the caller sizes info.
@@ -115,6 +131,7 @@ struct PeelArgs {
   const float2* nmi;          // {nm[j], 1/nm[j]} (1/nm NaN when nm is not a positive normal)
   int C, L, K, P, nt;
   float th2;
+  float one;                  // 1 (see f2_add_prod)
   int max_peels;
   long long capacity;
   long long* st;
@@ -144,7 +161,8 @@ struct PeelArgs {
   // grouped update (null rperm: every row of a touched column is rewritten)
   const int* rperm;           // [K] template rows in group order (group g: rows
                               //     rperm[32g .. 32g+31])
-  const float2* nmip;         // [K] {nm, 1/nm} in group order, nmip[r] = nmi[rperm[r]]
+  const float2* nmip;         // [K] {nm, 1/sqrt(nm)} in group order (the scale NaN for an
+                              //     nm outside [2^-30, 2^30])
   const float* mg;            // [K][ng] largest |ctcT[k][j][l]| over the rows j
                               //     of group g and all lags
   unsigned long long* gbest;  // [nblk][ng][32] packed best score of each group
@@ -160,23 +178,34 @@ struct PeelArgs {
   unsigned long long limit_ns;
 };
 
+// Detection by one warp per chunk: where a chunk's two window buffers and its
+// template indices fit in the warp's tile (nt <= 64) and the team has fewer
+// blocks than the batch has chunks.  A block finishes one chunk sooner (3 us
+// against 5 us), but a team of 18 blocks took 50 us an iteration for the 235
+// chunks of 60122 samples one after the other, and 14 us by warps.
+__host__ __device__ inline bool warp_detection(int nt, bool grouped, int nchunks, unsigned G) {
+  return grouped && (2 * (kChunk + 2 * nt) + kChunk) * 4 <= kTileBytes && (unsigned)nchunks > G;
+}
+
+constexpr int kUnitBytes = 2 * 512;  // inputs of a warp's units in flight (UnitIn)
+
 struct Smem {
   float* W;        // [8][nt] (the fused residual's basis)
   int* prefix;     // nchunks+1   exclusive prefix of chunk peak counts
   int* wprefix;    // nwords+1    exclusive prefix of dirty-bitmap popcounts
-  float* win;      // kChunk + 2*nt   column scores around the chunk
+  unsigned* dw;    // nwords      the iteration's dirty bitmap
+  float* win;      // kChunk + 2*nt   column scores around the chunk (block detection)
   float* mx0;      // kChunk + 2*nt   sliding-max doubling levels (ping-pong)
   float* mx1;      // kChunk + 2*nt
   int* kidx;       // kChunk          best template of the chunk's own columns
   int* wcnt;       // kWarps+1
-  int* tl_tau;     // kWarps*kTouch   ordered touch list of each warp's item
+  int* tl_tau;     // kWarps*kTouch ordered touch list of each warp's item
   int* tl_k;       // kWarps*kTouch
   float* tl_amp;   // kWarps*kTouch
   unsigned char* eb;  // kWarps*kTouch*32  bound exponents of a warp's touching peaks
-  float* stage;       // kWarps*2*kGroup*32 (grouped update only): a warp's tile of
-                      //   B rows [kGroup][32] and of ctc rows [kGroup][32]
-  float2* rtab;       // kWarps*kGroup (grouped update only): row index bits and nm
-                      //   of the rows of the group a warp processes
+  float* stage;       // kWarps*kTileBytes (grouped update only): a warp's tile (of ctc
+                      //   rows [kGroup][32], then of the updated scores)
+  struct UnitIn* unit;  // kWarps*kUnitSlots (grouped update only): inputs of a warp's units
 };
 
 // The basis [P][nt] in shared memory with rows P .. 7 zero.
@@ -197,6 +226,7 @@ __device__ __forceinline__ Smem carve_smem(const PeelArgs& a, char* base, bool g
   s.W = reinterpret_cast<float*>(take(sizeof(float) * 8 * a.nt));
   s.prefix = reinterpret_cast<int*>(take(sizeof(int) * (a.nchunks + 1)));
   s.wprefix = reinterpret_cast<int*>(take(sizeof(int) * (a.nwords + 1)));
+  s.dw = reinterpret_cast<unsigned*>(take(sizeof(unsigned) * a.nwords));
   s.win = reinterpret_cast<float*>(take(sizeof(float) * wn));
   s.mx0 = reinterpret_cast<float*>(take(sizeof(float) * wn));
   s.mx1 = reinterpret_cast<float*>(take(sizeof(float) * wn));
@@ -206,9 +236,8 @@ __device__ __forceinline__ Smem carve_smem(const PeelArgs& a, char* base, bool g
   s.tl_k = reinterpret_cast<int*>(take(sizeof(int) * kWarps * kTouch));
   s.tl_amp = reinterpret_cast<float*>(take(sizeof(float) * kWarps * kTouch));
   s.eb = reinterpret_cast<unsigned char*>(take(kWarps * kTouch * 32));
-  s.stage = grouped ? reinterpret_cast<float*>(take(sizeof(float) * kWarps * 2 * kGroup * 32))
-                    : nullptr;
-  s.rtab = grouped ? reinterpret_cast<float2*>(take(sizeof(float2) * kWarps * kGroup)) : nullptr;
+  s.stage = grouped ? reinterpret_cast<float*>(take(kWarps * kTileBytes)) : nullptr;
+  s.unit = grouped ? reinterpret_cast<UnitIn*>(take(kWarps * kUnitBytes)) : nullptr;
   return s;
 }
 
@@ -217,11 +246,11 @@ size_t smem_bytes(int P, int nt, int nchunks, int nwords, bool grouped) {
   const size_t wn = kChunk + 2 * (size_t)nt;
   (void)P;
   return r(sizeof(float) * 8 * nt) + r(sizeof(int) * (nchunks + 1)) +
-         r(sizeof(int) * (nwords + 1)) + 3 * r(sizeof(float) * wn) +
+         r(sizeof(int) * (nwords + 1)) + r(sizeof(unsigned) * nwords) +
+         3 * r(sizeof(float) * wn) +
          r(sizeof(int) * kChunk) + r(sizeof(int) * (kWarps + 1)) +
          3 * r(sizeof(int) * kWarps * kTouch) + r(kWarps * kTouch * 32) +
-         (grouped ? r(sizeof(float) * kWarps * 2 * kGroup * 32) + r(sizeof(float2) * kWarps * kGroup)
-                  : 0);
+         (grouped ? r(kWarps * kTileBytes) + r(kWarps * kUnitBytes) : 0);
 }
 
 __device__ __forceinline__ unsigned long long pack_score(float cf, int j) {
@@ -255,6 +284,11 @@ __device__ __forceinline__ void fold_score(float b, float2 nmi, int j, float& be
 
 __device__ __forceinline__ const float* bt_row(const PeelArgs& a, int blk, int j) {
   return a.Bt + ((size_t)blk * a.K + j) * kCol;
+}
+
+// A warp's tile.
+__device__ __forceinline__ float* unit_tile(const Smem& s, int warp) {
+  return s.stage + (size_t)warp * (kTileBytes / 4);
 }
 
 // ---------------------------------------------------------------- DETECT
@@ -374,6 +408,141 @@ __device__ void detect_chunk(const PeelArgs& a, const Smem& s, int ch, int it) {
   __syncthreads();
 }
 
+// detect_chunk by one warp in its tile, so that a team's chunks proceed side by
+// side instead of one per block and latency chain.  The columns whose blocks
+// were rescored come from pack[q], the others from cfmax (one load each); a
+// chunk without a rescored block within +-nt has no peak.
+//
+// What bounds it: the latency of its few dependent loads and atomics.
+__device__ void detect_chunk_warp(const PeelArgs& a, float* tile, int ch, int it, int lane) {
+  const int nt = a.nt, L = a.L;
+  const int p = it & 1, q = p ^ 1;
+  const int a0 = ch * kChunk, a1 = min(a0 + kChunk, L);
+  const int wn = kChunk + 2 * nt;
+  const unsigned long long* pprev = a.pack + (size_t)q * L;
+  // rescored blocks among those within +-nt (at most 13: nt <= 64)
+  const int bb0 = max(a0 - nt, 0) / kCol, bb1 = min(a1 - 1 + nt, L - 1) / kCol;
+  unsigned fresh = 0xffffffffu;
+  if (it > 0) {
+    const bool f = bb0 + lane <= bb1 && a.tcount[(size_t)q * a.nblk + bb0 + lane] > 0;
+    fresh = __ballot_sync(0xffffffffu, f);
+    if (!fresh) {
+      if (lane == 0) a.chunk_cnt[ch] = 0;
+      return;
+    }
+  }
+  float* w0 = tile;
+  float* w1 = tile + wn;
+  int* kidx = reinterpret_cast<int*>(tile + 2 * wn);
+  __syncwarp();                         // the tile's earlier readers are done
+  for (int i0 = 0; i0 < wn; i0 += 128) {
+    unsigned long long pv[4];
+    float cv[4];
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+      const int i = i0 + 32 * h + lane, col = a0 - nt + i;
+      const bool in = i < wn && col >= nt && col < L - nt;
+      const bool fr = in && ((fresh >> (col / kCol - bb0)) & 1u);
+      pv[h] = fr ? pprev[col] : 0ull;
+      cv[h] = in && !fr ? a.cfmax[col] : 0.f;
+    }
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+      const int i = i0 + 32 * h + lane, col = a0 - nt + i;
+      if (i >= wn) continue;
+      const bool in = col >= nt && col < L - nt;
+      const bool fr = in && ((fresh >> (col / kCol - bb0)) & 1u);
+      const float v = col < 0 || col >= L ? -INFINITY : (fr ? pack_value(pv[h]) : cv[h]);
+      w0[i] = v;
+      if (i >= nt && i < nt + kChunk) {
+        kidx[i - nt] = fr ? pack_index(pv[h]) : -1;
+        if (fr) {
+          a.cfmax[col] = v;
+          a.imax[col] = pack_index(pv[h]);
+        }
+      }
+    }
+  }
+  __syncwarp();
+  const int len = 2 * nt + 1;
+  // the chunk's own scores leave the window before the levels overwrite it
+  float own[kChunk / 32];
+#pragma unroll
+  for (int h = 0; h < kChunk / 32; ++h) own[h] = w0[nt + 32 * h + lane];
+  int m = 1;
+  float* src = w0;
+  float* dst = w1;
+  while (2 * m <= len) {
+    for (int i = lane; i + 2 * m <= wn; i += 32) dst[i] = fmaxf(src[i], src[i + m]);
+    __syncwarp();
+    m *= 2;
+    float* t = src;
+    src = dst;
+    dst = t;
+  }
+  // peaks in time order: their columns to the free buffer
+  int* list = reinterpret_cast<int*>(dst);
+  int total = 0;
+#pragma unroll
+  for (int h = 0; h < kChunk / 32; ++h) {
+    const int i = 32 * h + lane, tau = a0 + i;
+    bool pk = false;
+    if (tau < a1 && tau >= nt && tau < L - nt) {
+      const float pooled = fmaxf(src[i], src[i + len - m]);
+      pk = (pooled > a.th2) && (fabsf(__fsub_rn(pooled, own[h])) < 1e-9f);
+    }
+    const unsigned bal = __ballot_sync(0xffffffffu, pk);
+    if (pk) list[total + __popc(bal & ((1u << lane) - 1u))] = i;
+    total += __popc(bal);
+  }
+  __syncwarp();
+  int* tcur = a.tcount + (size_t)p * a.nblk;
+  Touch* tch = a.touch + (size_t)p * a.nblk * kTouch;
+  unsigned* bits = a.dbits + (size_t)p * a.nwords;
+  unsigned long long* pcur = a.pack + (size_t)p * L;
+  for (int e0 = 0; e0 < total; e0 += 32) {
+    const int e = e0 + lane;
+    const bool have = e < total;
+    int tau = 0, k = 0;
+    float amp = 0.f;
+    const int slot = ch * kChunk + e;
+    if (have) {
+      const int i = list[e];
+      tau = a0 + i;
+      k = kidx[i];
+      if (k < 0) k = a.imax[tau];
+      amp = __fdiv_rn(bt_row(a, tau / kCol, k)[tau % kCol], a.nm[k]);
+      a.chunk_tau[slot] = tau;
+      a.chunk_k[slot] = k;
+      a.chunk_amp[slot] = amp;
+      a.chunk_th[slot] = __fsqrt_rn(fmaxf(src[i], src[i + len - m]));
+    }
+    const int b0 = (tau - nt) / kCol, b1 = have ? (tau + nt) / kCol : b0 - 1;
+    const int nb = (2 * nt) / kCol + 2;               // blocks a peak can touch
+    for (int o = 0; o < nb; o += 8) {
+      int pos[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        pos[i] = (b0 + o + i <= b1) ? atomicAdd(&tcur[b0 + o + i], 1) : -1;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int b = b0 + o + i;
+        if (pos[i] == 0) atomicOr(&bits[b >> 5], 1u << (b & 31));
+        if (pos[i] >= 0) {
+          if (pos[i] < kTouch) tch[(size_t)b * kTouch + pos[i]] = Touch{tau, k, amp, slot};
+          else atomicCAS(a.err, 0, KS_ERR_DEGENERATE);
+        }
+        // a block's first registration clears its rescoring slots
+        for (unsigned f = __ballot_sync(0xffffffffu, pos[i] == 0); f; f &= f - 1u) {
+          const int c = __shfl_sync(0xffffffffu, b, __ffs(f) - 1) * kCol + lane;
+          if (c < L) pcur[c] = 0ull;
+        }
+      }
+    }
+  }
+  if (lane == 0) a.chunk_cnt[ch] = total;
+}
+
 // Both exclusive prefixes an iteration needs, in one pass: of the chunk peak
 // counts into s.prefix[0..nchunks] and of the dirty-bitmap word popcounts into
 // s.wprefix[0..nwords].  All threads of the block take part.
@@ -418,7 +587,12 @@ __device__ void two_prefix(const int* cnt, int nchunks, const unsigned* bits, in
   }
   for (int i = 0; i < pw; ++i) {
     const int w = tid * pw + i;
-    if (w < nwords) { s.wprefix[w] = rw; rw += __popc(bits[w]); }
+    if (w < nwords) {
+      const unsigned v = bits[w];
+      s.dw[w] = v;
+      s.wprefix[w] = rw;
+      rw += __popc(v);
+    }
   }
   if (tid == 0) { s.prefix[nchunks] = wc[kWarps]; s.wprefix[nwords] = ww[kWarps]; }
   __syncthreads();
@@ -437,16 +611,25 @@ struct TouchList {
   const float* amp;
 };
 
-__device__ __forceinline__ TouchList load_touch_warp(const PeelArgs& a, const Smem& s,
-                                                     int p, int blk, int lane, int warp) {
-  Touch t{0, 0, 0.f, 0};
-  if (lane < kTouch) t = a.touch[((size_t)p * a.nblk + blk) * kTouch + lane];
-  int n = a.tcount[(size_t)p * a.nblk + blk];
-  n = min(n, kTouch);
+// The lane's registration of block blk (lanes below kTouch) and their number.
+struct TouchWord {
+  Touch t;
+  int n;
+};
+__device__ __forceinline__ TouchWord touch_word(const PeelArgs& a, int p, int blk, int lane) {
+  TouchWord w{Touch{0, 0, 0.f, 0}, 0};
+  if (lane < kTouch) w.t = a.touch[((size_t)p * a.nblk + blk) * kTouch + lane];
+  w.n = a.tcount[(size_t)p * a.nblk + blk];
+  return w;
+}
+
+__device__ __forceinline__ TouchList order_touch_warp(const Smem& s, const TouchWord& w, int lane,
+                                                      int warp) {
+  const int n = min(w.n, kTouch);
   int key = 0x7fffffff;
   if (lane < n) {
-    const int ch = t.slot / kChunk;
-    const int g = s.prefix[ch] + (t.slot - ch * kChunk);
+    const int ch = w.t.slot / kChunk;
+    const int g = s.prefix[ch] + (w.t.slot - ch * kChunk);
     key = ((g & 1) << 30) | g;
   }
   int rank = 0;
@@ -459,12 +642,17 @@ __device__ __forceinline__ TouchList load_touch_warp(const PeelArgs& a, const Sm
   float* amp = s.tl_amp + warp * kTouch;
   __syncwarp();
   if (lane < n) {
-    tau[rank] = t.tau;
-    kk[rank] = t.k;
-    amp[rank] = t.amp;
+    tau[rank] = w.t.tau;
+    kk[rank] = w.t.k;
+    amp[rank] = w.t.amp;
   }
   __syncwarp();
   return TouchList{n, tau, kk, amp};
+}
+
+__device__ __forceinline__ TouchList load_touch_warp(const PeelArgs& a, const Smem& s,
+                                                     int p, int blk, int lane, int warp) {
+  return order_touch_warp(s, touch_word(a, p, blk, lane), lane, warp);
 }
 
 // Columns of block blk x template rows [j_lo, j_hi): subtract the touching
@@ -560,13 +748,9 @@ __device__ __forceinline__ int bound_expo(float b) {
   return (int)((__float_as_uint(b) >> 23) & 0xffu);
 }
 
-// cp.async global -> shared: 4 bytes (L1-allocating) and 16 bytes (L2 only),
-// and the wait for this thread's copies.
-__device__ __forceinline__ void cp_async4(float* dst, const float* src) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async16(float* dst, const float* src) {
+// cp.async global -> shared of 16 bytes (L2 only), and the wait for this
+// thread's copies.
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
 }
@@ -575,6 +759,37 @@ __device__ __forceinline__ void cp_async_commit() {
 }
 __device__ __forceinline__ void cp_async_wait_all() {
   asm volatile("cp.async.wait_group 0;" ::: "memory");
+}
+
+// Two packed FP32 operations per instruction (each half rounds as the scalar
+// operation does).
+__device__ __forceinline__ unsigned long long f2_pack(float lo, float hi) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void f2_unpack(unsigned long long v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ unsigned long long f2_fma(unsigned long long a, unsigned long long b,
+                                                     unsigned long long c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ unsigned long long f2_mul(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+// a + fl(x y), the product and the sum rounded separately.  The sum is a fused
+// operation with a factor of one that the compiler cannot see (PeelArgs::one):
+// a packed product followed by a packed sum was contracted into one rounding.
+__device__ __forceinline__ unsigned long long f2_add_prod(unsigned long long a,
+                                                          unsigned long long x,
+                                                          unsigned long long y,
+                                                          unsigned long long one2) {
+  return f2_fma(one2, f2_mul(x, y), a);
 }
 
 // ----------------------------------------------------------- grouped update
@@ -603,11 +818,10 @@ __device__ __forceinline__ void cp_async_wait_all() {
 //
 // An iteration's update runs in two phases separated by a team barrier, so
 // that the uneven work (a dirty block needs anywhere from none to all of its
-// groups) is spread evenly: group_scan_block (one warp per dirty block) reads
+// groups) is spread evenly: group_scan (one warp per dirty block) reads
 // only metadata, folds the cached bests of the groups its columns leave
 // alone into the column maxima and appends each group that some column must
-// process to the iteration's unit list; unit_run (units taken from a
-// counter) processes one such group tile.
+// process to the iteration's unit list; run_units processes one such group tile.
 
 // Per-lane view of an ordered touch list: the first entry touching this
 // column (-1: none) and the mask of the others.
@@ -628,455 +842,515 @@ __device__ __forceinline__ LaneEntries lane_entries(const TouchList& tl, int c, 
   return le;
 }
 
-// One group tile (group g of block blk): when some column of the warp has nd
-// set, the warp stages the group's 32 rows of B (whole rows, 16-byte copies)
-// and every nd column stages its first touching peak's cross-correlations,
-// into the warp's shared tiles with cp.async (one round trip, no registers
-// held in flight); the columns subtract their touching peaks in application
-// order (further peaks stage their cross-correlations into the same tile),
-// write the rows back when `store`, and rewrite the group's gbest and gexp.
-// jl / nl: row index and {nm, 1/nm} of group position `lane` (rperm, nmip).
-// Returns the group's packed best for nd columns (0 otherwise).  Called by
-// the whole warp.
-//
-// The best over the group's rows is found without a division per row: with
-// approx = fl(sq * fl(1/nm)) within a relative 2^-22 of the exact quotient
-// cf = fl(sq / nm) (sq and the quotient normal), a row whose approx is below
-// (1 - 2^-20) times the largest approx m of the group cannot reach the exact
-// quotient of the row holding m, so only the rows at or above that level
-// have their exact quotient computed and folded (larger score, then the
-// smaller template index); rows with sq = 0 and a normal nm have the
-// quotient +0 exactly, and rows whose approx is NaN or tiny are folded
-// exactly too.
-// kLazy selects the lean form of that fold (the batched launch): the same
-// result with fewer instructions per row, the rare cases (zero scores, NaN or
-// tiny approximations) found by second passes that run only when needed.
-template <bool kLazy>
-__device__ unsigned long long group_tile(const PeelArgs& a, const Smem& s, const TouchList& tl,
-                                         int blk, int g, bool nd, const LaneEntries& le,
-                                         bool store, int jl, float2 nl, int lane, int warp) {
-  const int c = blk * kCol + lane;
-  const int nt = a.nt, K = a.K, nlag = 2 * nt + 1;
-  const int nrow = min(kGroup, K - g * kGroup);
-  float* Bs = s.stage + (size_t)warp * (2 * kGroup * 32);
-  float* Cs = Bs + kGroup * 32;
-  float2* rtab = s.rtab + warp * kGroup;
-  const float* brow = a.Bt + (size_t)blk * K * kCol;
-  const float* cp0 = a.ctcT;
-  float amp0 = 0.f;
-  if (le.e0 >= 0) {
-    cp0 = a.ctcT + (size_t)tl.k[le.e0] * K * nlag + (c - tl.tau[le.e0] + nt);
-    amp0 = tl.amp[le.e0];
-  }
-  const bool any_nd = __any_sync(0xffffffffu, nd);
-  const unsigned rest_any = __reduce_or_sync(0xffffffffu, nd ? le.rest : 0u);
-  __syncwarp();                       // earlier readers of the tiles are done
-  if (lane < nrow) rtab[lane] = make_float2(__int_as_float(jl), nl.x);
-  // whole rows of B: lane copies 16 bytes (4 columns) of rows 4i + lane/8
-#pragma unroll
-  for (int i = 0; i < kGroup / 4; ++i) {
-    const int r = 4 * i + (lane >> 3);
-    const int j = __shfl_sync(0xffffffffu, jl, r);
-    if (any_nd && r < nrow)
-      cp_async16(Bs + r * 32 + (lane & 7) * 4, brow + (size_t)j * kCol + (lane & 7) * 4);
-  }
-  for (int r = 0; r < nrow; ++r) {
-    const int j = __shfl_sync(0xffffffffu, jl, r);
-    if (nd && le.e0 >= 0) cp_async4(Cs + r * 32 + lane, cp0 + (size_t)j * nlag);
+// Inputs of a unit (a group tile that some columns of a block must process)
+// in shared memory: the block's ordered touch list as the scan published it,
+// the group's row indices and {nm, 1/sqrt(nm)}.  The tables are padded to whole
+// groups with copies of the last template, whose rows are then read, updated
+// and written with the same values more than once and fold to the same best.
+struct UnitIn {
+  int list[32];        // n, tau[kTouch], k[kTouch], amp bits[kTouch]
+  int row[kGroup];
+  float2 nm[kGroup];
+};
+constexpr int kUnitSlots = 2;
+static_assert(sizeof(UnitIn) * kUnitSlots == kUnitBytes && sizeof(UnitIn) == 512 && 1 + 3 * kTouch <= 32, "one 16-byte piece per lane");
+
+__device__ __forceinline__ UnitIn* unit_in(const Smem& s, int warp, int i) {
+  return s.unit + warp * kUnitSlots + i % kUnitSlots;
+}
+
+// Request unit u's inputs (cp.async, a 16-byte piece per lane).
+template <bool kInit>
+__device__ __forceinline__ void unit_fetch(const PeelArgs& a, uint2 u, UnitIn* in, int lane) {
+  const char* src;
+  if (lane < 8) src = reinterpret_cast<const char*>(a.blist + (size_t)(u.x >> 11) * 32) + lane * 16;
+  else if (lane < 16) src = reinterpret_cast<const char*>(a.rperm + (u.x & 2047u) * kGroup) + (lane - 8) * 16;
+  else src = reinterpret_cast<const char*>(a.nmip + (u.x & 2047u) * kGroup) + (lane - 16) * 16;
+  if (!kInit || lane >= 8) cp_async16(reinterpret_cast<char*>(in) + lane * 16, src);
+  cp_async_commit();
+}
+
+// min(m, |x|, |y|), NaN when any of them is; max(m, x, y), NaNs passed over.
+__device__ __forceinline__ float min_abs_nan(float m, float x, float y) {
+  float r;
+  asm("min.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(m), "f"(fabsf(x)), "f"(fabsf(y)));
+  return r;
+}
+// All ones where x >= y, else 0 (also for NaN).
+__device__ __forceinline__ unsigned mask_ge(float x, float y) {
+  unsigned r;
+  asm("set.ge.u32.f32 %0, %1, %2;" : "=r"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ float max3(float m, float x, float y) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(m), "f"(x), "f"(y));
+  return r;
+}
+
+// The columns of a group tile a lane reads, and the one it owns: lane
+// (rq, cq) = (lane / 8, lane % 8) holds rows 4i + rq and columns 4cq .. 4cq+3
+// of the 32 x 32 tile, and owns column 4cq + rq.
+__device__ __forceinline__ int own_column(int lane) { return 4 * (lane & 7) + (lane >> 3); }
+
+// Stage, for the columns with `mine`, the cross-correlations of one peak (cp:
+// row 0 of its slab at this lane's column) with the group's rows into a tile;
+// the other columns get zeros.
+__device__ __forceinline__ void stage_ctc(float* Cs, const float* cp, bool mine, const int* row,
+                                          int nlag, int lane) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(Cs + lane);
+  const int bytes = mine ? 4 : 0;
+#pragma unroll 2
+  for (int r = 0; r < kGroup; r += 4) {
+    const int4 j = *reinterpret_cast<const int4*>(row + r);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d + r * 128), "l"(cp + (unsigned)(j.x * nlag)), "r"(bytes) : "memory");
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d + r * 128 + 128), "l"(cp + (unsigned)(j.y * nlag)), "r"(bytes) : "memory");
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d + r * 128 + 256), "l"(cp + (unsigned)(j.z * nlag)), "r"(bytes) : "memory");
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d + r * 128 + 384), "l"(cp + (unsigned)(j.w * nlag)), "r"(bytes) : "memory");
   }
   cp_async_commit();
-  cp_async_wait_all();
-  __syncwarp();                       // every lane's rows of B have landed
-  // a column touched by further peaks applies them here in application
-  // order; otherwise its single peak is applied in the first pass below
-  const bool fused = rest_any == 0u;
-  if (!fused) {
-    if (nd && le.e0 >= 0) {
-      for (int r = 0; r < nrow; ++r)
-        Bs[r * 32 + lane] = __fsub_rn(Bs[r * 32 + lane], __fmul_rn(amp0, Cs[r * 32 + lane]));
-    }
-    for (unsigned m = rest_any; m; m &= m - 1u) {
-      const int e = __ffs(m) - 1;
-      const bool mine = nd && ((le.rest >> e) & 1u);
-      const float* cp = a.ctcT + (size_t)tl.k[e] * K * nlag + (c - tl.tau[e] + nt);
-      for (int r = 0; r < nrow; ++r) {
-        const int j = __shfl_sync(0xffffffffu, jl, r);
-        if (mine) cp_async4(Cs + r * 32 + lane, cp + (size_t)j * nlag);
+}
+
+// b += (-amp) * c over the lane's 8 x 4 elements: the product and the sum are
+// rounded separately, b - fl(amp c).  A column that takes no part has
+// n = -0 and c = +0: b + (-0) = b exactly.
+__device__ __forceinline__ void apply_ctc(const float* Cs, unsigned long long n01,
+                                          unsigned long long n23, unsigned long long one2,
+                                          unsigned long long (&b)[8][2], int lane) {
+  const float* c = Cs + (lane >> 3) * 32 + (lane & 7) * 4;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(c + i * 128);
+    b[i][0] = f2_add_prod(b[i][0], n01, v.x, one2);
+    b[i][1] = f2_add_prod(b[i][1], n23, v.y, one2);
+  }
+}
+
+// The four columns' values of a per-column quantity, packed in pairs.
+__device__ __forceinline__ void column_pairs(float v, int lane, unsigned long long& p01,
+                                             unsigned long long& p23) {
+  const int c = 4 * (lane & 7);
+  const float v0 = __shfl_sync(0xffffffffu, v, c), v1 = __shfl_sync(0xffffffffu, v, c + 1);
+  const float v2 = __shfl_sync(0xffffffffu, v, c + 2), v3 = __shfl_sync(0xffffffffu, v, c + 3);
+  p01 = f2_pack(v0, v1);
+  p23 = f2_pack(v2, v3);
+}
+
+// This lane's column's address in the slab of entry e's template.
+__device__ __forceinline__ const float* entry_slab(const PeelArgs& a, const UnitIn* in, int e, int c) {
+  return a.ctcT + (size_t)in->list[1 + kTouch + e] * a.K * (2 * a.nt + 1) +
+         (c - in->list[1 + e] + a.nt);
+}
+
+// Start of a unit whose inputs have landed: every column in `cols` stages its
+// first touching peak's cross-correlations (not waited for).  Returns the
+// lane's column's entries.
+__device__ __forceinline__ LaneEntries unit_begin(const PeelArgs& a, const UnitIn* in, uint2 u,
+                                                  float* Cs, int lane) {
+  const int c = (int)(u.x >> 11) * kCol + lane;
+  LaneEntries le{-1, 0u};
+  if ((u.y >> lane) & 1u) {
+    const int n = in->list[0];
+    for (int e = 0; e < n; ++e) {
+      const int d = c - in->list[1 + e];
+      if (c < a.L && d >= -a.nt && d <= a.nt) {
+        if (le.e0 < 0) le.e0 = e;
+        else le.rest |= 1u << e;
       }
-      cp_async_commit();
-      cp_async_wait_all();
-      if (mine) {
-        const float amp = tl.amp[e];
-        for (int r = 0; r < nrow; ++r)
-          Bs[r * 32 + lane] = __fsub_rn(Bs[r * 32 + lane], __fmul_rn(amp, Cs[r * 32 + lane]));
-      }
     }
   }
-  float best = -1.f;
-  int arg = 0x7fffffff;
-  int emin = 255;                             // smallest exponent field over the rows
-  if constexpr (!kLazy) {
-  // pass 1, branch-free over all kGroup rows (rows past nrow and columns
-  // without nd only compute, their results unused): the (single peak)
-  // subtraction, the write-back, the smallest exponent, and for the best
-  // score the largest approx m with its first row rm, the largest approx m2
-  // of the other rows, the smallest row index whose score is exactly 0
-  // (sq = 0 and a normal nm), and the rows that need an exact quotient
-  // whatever m is (approx NaN, or below 2^-100 with sq > 0).
-  float* bdst = a.Bt + (size_t)blk * K * kCol + lane;
-  const bool sub = fused && le.e0 >= 0;
-  constexpr float kTiny = 7.8886091e-31f;     // 2^-100
-  float m = -1.f, m2 = -1.f;
-  int rm = -1, jz = 0x7fffffff;
-  unsigned spec = 0u;
-#pragma unroll 8
-  for (int r = 0; r < kGroup; ++r) {
-    const int j = __shfl_sync(0xffffffffu, jl, r);
-    const float nmy = __shfl_sync(0xffffffffu, nl.y, r);
-    const bool ok = nd && r < nrow;
-    const float b0 = Bs[r * 32 + lane];
-    const float b1 = __fsub_rn(b0, __fmul_rn(amp0, Cs[r * 32 + lane]));
-    const float b = sub ? b1 : b0;
-    if (ok && store) bdst[(size_t)j * kCol] = b;
-    emin = ok ? min(emin, noop_expo(b)) : emin;
-    const float rl = b > 0.f ? b : 0.f;
-    const float sq = __fmul_rn(rl, rl);
-    const float ap = __fmul_rn(sq, nmy);
-    const bool big = ok && ap >= kTiny;
-    const bool top = big && ap > m;
-    m2 = top ? m : (big ? fmaxf(m2, ap) : m2);
-    rm = top ? r : rm;
-    m = top ? ap : m;
-    jz = (ok && sq == 0.f && nmy == nmy && j < jz) ? j : jz;
-    spec |= (ok && (ap != ap || (ap < kTiny && sq != 0.f))) ? (1u << r) : 0u;
+  __syncwarp();
+  const bool first = le.e0 >= 0;
+  stage_ctc(Cs, first ? entry_slab(a, in, le.e0, c) : a.ctcT, first, in->row, 2 * a.nt + 1, lane);
+  return le;
+}
+
+// The unit's 32 rows x 32 columns of B, whole rows as 16-byte pieces: a lane
+// holds 8 rows x 4 columns.
+__device__ __forceinline__ void unit_rows(const PeelArgs& a, const UnitIn* in, uint2 u,
+                                          unsigned long long (&b)[8][2], int lane) {
+  const int* row = in->row + (lane >> 3);
+  const float* brow = a.Bt + (size_t)(u.x >> 11) * a.K * kCol + (lane & 7) * 4;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(brow + (unsigned)row[4 * i] * kCol);
+    b[i][0] = v.x;
+    b[i][1] = v.y;
   }
-  // Candidates for the best: with m >= 2^-90 the rows whose approx is at
-  // least (1 - 2^-20) m -- only rm, unless m2 reaches that level; below
-  // 2^-90 every row with approx >= 2^-100.  Rows with a smaller approx
-  // cannot reach the exact quotient of rm (or 2^-100 and the zeros), so the
-  // result is that of folding every row.
-  const bool regime_a = m >= 8.0779356e-28f;  // 2^-90
-  const float thr = regime_a ? m * 0.99999905f : kTiny;
-  const bool scan = !regime_a || m2 >= thr;
-  if (jz != 0x7fffffff) {
-    best = 0.f;
-    arg = jz;
-  }
-  unsigned cand = spec;
-  if (regime_a && !scan) cand |= 1u << rm;
-  if (__any_sync(0xffffffffu, nd && scan)) {
-#pragma unroll 8
-    for (int r = 0; r < kGroup; ++r) {
-      const float nmy = __shfl_sync(0xffffffffu, nl.y, r);
-      const bool ok = nd && scan && r < nrow;
-      const float b0 = Bs[r * 32 + lane];
-      const float b1 = __fsub_rn(b0, __fmul_rn(amp0, Cs[r * 32 + lane]));
-      const float b = sub ? b1 : b0;
-      const float rl = b > 0.f ? b : 0.f;
-      const float ap = __fmul_rn(__fmul_rn(rl, rl), nmy);
-      cand |= (ok && ap >= thr) ? (1u << r) : 0u;
+}
+
+// The scores of a unit's updated rows (b, and kept in the slot's tile): the
+// smallest magnitude e0, the largest t and the candidate rows of the lane's
+// own column (own_column), found in two passes over the lane's 8 x 4 elements;
+// unit_fold then folds the candidates.
+//
+// The best over the group's rows is found without a division per row.  With
+// t = fl(b * fl(1/sqrt(nm))), nm in [2^-30, 2^30], t is within a relative
+// 2^-23 of b/sqrt(nm), so for t in [2^-45, 2^60] (b^2 and the quotient then
+// normal) the exactly rounded scores cf = fl(fl(b^2) / nm) of two rows are
+// ordered as their t wherever those differ by more than a relative 2^-21: only
+// rows with t >= (1 - 2^-20) max t can hold the best, and only their quotients
+// are computed and folded (larger score, then the smaller template index).
+// When no t is above 0 every row's score is +0 exactly (NaN scores count as 0,
+// as relu of a failed comparison), and the smallest template index wins.  A
+// largest t outside that interval, or a group with an nm outside its range
+// (marked by a NaN scale), folds every row's quotient.
+//
+// What bounds it: the L1 and L2 traffic of the unit's rows (about 14 KB) and
+// the instructions around it.  Four columns per lane make one 16-byte access, one
+// row index and one scale serve four elements, and the products, differences
+// and scores run two per packed FP32 instruction; the form with one column per
+// lane and a division-free fold of larger state took about three times the
+// instructions (peel of a C=384, K=600 batch 2.40 -> 1.70 ms, of 16 such
+// batches by 16 teams 21.6 -> 14.0 ms, with the scan and detection below).
+// Measured and dropped: the next unit's rows and cross-correlations requested
+// a unit ahead (registers and a second tile: 6.5-7.5 ms of units in the
+// 16-batch launch against 6.2), loads past L1, cross-correlations through
+// registers instead of cp.async, more or fewer warps per SM at equal tiles.
+struct UnitScore {
+  float e0;        // smallest |b| (NaN if any is)
+  float mo;        // largest t
+  unsigned rows;   // bit 8k + i: row 4i + k is a candidate
+};
+
+// b becomes t.
+__device__ __forceinline__ UnitScore unit_score(const UnitIn* in, unsigned long long (&b)[8][2],
+                                                int lane) {
+  const int rq = lane >> 3;
+  float ea[4] = {INFINITY, INFINITY, INFINITY, INFINITY};
+  float m[4] = {-1.f, -1.f, -1.f, -1.f};
+#pragma unroll
+  for (int i = 0; i < 8; i += 2) {
+    const float sa = in->nm[4 * i + rq].y, sb = in->nm[4 * i + 4 + rq].y;
+    const unsigned long long s2 = f2_pack(sa, sa), s3 = f2_pack(sb, sb);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      float x0, x1, y0, y1, t0, t1, u0, u1;
+      f2_unpack(b[i][h], x0, x1);
+      f2_unpack(b[i + 1][h], y0, y1);
+      ea[2 * h] = min_abs_nan(ea[2 * h], x0, y0);
+      ea[2 * h + 1] = min_abs_nan(ea[2 * h + 1], x1, y1);
+      b[i][h] = f2_mul(b[i][h], s2);
+      b[i + 1][h] = f2_mul(b[i + 1][h], s3);
+      f2_unpack(b[i][h], t0, t1);
+      f2_unpack(b[i + 1][h], u0, u1);
+      m[2 * h] = max3(m[2 * h], t0, u0);
+      m[2 * h + 1] = max3(m[2 * h + 1], t1, u1);
     }
   }
-  // exact quotients of the candidates (usually only rm, converged)
-  if (!nd) cand = 0u;
-  for (unsigned mm = cand; mm; mm &= mm - 1u) {
-    const int r = __ffs(mm) - 1;
-    float b = Bs[r * 32 + lane];
-    if (sub) b = __fsub_rn(b, __fmul_rn(amp0, Cs[r * 32 + lane]));
-    const float2 jn = rtab[r];
-    const int j = __float_as_int(jn.x);
-    const float rl = b > 0.f ? b : 0.f;
-    const float sq = __fmul_rn(rl, rl);
-    const bool normal = jn.y >= 1.17549435e-38f && jn.y <= 3.40282347e38f;
-    const float cf = (sq == 0.f && normal) ? 0.f : __fdiv_rn(sq, jn.y);
-    if (cf > best || (cf == best && j < arg)) {
-      best = cf;
-      arg = j;
-    }
-  }
-  } else {
-  // pass 1 over the group's rows, branch-free in the columns (a column
-  // without nd computes too, its results unused): the (single peak)
-  // subtraction, the write-back, the smallest exponent, and for the best
-  // score the largest approx m with its first row rm and the largest approx
-  // m2 of the other rows.  Rows with an approx below 2^-100 take part in m
-  // and m2 without changing what follows (the candidate level is at least
-  // 2^-90 when m is, and below it every row >= 2^-100 is a candidate), NaN
-  // approx never does.  Rows that need an exact quotient whatever m is
-  // (approx NaN, or below 2^-100 with sq > 0) only raise a flag here and are
-  // found by a second pass when some column has one.
-  float* bdst = a.Bt + (size_t)blk * K * kCol + lane;
-  const bool sub = fused && le.e0 >= 0;
-  constexpr float kTiny = 7.8886091e-31f;     // 2^-100
-  float m = -1.f, m2 = -1.f;
-  int rm = -1;
-  bool anyspec = false;
-#pragma unroll 8
-  for (int r = 0; r < nrow; ++r) {
-    const int j = __shfl_sync(0xffffffffu, jl, r);
-    const float nmy = __shfl_sync(0xffffffffu, nl.y, r);
-    const float b0 = Bs[r * 32 + lane];
-    const float b1 = __fsub_rn(b0, __fmul_rn(amp0, Cs[r * 32 + lane]));
-    const float b = sub ? b1 : b0;
-    if (nd && store) bdst[(size_t)j * kCol] = b;
-    emin = min(emin, noop_expo(b));
-    const float rl = b > 0.f ? b : 0.f;
-    const float sq = __fmul_rn(rl, rl);
-    const float ap = __fmul_rn(sq, nmy);
-    const bool top = ap > m;
-    m2 = top ? m : fmaxf(m2, ap);
-    rm = top ? r : rm;
-    m = top ? ap : m;
-    anyspec |= (ap != ap) || (ap < kTiny && sq != 0.f);
-  }
-  // Candidates for the best: with m >= 2^-90 the rows whose approx is at
-  // least (1 - 2^-20) m -- only rm, unless m2 reaches that level; below
-  // 2^-90 every row with approx >= 2^-100.  Rows with a smaller approx
-  // cannot reach the exact quotient of rm (or 2^-100 and the zeros), so the
-  // result is that of folding every row.
-  const bool regime_a = m >= 8.0779356e-28f;  // 2^-90
-  const float thr = regime_a ? m * 0.99999905f : kTiny;
-  const bool scan = !regime_a || m2 >= thr;
+#pragma unroll
+  for (int o = 8; o <= 16; o <<= 1)
+#pragma unroll
+    for (int h = 0; h < 4; ++h) m[h] = fmaxf(m[h], __shfl_xor_sync(0xffffffffu, m[h], o));
+  // candidate rows: bit i of byte h stands for row 4i + rq of column 4cq + h
   unsigned cand = 0u;
-  if (regime_a && !scan) cand |= 1u << rm;
-  if (__any_sync(0xffffffffu, nd && (scan || anyspec))) {
-#pragma unroll 8
-    for (int r = 0; r < nrow; ++r) {
-      const float nmy = __shfl_sync(0xffffffffu, nl.y, r);
-      const float b0 = Bs[r * 32 + lane];
-      const float b1 = __fsub_rn(b0, __fmul_rn(amp0, Cs[r * 32 + lane]));
-      const float b = sub ? b1 : b0;
-      const float rl = b > 0.f ? b : 0.f;
-      const float sq = __fmul_rn(rl, rl);
-      const float ap = __fmul_rn(sq, nmy);
-      const bool sp = ap != ap || (ap < kTiny && sq != 0.f);
-      cand |= ((scan && ap >= thr) || sp) ? (1u << r) : 0u;
+  {
+    float thr[4];
+#pragma unroll
+    for (int h = 0; h < 4; ++h) thr[h] = m[h] > 0.f ? m[h] * 0.99999905f : INFINITY;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        float t0, t1;
+        f2_unpack(b[i][h], t0, t1);
+        cand |= mask_ge(t0, thr[2 * h]) & (1u << (8 * (2 * h) + i));
+        cand |= mask_ge(t1, thr[2 * h + 1]) & (1u << (8 * (2 * h + 1) + i));
+      }
     }
   }
-  // exact quotients of the candidates (usually only rm, converged)
-  if (!nd) cand = 0u;
-  for (unsigned mm = cand; mm; mm &= mm - 1u) {
-    const int r = __ffs(mm) - 1;
-    float b = Bs[r * 32 + lane];
-    if (sub) b = __fsub_rn(b, __fmul_rn(amp0, Cs[r * 32 + lane]));
-    const float2 jn = rtab[r];
-    const int j = __float_as_int(jn.x);
-    const float rl = b > 0.f ? b : 0.f;
-    const float sq = __fmul_rn(rl, rl);
-    const bool normal = jn.y >= 1.17549435e-38f && jn.y <= 3.40282347e38f;
-    const float cf = (sq == 0.f && normal) ? 0.f : __fdiv_rn(sq, jn.y);
+  // hand every column to its owner: its smallest magnitude, largest t and the
+  // candidate bits of the four lanes that hold its rows
+  const bool up = lane & 16, odd = lane & 8;
+  UnitScore r;
+  float e0 = up ? ea[2] : ea[0], e1 = up ? ea[3] : ea[1];
+  const float x0 = up ? ea[0] : ea[2], x1 = up ? ea[1] : ea[3];
+  const float y0 = __shfl_xor_sync(0xffffffffu, x0, 16), y1 = __shfl_xor_sync(0xffffffffu, x1, 16);
+  e0 = min_abs_nan(e0, y0, y0);
+  e1 = min_abs_nan(e1, y1, y1);
+  const float z = __shfl_xor_sync(0xffffffffu, odd ? e0 : e1, 8);
+  r.e0 = min_abs_nan(odd ? e1 : e0, z, z);
+  r.mo = up ? (odd ? m[3] : m[2]) : (odd ? m[1] : m[0]);
+  r.rows = 0u;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const unsigned v = __shfl_sync(0xffffffffu, cand, 8 * k + (lane & 7));
+    r.rows |= ((v >> (8 * rq)) & 0xffu) << (8 * k);
+  }
+  return r;
+}
+
+// The group's packed best of the lane's own column when it is in `cols` (its
+// gbest and gexp are rewritten), 0 otherwise.
+__device__ __forceinline__ unsigned long long unit_fold(const PeelArgs& a, const UnitScore& us,
+                                                        const float* Cs, const UnitIn* in, uint2 u,
+                                                        int lane) {
+  const int oc = own_column(lane);
+  const bool ond = (u.y >> oc) & 1u;
+  const float scale = in->nm[lane].y;
+  const bool odd_nm = __any_sync(0xffffffffu, scale != scale);
+  const float mo = us.mo;
+  float best = 0.f;
+  int arg = __reduce_min_sync(0xffffffffu, in->row[lane]);
+  const bool all = odd_nm || !(mo <= 0.f || (mo >= 2.8421709e-14f && mo <= 1.1529215e18f));
+  unsigned rows = us.rows;
+  if (!ond || all || !(mo > 0.f)) rows = 0u;
+  if (rows) best = -1.f;
+  for (; rows; rows &= rows - 1u) {   // usually one row
+    const int bit = __ffs(rows) - 1;
+    const int r = 4 * (bit & 7) + (bit >> 3);
+    const float x = Cs[r * 32 + oc];
+    const float cf = __fdiv_rn(__fmul_rn(x, x), in->nm[r].x);
+    const int j = in->row[r];
     if (cf > best || (cf == best && j < arg)) {
       best = cf;
       arg = j;
     }
   }
-  // rows whose score is exactly 0 (sq = 0 and 1/nm not NaN) can only matter
-  // when no candidate scored above 0: fold them then (score 0, smaller
-  // template index first)
-  if (__any_sync(0xffffffffu, nd && !(best > 0.f))) {
-    for (int r = 0; r < nrow; ++r) {
-      const int j = __shfl_sync(0xffffffffu, jl, r);
-      const float nmy = __shfl_sync(0xffffffffu, nl.y, r);
-      float b = Bs[r * 32 + lane];
-      if (sub) b = __fsub_rn(b, __fmul_rn(amp0, Cs[r * 32 + lane]));
-      const float rl = b > 0.f ? b : 0.f;
-      const float sq = __fmul_rn(rl, rl);
-      if (nd && sq == 0.f && nmy == nmy && (0.f > best || (0.f == best && j < arg))) {
-        best = 0.f;
-        arg = j;
+  if (__any_sync(0xffffffffu, ond && all)) {
+    if (all) {
+      best = -1.f;
+      arg = 0x7fffffff;
+      for (int r = 0; r < kGroup; ++r) {
+        const float x = Cs[r * 32 + oc];
+        const float rl = x > 0.f ? x : 0.f;
+        const float sq = __fmul_rn(rl, rl);
+        const float nm = in->nm[r].x;
+        const bool normal = nm >= 1.17549435e-38f && nm <= 3.40282347e38f;
+        const float cf = (sq == 0.f && normal) ? 0.f : __fdiv_rn(sq, nm);
+        const int j = in->row[r];
+        if (cf > best || (cf == best && j < arg)) {
+          best = cf;
+          arg = j;
+        }
       }
     }
-  }
   }
   unsigned long long gb = 0ull;
-  if (nd) {
+  if (ond) {
     gb = best >= 0.f ? pack_score(best, arg) : 0ull;
-    const size_t mi = ((size_t)blk * a.ng + g) * 32 + lane;
+    const size_t mi = ((size_t)(u.x >> 11) * a.ng + (u.x & 2047u)) * 32 + oc;
     a.gbest[mi] = gb;
-    a.gexp[mi] = (unsigned char)emin;
+    a.gexp[mi] = (unsigned char)noop_expo(us.e0);
   }
   return gb;
 }
 
-// Row indices and {nm, 1/nm} of group g, lane r holding position r.
-__device__ __forceinline__ void group_rows(const PeelArgs& a, int g, int lane, int& jl, float2& nl) {
-  const int rr = g * kGroup + lane;
-  jl = 0;
-  nl = make_float2(1.f, 1.f);
-  if (rr < a.K) {
-    jl = __ldg(a.rperm + rr);
-    nl = __ldg(a.nmip + rr);
-  }
-}
-
-// Initial scores of groups [g_lo, g_hi) of block blk (nothing subtracted):
-// every group's gbest and gexp, and the column maxima folded into pack_out.
-template <bool kLazy>
-__device__ void group_init_item(const PeelArgs& a, const Smem& s, int blk, int g_lo, int g_hi,
-                                unsigned long long* pack_out, int lane, int warp) {
-  const int c = blk * kCol + lane;
-  const bool colok = c < a.L;
-  const TouchList none{0, nullptr, nullptr, nullptr};
-  const LaneEntries le{-1, 0u};
-  unsigned long long colbest = 0ull;
-  for (int g = g_lo; g < g_hi; ++g) {
-    int jl;
-    float2 nl;
-    group_rows(a, g, lane, jl, nl);
-    const unsigned long long gb =
-        group_tile<kLazy>(a, s, none, blk, g, colok, le, false, jl, nl, lane, warp);
-    colbest = gb > colbest ? gb : colbest;
-  }
-  if (colok && colbest) atomicMax(&pack_out[c], colbest);
-}
-
-// Phase A for dirty block blk (iteration parity p): publish the block's
-// ordered touch list for its units, decide per column and group from the
-// metadata, fold the cached bests of the groups a column leaves alone (and
-// the settled score of a column no peak touches) into pack_out, and append
-// the groups some column must process to the unit list.
-__device__ void group_scan_block(const PeelArgs& a, const Smem& s, int p, int blk,
-                                 unsigned long long* pack_out, int lane, int warp) {
-  const TouchList tl = load_touch_warp(a, s, p, blk, lane, warp);
-  int* bl = a.blist + (size_t)blk * 32;
-  if (lane == 0) bl[0] = tl.n;
-  if (lane < tl.n) {
-    bl[1 + lane] = tl.tau[lane];
-    bl[1 + kTouch + lane] = tl.k[lane];
-    bl[1 + 2 * kTouch + lane] = __float_as_int(tl.amp[lane]);
-  }
-  const int c = blk * kCol + lane;
-  const bool colok = c < a.L;
-  const int nt = a.nt, ng = a.ng;
-  unsigned tmask = 0u;
-  for (int e = 0; e < tl.n; ++e) {
-    const int d = c - tl.tau[e];
-    if (colok && d >= -nt && d <= nt) tmask |= 1u << e;
-  }
-  const bool touched = tmask != 0u;
-  const size_t meta = (size_t)blk * ng * 32 + lane;
-  unsigned char* eb = s.eb + warp * (kTouch * 32);
-  unsigned* ucount = a.wctr + 2 + p;
-  unsigned long long colbest = 0ull;
-  for (int gc = 0; gc < ng; gc += 32) {
-    const int gn = min(32, ng - gc);
-    const unsigned gmask = gn == 32 ? 0xffffffffu : ((1u << gn) - 1u);
-    // exponent fields of the product bounds of every touching peak, for the
-    // groups gc + lane
-    __syncwarp();
-    for (int e = 0; e < tl.n; ++e) {
-      int x = 255;
-      if (lane < gn)
-        x = bound_expo(__fmul_rn(fabsf(tl.amp[e]), __ldg(a.mg + (size_t)tl.k[e] * ng + gc + lane)));
-      eb[e * 32 + lane] = (unsigned char)x;
+// The units first, first + step, ... (nu of them) of the iteration's list, or
+// (kInit) of all nblk * ng tiles, whose initial scores are folded (nothing is
+// subtracted or written back).  Per unit: its rows and staged
+// cross-correlations are waited for, the columns subtract their touching
+// peaks in application order (further peaks stage theirs in the slot's tile),
+// the rows are written back and scored.  The next unit's cross-correlations
+// are staged in the other slot once this unit's are applied, its rows are
+// requested once this unit's registers are free, and the one after it has its
+// inputs fetched.
+template <bool kInit>
+__device__ void run_units(const PeelArgs& a, const Smem& s, long long first, long long step,
+                          int nu, unsigned long long* pack_out, int lane, int warp) {
+  uint2 rec = make_uint2(0u, 0u);
+  auto record = [&](int i) {
+    if (kInit) {
+      const unsigned w = (unsigned)first + (unsigned)i * (unsigned)step, ng = (unsigned)a.ng;
+      const int blk = (int)(w / ng), left = a.L - blk * kCol;
+      return make_uint2(((unsigned)blk << 11) | (w % ng),
+                        left >= kCol ? 0xffffffffu : (1u << left) - 1u);
     }
-    __syncwarp();
-    unsigned need = 0u;
-    if (touched) {
-#pragma unroll 8
-      for (int i = 0; i < gn; ++i) {
-        const int ex = a.gexp[meta + (size_t)(gc + i) * 32];
-        bool nd = false;
-        for (unsigned m = tmask; m; m &= m - 1u) {
-          const int e = __ffs(m) - 1;
-          nd |= (int)eb[e * 32 + i] + 26 > ex;
-        }
-        if (nd) need |= 1u << i;
-      }
-      const unsigned keep = ~need & gmask;
-#pragma unroll 8
-      for (int i = 0; i < gn; ++i) {
-        if ((keep >> i) & 1u) {
-          const unsigned long long gb = a.gbest[meta + (size_t)(gc + i) * 32];
-          colbest = gb > colbest ? gb : colbest;
-        }
+    return make_uint2(__shfl_sync(0xffffffffu, rec.x, i), __shfl_sync(0xffffffffu, rec.y, i));
+  };
+  if (nu <= 0) return;
+  if (!kInit && lane < nu) rec = a.units[first + lane * step];
+  uint2 u = record(0);
+  float* Cs = unit_tile(s, warp);
+  __syncwarp();                       // the tile's and the slots' earlier readers are done
+  unit_fetch<kInit>(a, u, unit_in(s, warp, 0), lane);
+#pragma unroll 1
+  for (int i = 0; i < nu; ++i) {
+    const UnitIn* in = unit_in(s, warp, i);
+    cp_async_wait_all();
+    __syncwarp();                     // the unit's inputs have landed
+    unsigned long long b[8][2];
+    LaneEntries le{-1, 0u};
+    if (!kInit) le = unit_begin(a, in, u, Cs, lane);
+    unit_rows(a, in, u, b, lane);
+    uint2 un = u;
+    if (i + 1 < nu) un = record(i + 1);
+    if (!kInit) {
+      const unsigned long long one2 = f2_pack(a.one, a.one);
+      unsigned long long n01, n23;
+      column_pairs(le.e0 >= 0 ? -__int_as_float(in->list[1 + 2 * kTouch + le.e0]) : -0.f, lane, n01,
+                   n23);
+      cp_async_wait_all();
+      __syncwarp();                   // every lane's staged column has landed
+      apply_ctc(Cs, n01, n23, one2, b, lane);
+#pragma unroll 1
+      for (unsigned m = __reduce_or_sync(0xffffffffu, le.rest); m; m &= m - 1u) {
+        const int e = __ffs(m) - 1;
+        const bool mine = (le.rest >> e) & 1u;
+        __syncwarp();                 // the tile is read
+        stage_ctc(Cs, mine ? entry_slab(a, in, e, (int)(u.x >> 11) * kCol + lane) : a.ctcT, mine,
+                  in->row, 2 * a.nt + 1, lane);
+        column_pairs(mine ? -__int_as_float(in->list[1 + 2 * kTouch + e]) : -0.f, lane, n01, n23);
+        cp_async_wait_all();
+        __syncwarp();
+        apply_ctc(Cs, n01, n23, one2, b, lane);
       }
     }
-    const unsigned proc = __reduce_or_sync(0xffffffffu, need);
-    if (proc) {
-      unsigned base = 0u;
-      if (lane == 0) base = atomicAdd(ucount, (unsigned)__popc(proc));
-      base = __shfl_sync(0xffffffffu, base, 0);
-      unsigned cols = 0u;             // lane i: the columns that process group gc + i
-      for (unsigned m = proc; m; m &= m - 1u) {
-        const int i = __ffs(m) - 1;
-        const unsigned b = __ballot_sync(0xffffffffu, (need >> i) & 1u);
-        if (lane == i) cols = b;
+    if (i + 1 < nu) unit_fetch<kInit>(a, un, unit_in(s, warp, i + 1), lane);
+    // write back; the tile keeps the scores for the quotients
+    {
+      const int rq = lane >> 3;
+      float* cs = Cs + rq * 32 + (lane & 7) * 4;
+      float* brow = a.Bt + (size_t)(u.x >> 11) * a.K * kCol + (lane & 7) * 4;
+#pragma unroll
+      for (int r = 0; r < 8; ++r) {
+        const ulonglong2 v = make_ulonglong2(b[r][0], b[r][1]);
+        if (!kInit)
+          *reinterpret_cast<ulonglong2*>(brow + (unsigned)in->row[4 * r + rq] * kCol) = v;
+        *reinterpret_cast<ulonglong2*>(cs + r * 128) = v;
       }
-      if ((proc >> lane) & 1u)
-        a.units[base + __popc(proc & ((1u << lane) - 1u))] =
-            make_uint2(((unsigned)blk << 11) | (unsigned)(gc + lane), cols);
     }
+    const UnitScore us = unit_score(in, b, lane);
+    __syncwarp();                     // the tile holds every lane's scores
+    const unsigned long long gb = unit_fold(a, us, Cs, in, u, lane);
+    if (gb) atomicMax(&pack_out[(u.x >> 11) * kCol + own_column(lane)], gb);
+    u = un;
   }
-  if (colok) {
-    if (touched) {
-      if (colbest) atomicMax(&pack_out[c], colbest);
-    } else {
-      atomicMax(&pack_out[c], pack_score(a.cfmax[c], a.imax[c]));
-    }
-  }
-}
-
-// Phase B: one unit (a group tile that some columns of a block must
-// process), its block's ordered touch list read back from the scan.
-// unit_fetch issues the unit's loads (the block's list, the group's rows);
-// unit_run uses them, so a warp fetches its next unit before running the
-// current one.
-struct UnitFetch {
-  uint2 u;
-  int v;        // word `lane` of the block's list (n, tau[], k[], amp bits[])
-  int jl;       // row index of group position `lane`
-  float2 nl;    // its {nm, 1/nm}
-};
-
-__device__ __forceinline__ UnitFetch unit_fetch(const PeelArgs& a, uint2 u, int lane) {
-  UnitFetch f;
-  f.u = u;
-  const int blk = (int)(u.x >> 11), g = (int)(u.x & 2047u);
-  f.v = lane < 1 + 3 * kTouch ? a.blist[(size_t)blk * 32 + lane] : 0;
-  group_rows(a, g, lane, f.jl, f.nl);
-  return f;
-}
-
-template <bool kLazy>
-__device__ void unit_run(const PeelArgs& a, const Smem& s, const UnitFetch& f,
-                         unsigned long long* pack_out, int lane, int warp) {
-  const int blk = (int)(f.u.x >> 11), g = (int)(f.u.x & 2047u);
-  const bool nd = (f.u.y >> lane) & 1u;
-  const int n = __shfl_sync(0xffffffffu, f.v, 0);
-  int* tau = s.tl_tau + warp * kTouch;
-  int* kk = s.tl_k + warp * kTouch;
-  float* amp = s.tl_amp + warp * kTouch;
-  const int tv = __shfl_sync(0xffffffffu, f.v, 1 + (lane & (kTouch - 1)));
-  const int kv = __shfl_sync(0xffffffffu, f.v, 1 + kTouch + (lane & (kTouch - 1)));
-  const int av = __shfl_sync(0xffffffffu, f.v, 1 + 2 * kTouch + (lane & (kTouch - 1)));
-  __syncwarp();
-  if (lane < n) {
-    tau[lane] = tv;
-    kk[lane] = kv;
-    amp[lane] = __int_as_float(av);
-  }
-  __syncwarp();
-  const TouchList tl{n, tau, kk, amp};
-  const int c = blk * kCol + lane;
-  const LaneEntries le = lane_entries(tl, c, c < a.L, a.nt);
-  const unsigned long long gb =
-      group_tile<kLazy>(a, s, tl, blk, g, nd, le, true, f.jl, f.nl, lane, warp);
-  if (nd && gb) atomicMax(&pack_out[c], gb);
 }
 
 // Block of the rank-th set bit of the dirty bitmap (s.wprefix holds the
 // exclusive prefix of the word popcounts).
-__device__ __forceinline__ int dirty_block(const Smem& s, const unsigned* bits,
-                                           int nwords, int rank) {
+__device__ __forceinline__ int dirty_block(const Smem& s, int nwords, int rank) {
   int lo = 0, hi = nwords - 1;
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
     if (s.wprefix[mid] <= rank) lo = mid; else hi = mid - 1;
   }
-  const unsigned word = bits[lo];
+  const unsigned word = s.dw[lo];
   const int bit = (int)__fns(word, 0, rank - s.wprefix[lo] + 1);
   return lo * 32 + bit;
+}
+
+// Phase A over the dirty blocks w, w + step, ... below ndirty, one warp per
+// block: publish the block's ordered touch list for its units, decide per
+// column and group from the metadata, fold the cached bests of the groups a
+// column leaves alone (and the settled score of a column no peak touches)
+// into pack_out, and append the groups some column must process to the unit
+// list.  The next block's touch list is read, and the place of this block's
+// units in the list comes back, while the next block's metadata is on its way.
+//
+// What bounds it: the latency of its chain (touch list, bounds, metadata); with
+// every step of it exposed, a block took 13 us at K = 600.
+__device__ void group_scan(const PeelArgs& a, const Smem& s, int p, long long w, long long step,
+                           int ndirty, unsigned long long* pack_out, int lane, int warp) {
+  if (w >= ndirty) return;
+  const int nt = a.nt, ng = a.ng;
+  // the block's metadata, kScanGroups groups at a time: [gn][32] bests, then
+  // [gn][32] exponents
+  unsigned long long* sb = reinterpret_cast<unsigned long long*>(unit_tile(s, warp));
+  unsigned char* se = reinterpret_cast<unsigned char*>(sb + kScanGroups * 32);
+  auto fetch = [&](int blk, int gc, int gn) {
+    const char* gb = reinterpret_cast<const char*>(a.gbest + ((size_t)blk * ng + gc) * 32);
+    const char* ge = reinterpret_cast<const char*>(a.gexp + ((size_t)blk * ng + gc) * 32);
+    for (int i = lane; i < gn * 16; i += 32) cp_async16(reinterpret_cast<char*>(sb) + i * 16, gb + i * 16);
+    for (int i = lane; i < gn * 2; i += 32) cp_async16(reinterpret_cast<char*>(se) + i * 16, ge + i * 16);
+    cp_async_commit();
+  };
+  unsigned char* eb = s.eb + warp * (kTouch * 32);
+  unsigned* ucount = a.wctr + 2 + p;
+  // units whose place in the list has been asked for: lane i holds group
+  // (at & 2047) + i's columns
+  unsigned base = 0u, pend = 0u, pcols = 0u, at = 0u;
+  auto flush = [&]() {
+    if (pend) {
+      const unsigned first = __shfl_sync(0xffffffffu, base, 0);
+      if ((pend >> lane) & 1u)
+        a.units[first + __popc(pend & ((1u << lane) - 1u))] = make_uint2(at + lane, pcols);
+      pend = 0u;
+    }
+  };
+  int blk = dirty_block(s, a.nwords, (int)w);
+  TouchWord t = touch_word(a, p, blk, lane);
+  while (true) {
+    const int c = blk * kCol + lane;
+    const bool colok = c < a.L;
+    __syncwarp();                       // the tile's earlier readers are done
+    fetch(blk, 0, min(kScanGroups, ng));
+    const TouchList tl = order_touch_warp(s, t, lane, warp);
+    w += step;
+    const int next = w < ndirty ? dirty_block(s, a.nwords, (int)w) : -1;
+    if (next >= 0) t = touch_word(a, p, next, lane);
+    int* bl = a.blist + (size_t)blk * 32;
+    if (lane == 0) bl[0] = tl.n;
+    if (lane < tl.n) {
+      bl[1 + lane] = tl.tau[lane];
+      bl[1 + kTouch + lane] = tl.k[lane];
+      bl[1 + 2 * kTouch + lane] = __float_as_int(tl.amp[lane]);
+    }
+    unsigned tmask = 0u;
+    for (int e = 0; e < tl.n; ++e) {
+      const int d = c - tl.tau[e];
+      if (colok && d >= -nt && d <= nt) tmask |= 1u << e;
+    }
+    const bool touched = tmask != 0u;
+    unsigned long long colbest = 0ull;
+    for (int gc = 0; gc < ng; gc += kScanGroups) {
+      const int gn = min(kScanGroups, ng - gc);
+      if (gc > 0) {
+        __syncwarp();
+        fetch(blk, gc, gn);
+      }
+      // exponent fields of the product bounds of every touching peak plus 26,
+      // for the groups gc + lane
+      for (int e = 0; e < tl.n; ++e) {
+        int x = 255;
+        if (lane < gn)
+          x = min(255, 26 + bound_expo(__fmul_rn(fabsf(tl.amp[e]),
+                                                 __ldg(a.mg + (size_t)tl.k[e] * ng + gc + lane))));
+        eb[e * 32 + lane] = (unsigned char)x;
+      }
+      flush();
+      cp_async_wait_all();
+      __syncwarp();
+      // groups that the lane's first peak can change, then those that a further
+      // peak can (exponents are at most 254: a bound of 255 always passes)
+      unsigned need = 0u;
+      if (touched) {
+        const unsigned char* b0 = eb + (__ffs(tmask) - 1) * 32;
+#pragma unroll 4
+        for (int i = 0; i < gn; ++i) need |= b0[i] > se[i * 32 + lane] ? 1u << i : 0u;
+        for (unsigned m = tmask & (tmask - 1u); m; m &= m - 1u) {
+          const unsigned char* b1 = eb + (__ffs(m) - 1) * 32;
+          for (int i = 0; i < gn; ++i) need |= b1[i] > se[i * 32 + lane] ? 1u << i : 0u;
+        }
+        for (unsigned m = ~need & (gn == 32 ? 0xffffffffu : (1u << gn) - 1u); m; m &= m - 1u) {
+          const unsigned long long gb = sb[(__ffs(m) - 1) * 32 + lane];
+          colbest = gb > colbest ? gb : colbest;
+        }
+      }
+      const unsigned proc = __reduce_or_sync(0xffffffffu, need);
+      if (proc) {
+        if (lane == 0) base = atomicAdd(ucount, (unsigned)__popc(proc));
+        for (unsigned m = proc; m; m &= m - 1u) {
+          const int i = __ffs(m) - 1;
+          const unsigned b = __ballot_sync(0xffffffffu, (need >> i) & 1u);
+          if (lane == i) pcols = b;
+        }
+        pend = proc;
+        at = ((unsigned)blk << 11) | (unsigned)gc;
+      }
+    }
+    if (colok) {
+      if (touched) {
+        if (colbest) atomicMax(&pack_out[c], colbest);
+      } else {
+        atomicMax(&pack_out[c], pack_score(a.cfmax[c], a.imax[c]));
+      }
+    }
+    if (next < 0) break;
+    blk = next;
+  }
+  flush();
 }
 
 // Outcome of one batch's peel, the same in every block of the team.
@@ -1093,12 +1367,14 @@ struct PeelOutcome {
 // (written by one thread) and is returned to every thread.  When the status
 // is KS_OK every record and residual list of the batch is complete and
 // visible to the team (the last pass ended at a team barrier).
-template <int kRows, bool kGrouped, bool kLazy = false>
+template <int kRows, bool kGrouped>
 __device__ PeelOutcome run_peel(const PeelArgs& a, const Smem& s, int rank, unsigned G,
                                 unsigned& epoch) {
   const int tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5;
-  const long long gwarp = (long long)rank * kWarps + warp;
+  // warps are numbered across the blocks, so that fewer items than warps are
+  // spread over every SM
+  const long long gwarp = (long long)warp * G + rank;
   const long long nwarps = (long long)G * kWarps;
   stage_basis(a.W, a.P, a.nt, s.W, kThreads);
   // a failed producer of the score matrix fails the peel
@@ -1132,14 +1408,11 @@ __device__ PeelOutcome run_peel(const PeelArgs& a, const Smem& s, int rank, unsi
   {
     unsigned long long* pinit = a.pack + (size_t)a.L;
     if (kGrouped) {
-      // items of kInitGroups groups: the group metadata of every column too
-      const int rg = (a.ng + kInitGroups - 1) / kInitGroups;
-      const long long n_items = (long long)a.nblk * rg;
-      for (long long w = gwarp; w < n_items; w += nwarps) {
-        const int blk = (int)(w / rg), r = (int)(w % rg);
-        group_init_item<kLazy>(a, s, blk, r * kInitGroups, min(a.ng, (r + 1) * kInitGroups), pinit,
+      // every (block, group) tile: the group metadata of every column too
+      const long long n_items = (long long)a.nblk * a.ng;
+      if (gwarp < n_items)
+        run_units<true>(a, s, gwarp, nwarps, (int)((n_items - gwarp + nwarps - 1) / nwarps), pinit,
                         lane, warp);
-      }
     } else {
       const int rg = (a.K + kItemRows - 1) / kItemRows;
       const TouchList none{0, nullptr, nullptr, nullptr};
@@ -1155,12 +1428,17 @@ __device__ PeelOutcome run_peel(const PeelArgs& a, const Smem& s, int rank, unsi
   long long n_out = 0;
   int it = 0;
   int status = KS_OK;
-  KS_TRACE(0, 7, ks_globaltimer());
+  KS_TRACE(199, 0, ks_globaltimer());
   bool ok = ks_grid_sync(a.bar, G, epoch, a.err, a.limit_ns);
   for (; ok && it < a.max_peels; ++it) {
     const int p = it & 1, q = p ^ 1;
     KS_TRACE(it, 0, ks_globaltimer());
-    for (int ch = rank; ch < a.nchunks; ch += (int)G) detect_chunk(a, s, ch, it);
+    if (warp_detection(a.nt, kGrouped, a.nchunks, G)) {
+      for (long long ch = gwarp; ch < a.nchunks; ch += nwarps)
+        detect_chunk_warp(a, unit_tile(s, warp), (int)ch, it, lane);
+    } else {
+      for (int ch = rank; ch < a.nchunks; ch += (int)G) detect_chunk(a, s, ch, it);
+    }
     KS_TRACE(it, 1, ks_globaltimer());
     if (!ks_grid_sync(a.bar, G, epoch, a.err, a.limit_ns)) break;
     KS_TRACE(it, 2, ks_globaltimer());
@@ -1209,34 +1487,31 @@ __device__ PeelOutcome run_peel(const PeelArgs& a, const Smem& s, int rank, unsi
     if (kGrouped) {
       // phase A: one warp per dirty block, dealt round-robin (metadata only,
       // about the same work per block)
-      for (long long w = gwarp; w < ndirty; w += nwarps)
-        group_scan_block(a, s, p, dirty_block(s, bits, a.nwords, (int)w), pcur, lane, warp);
+      group_scan(a, s, p, gwarp, nwarps, ndirty, pcur, lane, warp);
       if (!ks_grid_sync(a.bar, G, epoch, a.err, a.limit_ns)) break;
-      // phase B: the units, taken from a counter in claims of about a quarter
-      // of a warp's share (at most 32), so thousands of warps do not queue on
-      // it; a warp reads its claim's records at once and fetches each unit's
-      // inputs while it runs the one before
+      // phase B: the units.  Up to kStaticUnits per warp are dealt round-robin
+      // (neighbouring warps run one block's groups at the same time; a counter
+      // taken one unit at a time by thousands of warps would be their queue);
+      // more are taken from a counter in claims of about a quarter of a warp's
+      // share (at most 32).  A warp reads its records at once and fetches each
+      // unit's inputs while it runs the one before.
+      KS_TRACE(it, 7, ks_globaltimer());
       const unsigned n_units = ks_ld_acquire(a.wctr + 2 + p);
+      const bool dealt = (long long)n_units <= kStaticUnits * nwarps;
       const unsigned claim =
           (unsigned)min(32LL, max(1LL, (long long)n_units / (nwarps * 4)));
-      while (true) {
-        unsigned first = 0;
-        if (lane == 0) first = atomicAdd(&a.wctr[4 + p], claim);
-        first = __shfl_sync(0xffffffffu, first, 0);
-        if (first >= n_units) break;
-        const int nu = (int)(min(n_units, first + claim) - first);
-        const uint2 rec = lane < nu ? a.units[first + lane] : make_uint2(0u, 0u);
-        UnitFetch cur = unit_fetch(
-            a, make_uint2(__shfl_sync(0xffffffffu, rec.x, 0), __shfl_sync(0xffffffffu, rec.y, 0)),
-            lane);
-        for (int i = 0; i < nu; ++i) {
-          UnitFetch nxt = cur;
-          if (i + 1 < nu)
-            nxt = unit_fetch(a, make_uint2(__shfl_sync(0xffffffffu, rec.x, i + 1),
-                                           __shfl_sync(0xffffffffu, rec.y, i + 1)),
-                             lane);
-          unit_run<kLazy>(a, s, cur, pcur, lane, warp);
-          cur = nxt;
+      if (dealt) {
+        if (gwarp < n_units)
+          run_units<false>(a, s, gwarp, nwarps, (int)((n_units - gwarp + nwarps - 1) / nwarps), pcur,
+                           lane, warp);
+      } else {
+        while (true) {
+          unsigned first = 0;
+          if (lane == 0) first = atomicAdd(&a.wctr[4 + p], claim);
+          first = __shfl_sync(0xffffffffu, first, 0);
+          if (first >= n_units) break;
+          run_units<false>(a, s, first, 1, (int)(min(n_units, first + claim) - first), pcur, lane,
+                           warp);
         }
       }
     } else {
@@ -1270,7 +1545,7 @@ __device__ PeelOutcome run_peel(const PeelArgs& a, const Smem& s, int rank, unsi
       const long long n_static =
           (nwarps >= kStaticWarps && rounds > 1) ? (rounds - 1) * nwarps : 0;
       for (long long w = gwarp; w < n_static; w += nwarps) {
-        const int blk = dirty_block(s, bits, a.nwords, (int)(w / rgroups));
+        const int blk = dirty_block(s, a.nwords, (int)(w / rgroups));
         const int r = (int)(w % rgroups);
         const TouchList tl = load_touch_warp(a, s, p, blk, lane, warp);
         update_warp_item<kRows>(a, tl, blk, r * rows, min(a.K, (r + 1) * rows), pcur, lane);
@@ -1280,7 +1555,7 @@ __device__ PeelOutcome run_peel(const PeelArgs& a, const Smem& s, int rank, unsi
         if (lane == 0) next = atomicAdd(&a.wctr[p], 1u);
         const long long w = n_static + (long long)__shfl_sync(0xffffffffu, next, 0);
         if (w >= n_items) break;
-        const int blk = dirty_block(s, bits, a.nwords, (int)(w / rgroups));
+        const int blk = dirty_block(s, a.nwords, (int)(w / rgroups));
         const int r = (int)(w % rgroups);
         const TouchList tl = load_touch_warp(a, s, p, blk, lane, warp);
         update_warp_item<kRows>(a, tl, blk, r * rows, min(a.K, (r + 1) * rows), pcur, lane);
@@ -1308,7 +1583,7 @@ __device__ PeelOutcome run_peel(const PeelArgs& a, const Smem& s, int rank, unsi
 // kGrouped: the grouped update (a.rperm, a.nmip, a.mg and the group metadata
 // set); the ungrouped form needs no group metadata.
 template <bool kGrouped>
-__global__ void __launch_bounds__(kThreads, 2) peel_kernel(PeelArgs a) {
+__global__ void __launch_bounds__(kThreads, kGrouped ? kBlocksPerSm : kTeamBlocksPerSm) peel_kernel(PeelArgs a) {
   extern __shared__ __align__(16) char smem_raw[];
   const Smem s = carve_smem(a, smem_raw, kGrouped);
   unsigned epoch = 0;
@@ -1322,7 +1597,7 @@ constexpr int kXStride = 20;                // floats of a channel pair's loadin
 constexpr int kXU = 8 * kXStride;           // floats of one spike's loadings of 16 channels
 constexpr int kXWarp = 3 * kXList + kXU;    // 4-byte words per warp
 // the batched peel's residual scratch fits in the stage tiles
-static_assert(kXWarp <= 2 * kGroup * 32 && (3 * kXList) % 4 == 0,
+static_assert(4 * kXWarp <= kTileBytes && (3 * kXList) % 4 == 0,
               "residual scratch exceeds a stage tile");
 
 struct ResSmem {
@@ -1422,33 +1697,6 @@ __device__ int load_residual_list(const PeelArgs& a, const ResSmem& s, int blk, 
   return n;
 }
 
-// Two packed FP32 operations per instruction (each half rounds as the scalar
-// operation does).
-__device__ __forceinline__ unsigned long long f2_pack(float lo, float hi) {
-  unsigned long long r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ void f2_unpack(unsigned long long v, float& lo, float& hi) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ unsigned long long f2_fma(unsigned long long a, unsigned long long b,
-                                                     unsigned long long c) {
-  unsigned long long r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ unsigned long long f2_mul(unsigned long long a, unsigned long long b) {
-  unsigned long long r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ unsigned long long f2_add(unsigned long long a, unsigned long long b) {
-  unsigned long long r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-
 // Channels of one residual tile, and tiles per bit of a template's support
 // mask: the tiles 0 .. ceil(C/16)-1 are spread over 64 bits.
 constexpr int kXCh = 16;
@@ -1478,6 +1726,7 @@ __device__ void residual_apply(const PeelArgs& a, const ResSmem& s, int n, int c
   const int ch = cbase + (lane & (kXCh - 1));
   const int p0 = (lane / kXCh) * (PP / 2);     // this lane loads components p0 .. p0 + PP/2 - 1
   const bool chok = ch < a.C;
+  const unsigned long long one2 = f2_pack(a.one, a.one);
   for (int e0 = 0; e0 < n; e0 += 32) {
     bool hit = e0 + lane < n;
     if (hit && a.sup) hit = (a.sup[s.xl_k[e0 + lane]] >> bit) & 1ull;
@@ -1523,8 +1772,7 @@ __device__ void residual_apply(const PeelArgs& a, const ResSmem& s, int n, int c
           v = f2_fma(uu.y, w2[p + 1], v);
         }
         // x - fl(amp v) = x + fl(-amp v), on the columns inside the window
-        const unsigned long long d = f2_mul(amp2, v);
-        if (in) x2[i] = f2_add(x2[i], d);
+        if (in) x2[i] = f2_add_prod(x2[i], amp2, v, one2);
       }
     }
   }
@@ -1729,6 +1977,9 @@ __global__ void __launch_bounds__(256) ks_group_order_kernel(const float* __rest
       }
   }
   if (k < K) rperm[rank] = k;
+  // whole groups: the last template fills the positions past K
+  if (k < K && rank == K - 1)
+    for (int r = K; r < n_groups(K) * kGroup; ++r) rperm[r] = k;
 }
 
 // mg[k][g] = the largest |ctcT[k][j][l]| over the rows j of group g (rows
@@ -1763,11 +2014,17 @@ __global__ void __launch_bounds__(256) ks_group_bound_kernel(const float* __rest
   }
 }
 
-// nmip[r] = nmi[rperm[r]]: {nm, 1/nm} of the template rows in group order.
+// {nm, 1/sqrt(nm)} of the template rows in group order; an nm outside
+// [2^-30, 2^30], where the group fold's comparison of scores by b/sqrt(nm)
+// could leave the normal range, gets a NaN scale.
 __global__ void ks_group_nmi_kernel(const float2* __restrict__ nmi, const int* __restrict__ rperm,
                                     int K, float2* __restrict__ nmip) {
-  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < K; r += gridDim.x * blockDim.x)
-    nmip[r] = nmi[rperm[r]];
+  const int n = n_groups(K) * kGroup;     // whole groups
+  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
+    const float nm = nmi[rperm[r]].x;
+    const bool ok = nm >= 9.3132257e-10f && nm <= 1.0737418e9f;
+    nmip[r] = make_float2(nm, ok ? __frsqrt_rn(nm) : __int_as_float(0x7fc00000));
+  }
 }
 
 // Scratch of one team (reused for every batch it processes), for batches of
@@ -1785,8 +2042,6 @@ struct TeamLayout {
 };
 
 __host__ __device__ inline size_t al256(size_t x) { return (x + 255) & ~size_t(255); }
-
-__host__ __device__ inline int n_groups(long long K) { return (int)((K + kGroup - 1) / kGroup); }
 
 __host__ __device__ inline TeamLayout team_layout(long long L, long long K) {
   const long long nchunks = (L + kChunk - 1) / kChunk, nblk = (L + kCol - 1) / kCol;
