@@ -16,8 +16,9 @@ static size_t group_setup_bytes(int64_t K) {
 }
 
 size_t peel_scratch_size(int64_t L, int64_t K, bool grouped) {
+  // 16 bytes to align the workspace (16-byte copies of its arrays)
   return al256(team_layout(L, grouped ? K : 0).bytes) + al256(list_layout(L).bytes) +
-         al256(8 * (size_t)K) + (grouped ? group_setup_bytes(K) : 0);
+         al256(8 * (size_t)K) + (grouped ? group_setup_bytes(K) + 16 : 0);
 }
 
 size_t group_tables_bytes(int64_t K) { return group_setup_bytes(K); }
@@ -169,6 +170,8 @@ int launch_peel_tiled(float* Bt, const float* X, float* Xres, const float* U, co
   a.st = reinterpret_cast<long long*>(st); a.amps = amps; a.th_amps = th_amps;
   a.info = reinterpret_cast<long long*>(info);
   char* base = static_cast<char*>(ws);
+  if (grouped)
+    base = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(ws) + 15) & ~uintptr_t(15));
   const size_t team_bytes = al256(team_layout(L, grouped ? K : 0).bytes);
   const size_t list_bytes = al256(list_layout(L).bytes);
   bind_scratch(a, base, base + team_bytes, grouped);
