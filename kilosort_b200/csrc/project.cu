@@ -15,10 +15,11 @@
 //                      channel and all P components (8*P FMA per tap, one
 //                      shared-memory load of X per tap); output staged in
 //                      shared memory and written as contiguous rows
-//   ks_sgemm_tn        FP32 SIMT contraction, 128x128x16 tiles, 8x8 per thread,
-//                      register double buffering; tile order puts the template
-//                      tiles of one time tile next to each other so each Yt tile
-//                      is read from HBM once
+//   ks_sgemm_tn        FP32 SIMT contraction with packed multiply-adds, tiles of
+//                      64 to 128 rows x 128 or 256 columns, register double
+//                      buffering; tile order puts the template tiles of one time
+//                      tile next to each other so each Yt tile is read from HBM
+//                      once
 #include "ks_common.cuh"
 #include "project.cuh"
 
@@ -234,79 +235,130 @@ size_t temporal_smem(int nt, int P) {
 }
 
 // ------------------------------------------------------------------ FP32 GEMM
-constexpr int kBM = 128, kBN = 128, kBK = 16;
+// Two FP32 fused operations in one instruction (each half rounds as fmaf).
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b,
+                                                   unsigned long long c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ unsigned long long dup2(float v) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(v));
+  return r;
+}
 
-// C[m, n] = sum_q A[m, q] * Bt[n, q]; A is [>= tiles_m*128, Kd], Bt is
-// [>= tiles_n*128, Kd] (both zero padded), Kd % 16 == 0.  Stores m < M, n < N,
-// row-major with leading dimension ldc, or (kTiled) in 32-column blocks
-// C[((n/32)*M + m)*32 + n%32].
-template <bool kTiled>
-__global__ void __launch_bounds__(256, 2)
+// C[m, n] = sum_q A[m, q] * Bt[n, q], every element one chain of fused
+// operations over q; A is [>= tiles_m*BM, Kd], Bt is [>= tiles_n*128, Kd]
+// (both zero padded), Kd % 16 == 0.  Stores m < M, n < N, row-major with
+// leading dimension ldc, or (kTiled) in 32-column blocks
+// C[((n/32)*M + m)*32 + n%32].  Tiles of BM = 16 TM rows x 128 columns, TM x 8
+// per thread, columns two at a time through packed operations.
+//
+// What bounds it: the FP32 pipe.  A packed operation does the work of two
+// issue slots, so loads and moves no longer compete with the multiply-adds:
+// 3.99 -> 3.11 ms at C=384, K=600, 60122 samples (41.6 -> 53.4 TFLOP/s), with 128
+// columns per tile 3.48 ms.  Measured and dropped at 256 columns: slices of 16
+// (3.60 ms), the next slice stored half way through this one (3.43), warps of 8 x
+// 4 threads (3.19).
+// Length of the slice of q staged at a time.
+__host__ __device__ constexpr int sgemm_slice(int TN) { return TN == 8 ? 16 : 8; }
+
+template <int TM, int TN, bool kTiled>
+__global__ void __launch_bounds__(256, TN == 8 ? 2 : 1)
 ks_sgemm_tn_kernel(const float* __restrict__ A, const float* __restrict__ Bt,
                    float* __restrict__ Cm, int M, int N, int Kd, long long ldc,
                    int tiles_m) {
-  __shared__ __align__(16) float As[2][kBK][kBM + 4];
-  __shared__ __align__(16) float Bs[2][kBK][kBN + 4];
+  constexpr int BM = 16 * TM, BN = 16 * TN, BK = sgemm_slice(TN);
+  constexpr int kP = BK / 4;                           // 16-byte pieces of a row's slice
+  constexpr int kALoads = (BM * kP + 255) / 256, kBLoads = BN * kP / 256;
+  extern __shared__ __align__(16) float sgemm_sm[];
+  float (*As)[BK][BM + 4] = reinterpret_cast<float (*)[BK][BM + 4]>(sgemm_sm);
+  float (*Bs)[BK][BN + 4] = reinterpret_cast<float (*)[BK][BN + 4]>(sgemm_sm + 2 * BK * (BM + 4));
   const int tid = threadIdx.x;
   const int tm = blockIdx.x % tiles_m;
   const int tn = blockIdx.x / tiles_m;
-  const long long m0 = (long long)tm * kBM, n0 = (long long)tn * kBN;
+  const long long m0 = (long long)tm * BM, n0 = (long long)tn * BN;
+  const long long last = ((N + 127LL) & ~127LL) - 1;   // the operand's last (padded) row
   const int tx = tid & 15, ty = tid >> 4;
-  // loader mapping: two float4 per operand per thread
-  int lrow[2], lc4[2];
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const int idx = tid + i * 256;
-    lrow[i] = idx >> 2;
-    lc4[i] = idx & 3;
-  }
-  float4 ra[2], rb[2];
+  // a thread's pieces: row idx / kP, columns 4 (idx % kP) of the slice
+  float4 ra[kALoads], rb[kBLoads];
   auto gload = [&](int k0) {
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      ra[i] = *reinterpret_cast<const float4*>(A + (m0 + lrow[i]) * Kd + k0 + lc4[i] * 4);
-      rb[i] = *reinterpret_cast<const float4*>(Bt + (n0 + lrow[i]) * Kd + k0 + lc4[i] * 4);
+    for (int i = 0; i < kALoads; ++i) {
+      const int idx = tid + i * 256;
+      if (BM * kP % 256 == 0 || idx < BM * kP)
+        ra[i] = *reinterpret_cast<const float4*>(A + (m0 + idx / kP) * Kd + k0 + idx % kP * 4);
+    }
+#pragma unroll
+    for (int i = 0; i < kBLoads; ++i) {
+      const int idx = tid + i * 256;
+      const long long n = n0 + idx / kP;
+      rb[i] = *reinterpret_cast<const float4*>(Bt + (n < last ? n : last) * Kd + k0 + idx % kP * 4);
     }
   };
   auto sstore = [&](int buf) {
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const int kk = lc4[i] * 4;
-      As[buf][kk + 0][lrow[i]] = ra[i].x;
-      As[buf][kk + 1][lrow[i]] = ra[i].y;
-      As[buf][kk + 2][lrow[i]] = ra[i].z;
-      As[buf][kk + 3][lrow[i]] = ra[i].w;
-      Bs[buf][kk + 0][lrow[i]] = rb[i].x;
-      Bs[buf][kk + 1][lrow[i]] = rb[i].y;
-      Bs[buf][kk + 2][lrow[i]] = rb[i].z;
-      Bs[buf][kk + 3][lrow[i]] = rb[i].w;
+    for (int i = 0; i < kALoads; ++i) {
+      const int idx = tid + i * 256, kk = idx % kP * 4, r = idx / kP;
+      if (BM * kP % 256 == 0 || idx < BM * kP) {
+        As[buf][kk + 0][r] = ra[i].x;
+        As[buf][kk + 1][r] = ra[i].y;
+        As[buf][kk + 2][r] = ra[i].z;
+        As[buf][kk + 3][r] = ra[i].w;
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < kBLoads; ++i) {
+      const int idx = tid + i * 256, kk = idx % kP * 4, r = idx / kP;
+      Bs[buf][kk + 0][r] = rb[i].x;
+      Bs[buf][kk + 1][r] = rb[i].y;
+      Bs[buf][kk + 2][r] = rb[i].z;
+      Bs[buf][kk + 3][r] = rb[i].w;
     }
   };
-  float acc[8][8];
+  // rows ty*4 .. ty*4+3 of the first 64, then TM-4 rows from 64 + ty*(TM-4) on;
+  // columns 64 g + tx*4 .. +3, in pairs
+  unsigned long long acc[TM][TN / 2];
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
+  for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+    for (int j = 0; j < TN / 2; ++j) acc[i][j] = 0ull;
 
   gload(0);
   sstore(0);
   __syncthreads();
-  const int nk = Kd / kBK;
+  const int nk = Kd / BK;
   for (int kt = 0; kt < nk; ++kt) {
     const int buf = kt & 1;
-    if (kt + 1 < nk) gload((kt + 1) * kBK);
+    if (kt + 1 < nk) gload((kt + 1) * BK);
 #pragma unroll
-    for (int kk = 0; kk < kBK; ++kk) {
-      const float4 a0 = *reinterpret_cast<const float4*>(&As[buf][kk][ty * 4]);
-      const float4 a1 = *reinterpret_cast<const float4*>(&As[buf][kk][64 + ty * 4]);
-      const float4 b0 = *reinterpret_cast<const float4*>(&Bs[buf][kk][tx * 4]);
-      const float4 b1 = *reinterpret_cast<const float4*>(&Bs[buf][kk][64 + tx * 4]);
-      const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-      const float bv[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+    for (int kk = 0; kk < BK; ++kk) {
+      float av[TM];
+      {
+        const float4 a0 = *reinterpret_cast<const float4*>(&As[buf][kk][ty * 4]);
+        av[0] = a0.x; av[1] = a0.y; av[2] = a0.z; av[3] = a0.w;
+        if (TM == 8) {
+          const float4 a1 = *reinterpret_cast<const float4*>(&As[buf][kk][64 + ty * 4]);
+          av[TM - 4] = a1.x; av[TM - 3] = a1.y; av[TM - 2] = a1.z; av[TM - 1] = a1.w;
+        } else if (TM == 6) {
+          const float2 a1 = *reinterpret_cast<const float2*>(&As[buf][kk][64 + ty * 2]);
+          av[TM - 2] = a1.x; av[TM - 1] = a1.y;
+        }
+      }
+      unsigned long long bv[TN / 2];
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
+      for (int g = 0; g < TN / 4; ++g) {
+        const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(&Bs[buf][kk][64 * g + tx * 4]);
+        bv[2 * g] = v.x;
+        bv[2 * g + 1] = v.y;
+      }
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+      for (int i = 0; i < TM; ++i) {
+        const unsigned long long a2 = dup2(av[i]);
+#pragma unroll
+        for (int j = 0; j < TN / 2; ++j) acc[i][j] = fma2(a2, bv[j], acc[i][j]);
+      }
     }
     if (kt + 1 < nk) sstore(buf ^ 1);
     __syncthreads();
@@ -314,16 +366,21 @@ ks_sgemm_tn_kernel(const float* __restrict__ A, const float* __restrict__ Bt,
   // the tiled layout's last block is written whole: columns past N get zeros
   const long long nw = kTiled ? (((long long)N + 31) & ~31LL) : N;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const long long m = m0 + (i < 4 ? ty * 4 + i : 64 + ty * 4 + (i - 4));
+  for (int i = 0; i < TM; ++i) {
+    const long long m = m0 + (i < 4 ? ty * 4 + i : 64 + ty * (TM - 4) + (i - 4));
     if (m >= M) continue;
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
+    for (int h = 0; h < TN / 4; ++h) {
       const long long n = n0 + h * 64 + tx * 4;
       float* dst = kTiled ? Cm + (((n >> 5) * M + m) << 5) + (n & 31) : Cm + m * ldc + n;
       float v[4];
 #pragma unroll
-      for (int e = 0; e < 4; ++e) v[e] = n + e < N ? acc[i][h * 4 + e] : 0.f;
+      for (int e = 0; e < 4; e += 2) {
+        float lo, hi;
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(acc[i][h * 2 + e / 2]));
+        v[e] = n + e < N ? lo : 0.f;
+        v[e + 1] = n + e + 1 < N ? hi : 0.f;
+      }
       if (n + 3 < nw && ((reinterpret_cast<uintptr_t>(dst) & 15) == 0)) {
         *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
       } else {
@@ -334,21 +391,58 @@ ks_sgemm_tn_kernel(const float* __restrict__ A, const float* __restrict__ Bt,
   }
 }
 
-int sgemm_tn(const float* A, const float* Bt, float* Cm, int64_t M, int64_t N,
-             int64_t Kd, int64_t ldc, cudaStream_t stream, bool tiled) {
-  if (Kd % kBK) return fail(KS_ERR_ARG, "sgemm_tn: Kd must be a multiple of 16");
-  const int tiles_m = (int)((M + kBM - 1) / kBM);
-  const int tiles_n = (int)((N + kBN - 1) / kBN);
+// Rows per tile: the height that covers M with the least work, a row of a lower
+// tile counted a little dearer (its loads serve fewer rows); the operand is
+// padded to 128 rows, which the tiles must not pass.
+static int sgemm_rows(int64_t M) {
+  const int64_t padded = round_up(M, 128);
+  int best = 128;
+  int64_t cost = padded * 100;
+  const int rows[2] = {96, 64}, weight[2] = {104, 112};
+  for (int i = 0; i < 2; ++i) {
+    const int64_t r = round_up(M, rows[i]);
+    if (r <= padded && r * weight[i] < cost) {
+      cost = r * weight[i];
+      best = rows[i];
+    }
+  }
+  return best;
+}
+
+template <int TM, int TN>
+static int launch_sgemm(const float* A, const float* Bt, float* Cm, int64_t M, int64_t N,
+                        int64_t Kd, int64_t ldc, cudaStream_t stream, bool tiled) {
+  const int tiles_m = (int)((M + 16 * TM - 1) / (16 * TM));
+  const int tiles_n = (int)((N + 16 * TN - 1) / (16 * TN));
   const long long nblocks = (long long)tiles_m * tiles_n;
   if (nblocks > 0x7fffffffLL) return fail(KS_ERR_UNSUPPORTED, "sgemm_tn: too many tiles");
-  if (tiled)
-    ks_sgemm_tn_kernel<true><<<(unsigned)nblocks, 256, 0, stream>>>(A, Bt, Cm, (int)M, (int)N,
-                                                                  (int)Kd, ldc, tiles_m);
-  else
-    ks_sgemm_tn_kernel<false><<<(unsigned)nblocks, 256, 0, stream>>>(A, Bt, Cm, (int)M, (int)N,
-                                                                   (int)Kd, ldc, tiles_m);
+  const size_t smem = sizeof(float) * 2 * sgemm_slice(TN) * (16 * TM + 4 + 16 * TN + 4);
+  const auto kernel = tiled ? ks_sgemm_tn_kernel<TM, TN, true> : ks_sgemm_tn_kernel<TM, TN, false>;
+  kernel<<<(unsigned)nblocks, 256, smem, stream>>>(A, Bt, Cm, (int)M, (int)N, (int)Kd, ldc, tiles_m);
   KS_CUDA(cudaGetLastError());
   return KS_OK;
+}
+
+int sgemm_tn(const float* A, const float* Bt, float* Cm, int64_t M, int64_t N,
+             int64_t Kd, int64_t ldc, cudaStream_t stream, bool tiled) {
+  if (Kd % 16) return fail(KS_ERR_ARG, "sgemm_tn: Kd must be a multiple of 16");
+  DeviceInfo dev;
+  const int rc = device_info(&dev);
+  if (rc) return rc;
+  const int rows = sgemm_rows(M);
+  // 256 columns need fewer shared-memory reads per multiply-add, one block per
+  // SM; with fewer than 2.5 tiles per SM their last wave costs more than that
+  // (80 x 60122 x 576: 249 us with 256 columns, 192 with 128; 3600 x 3600 x 384:
+  // 197 and 219)
+  const int64_t wide = ((M + rows - 1) / rows) * ((N + 255) / 256);
+  if (2 * wide >= 5 * dev.sm_count && rows != 64)
+    return rows == 96 ? launch_sgemm<6, 16>(A, Bt, Cm, M, N, Kd, ldc, stream, tiled)
+                      : launch_sgemm<8, 16>(A, Bt, Cm, M, N, Kd, ldc, stream, tiled);
+  switch (rows) {
+    case 64: return launch_sgemm<4, 8>(A, Bt, Cm, M, N, Kd, ldc, stream, tiled);
+    case 96: return launch_sgemm<6, 8>(A, Bt, Cm, M, N, Kd, ldc, stream, tiled);
+    default: return launch_sgemm<8, 8>(A, Bt, Cm, M, N, Kd, ldc, stream, tiled);
+  }
 }
 
 // ------------------------------------------------------------------ driver
