@@ -15,13 +15,15 @@
 // channels is staged, double-buffered by cp.async, the (s, k) sums of one
 // position over 32 samples per warp in registers; A is never stored;
 // ks_detect_scores_kernel is the form for more than 8192 channels),
-// ks_detect_peaks_kernel (a block per (f, 256-sample tile): only where the
-// score exceeds the threshold, the maximum over the neighbour rows and the
-// +-nt0 window, left at the first larger value; peak bits by warp ballot),
+// ks_detect_peaks_kernel (a block per (f, 1024-sample tile): only where the
+// score exceeds the threshold and both samples beside it, the maximum over the
+// neighbour rows and the +-nt0 window by a warp, left at the first larger
+// value),
 // count / scan / emit in (f, t) order, and one gather
 // kernel per spike (adist, y) and per (spike, channel) warp (features).
 #include "ks_common.cuh"
 #include "project.cuh"
+#include "residual_apply.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -122,27 +124,85 @@ __device__ __forceinline__ void cp_async_wait0() {
   asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
+// The largest magnitude of the sums a[size][waveform] of one sample (half h of
+// the packed pairs; -1 when all are NaN) and its signed index
+// (1 + size * nk + waveform) * sign, the first index on ties: the maximum of
+// each size (NaNs passed over), the first size that holds the largest, then its
+// first waveform.
+template <int NS, int NK>
+__device__ __forceinline__ int largest_magnitude(const unsigned long long (&a)[NS][NK], bool h,
+                                                 int ns, int nk, float& best) {
+  auto val = [&](int q, int k) {
+    float lo, hi;
+    f2_unpack(a[q][k], lo, hi);
+    return h ? hi : lo;
+  };
+  float mq[NS];
+  best = -1.f;
+#pragma unroll
+  for (int q = 0; q < NS; ++q) {
+    float m = fabsf(val(q, 0));
+#pragma unroll
+    for (int k = 1; k < NK; k += 2) {
+      if (k + 1 < NK && k + 1 < nk)
+        asm("max.f32 %0, %0, %1, %2;" : "+f"(m) : "f"(fabsf(val(q, k))), "f"(fabsf(val(q, k + 1 < NK ? k + 1 : k))));
+      else if (k < nk)
+        m = fmaxf(m, fabsf(val(q, k)));
+    }
+    mq[q] = m;
+    if (q < ns) best = fmaxf(best, m);
+  }
+  float v[NK], x = 0.f;
+  int qs = 0, ks = 0;
+#pragma unroll
+  for (int k = 0; k < NK; ++k) v[k] = 0.f;
+#pragma unroll
+  for (int q = NS - 1; q >= 0; --q) {
+    const bool p = q < ns && mq[q] == best;
+    qs = p ? q : qs;
+#pragma unroll
+    for (int k = 0; k < NK; ++k) v[k] = p ? val(q, k) : v[k];
+  }
+#pragma unroll
+  for (int k = NK - 1; k >= 0; --k) {
+    const bool p = k < nk && fabsf(v[k]) == best;
+    ks = p ? k : ks;
+    x = p ? v[k] : x;
+  }
+  const int idx = 1 + qs * nk + ks;
+  return x > 0.f ? idx : (x < 0.f ? -idx : 0);
+}
+
 // Persistent over time: block (position tile, y) takes the time tiles y,
 // y + gridDim.y, ...; the union of its positions' channels and their weights
 // are set up once, and the channels' convolution rows of the next time tile
 // are copied (cp.async, 16-byte pieces) while the current one is summed.
-template <int NS, int NK>
+//
+// What bounds it: the FP32 pipe and issue.  Two samples per lane through packed
+// multiply-adds (the weights held twice): 2.14 ms per C=384 batch of 60122
+// samples and 1532 positions; with one sample per lane 2.89 ms, with the channel
+// count not known at compile time 2.45 ms.
+template <int NS, int NK, int NCT>
 __global__ void __launch_bounds__(256)
 ks_detect_scores_tiled_kernel(const float* __restrict__ BT, long long ldb, int nk_rt, int C,
-                              const long long* __restrict__ iC, int nC,
+                              const long long* __restrict__ iC, int nC_rt,
                               const float* __restrict__ weigh, int ns_rt, int Nfilt, int L,
                               int n_ttiles, float* __restrict__ As,
                               signed char* __restrict__ imaxs, int* err) {
   // NS, NK: compile-time bounds of the sizes and waveforms; ns_rt, nk_rt the
-  // actual counts (equal to the bounds in the specialised instantiation)
+  // actual counts (equal to the bounds in the specialised instantiations); NCT:
+  // the nearest channels where they are known at compile time, else 0
   extern __shared__ __align__(16) float sm[];
+  const int nC = NCT ? NCT : nC_rt;
   float* sB = sm;                                                // [2][kMaxU][NK][kTT]
-  float* sw = sB + 2 * kMaxU * NK * kTT;                         // [kFT][nC][NS]
-  unsigned* bitmap = reinterpret_cast<unsigned*>(sw + kFT * NS * nC);   // [kMaxCBits / 32]
+  constexpr int kWS = (NS + 1) & ~1;                             // sizes, padded to pairs
+  unsigned long long* sw = reinterpret_cast<unsigned long long*>(sB + 2 * kMaxU * NK * kTT);
+                                                                 // [kFT][nC][kWS], each twice
+  unsigned* bitmap = reinterpret_cast<unsigned*>(sw + kFT * kWS * nC);  // [kMaxCBits / 32]
   int* wpre = reinterpret_cast<int*>(bitmap + kMaxCBits / 32);   // [kMaxCBits / 32]
   int* ulist = wpre + kMaxCBits / 32;                            // [kMaxU]
   int* cidx = ulist + kMaxU;                                     // [kMaxNC][kFT] channel
-  int* loc = cidx + kMaxNC * kFT;                                // [kMaxNC][kFT] union slot
+  int* loc = cidx + kMaxNC * kFT;                                // [kMaxNC][kFT] its rows' offset
   __shared__ int nU;
   const int ns = NS == kMaxNS ? ns_rt : NS;
   const int nk = NK == kMaxNK ? nk_rt : NK;
@@ -163,10 +223,11 @@ ks_detect_scores_tiled_kernel(const float* __restrict__ BT, long long ldb, int n
     atomicOr(bitmap + (c >> 5), 1u << (c & 31));
   }
   // weights [fl][j][q] (zero for missing sizes and positions)
-  for (int e = threadIdx.x; e < kFT * nC * NS; e += blockDim.x) {
-    const int fl = e / (nC * NS), r = e - fl * nC * NS, j = r / NS, q = r % NS;
+  for (int e = threadIdx.x; e < kFT * nC * kWS; e += blockDim.x) {
+    const int fl = e / (nC * kWS), r = e - fl * nC * kWS, j = r / kWS, q = r % kWS;
     const int f = f0 + fl;
-    sw[e] = (f < Nfilt && q < ns) ? weigh[((long long)q * nC + j) * Nfilt + f] : 0.f;
+    const float v = (f < Nfilt && q < ns) ? weigh[((long long)q * nC + j) * Nfilt + f] : 0.f;
+    sw[e] = f2_pack(v, v);
   }
   __syncthreads();
   if (threadIdx.x < 32) {
@@ -189,8 +250,9 @@ ks_detect_scores_tiled_kernel(const float* __restrict__ BT, long long ldb, int n
   const bool staged = nU <= kMaxU;
   for (int e = threadIdx.x; e < nC * kFT; e += blockDim.x) {
     const int c = cidx[e];
-    loc[e] = wpre[c >> 5] + __popc(bitmap[c >> 5] & ((1u << (c & 31)) - 1u));
-    if (staged) ulist[loc[e]] = c;
+    const int u = wpre[c >> 5] + __popc(bitmap[c >> 5] & ((1u << (c & 31)) - 1u));
+    loc[e] = u * NK * kTT;
+    if (staged) ulist[u] = c;
   }
   __syncthreads();
   // rows (u, k) of a time tile: kTT floats = kTT/4 16-byte pieces each
@@ -216,59 +278,59 @@ ks_detect_scores_tiled_kernel(const float* __restrict__ BT, long long ldb, int n
     else cp_async_commit();
     cp_async_wait1();
     __syncthreads();
-    const float* cur = sB + buf * kMaxU * NK * kTT;
-    const int t = tt * kTT + lane;
-    for (int fl = warp; fl < kFT; fl += 8) {
+    const float* cur = sB + buf * kMaxU * NK * kTT + 2 * (lane & 15);
+    // half a warp per position, two samples per lane
+    const int t = tt * kTT + 2 * (lane & 15);
+    for (int fl = 2 * warp + (lane >> 4); fl < kFT; fl += 16) {
       const int f = f0 + fl;
-      float a[NS][NK];
+      unsigned long long a[NS][NK];
 #pragma unroll
       for (int q = 0; q < NS; ++q)
 #pragma unroll
-        for (int k = 0; k < NK; ++k) a[q][k] = 0.f;
+        for (int k = 0; k < NK; ++k) a[q][k] = 0ull;
+#pragma unroll (NCT ? NCT : 1)
       for (int j = 0; j < nC; ++j) {
-        float bk[NK];
+        unsigned long long bk[NK];
         if (staged) {
-          const float* b = cur + (loc[j * kFT + fl] * NK) * kTT + lane;
+          const float* b = cur + loc[j * kFT + fl];
 #pragma unroll
-          for (int k = 0; k < NK; ++k) bk[k] = b[k * kTT];
+          for (int k = 0; k < NK; ++k) bk[k] = *reinterpret_cast<const unsigned long long*>(b + k * kTT);
         } else {
           const float* b = BT + (long long)cidx[j * kFT + fl] * nk * ldb + t;
 #pragma unroll
-          for (int k = 0; k < NK; ++k) bk[k] = k < nk ? __ldg(b + (long long)k * ldb) : 0.f;
+          for (int k = 0; k < NK; ++k)
+            bk[k] = k < nk ? __ldg(reinterpret_cast<const unsigned long long*>(b + (long long)k * ldb))
+                           : 0ull;
         }
-        const float* w = sw + (fl * nC + j) * NS;
+        const unsigned long long* w = sw + (fl * nC + j) * kWS;
 #pragma unroll
-        for (int q = 0; q < NS; ++q) {
-          const float wq = w[q];
+        for (int q = 0; q < NS; q += 2) {
+          const ulonglong2 wq = *reinterpret_cast<const ulonglong2*>(w + q);
 #pragma unroll
-          for (int k = 0; k < NK; ++k) a[q][k] = fmaf(wq, bk[k], a[q][k]);
+          for (int k = 0; k < NK; ++k) {
+            f2_fma_acc(a[q][k], wq.x, bk[k]);
+            if (q + 1 < NS) f2_fma_acc(a[q + 1][k], wq.y, bk[k]);
+          }
         }
       }
-      // largest magnitude, first index in (size, waveform) order: the
-      // maximum first (NaN never wins, as in a strict > scan), then the first
-      // entry that reaches it
-      float best = -1.f, bval = 0.f;
-      int bidx = 0;
-#pragma unroll
-      for (int q = 0; q < NS; ++q)
-#pragma unroll
-        for (int k = 0; k < NK; ++k)
-          if (q < ns && k < nk) best = fmaxf(best, fabsf(a[q][k]));
-      bool found = false;
-#pragma unroll
-      for (int q = NS - 1; q >= 0; --q)
-#pragma unroll
-        for (int k = NK - 1; k >= 0; --k)
-          if (q < ns && k < nk && fabsf(a[q][k]) == best) {
-            found = true;
-            bval = a[q][k];
-            bidx = q * nk + k;
+      float best0, best1;
+      const int i0 = largest_magnitude<NS, NK>(a, false, ns, nk, best0);
+      const int i1 = largest_magnitude<NS, NK>(a, true, ns, nk, best1);
+      if (f < Nfilt) {
+        const long long o = (long long)f * L + t;
+        if (t + 1 < L && (o & 1) == 0) {
+          *reinterpret_cast<float2*>(As + o) = make_float2(best0, best1);
+          *reinterpret_cast<char2*>(imaxs + o) = make_char2((signed char)i0, (signed char)i1);
+        } else {
+          if (t < L) {
+            As[o] = best0;
+            imaxs[o] = (signed char)i0;
           }
-      if (!found) best = -1.f;
-      if (f < Nfilt && t < L) {
-        const int sg = bval > 0.f ? 1 : (bval < 0.f ? -1 : 0);
-        As[(long long)f * L + t] = best;
-        imaxs[(long long)f * L + t] = (signed char)((1 + bidx) * sg);
+          if (t + 1 < L) {
+            As[o + 1] = best1;
+            imaxs[o + 1] = (signed char)i1;
+          }
+        }
       }
     }
     __syncthreads();          // the buffer is read: the next fetch may reuse it
@@ -279,75 +341,142 @@ ks_detect_scores_tiled_kernel(const float* __restrict__ BT, long long ldb, int n
 
 size_t scores_tiled_smem(int NK, int NS, int nC) {
   return sizeof(unsigned) * (kMaxCBits / 32) * 2 + sizeof(int) * (kMaxU + 2 * kMaxNC * kFT) +
-         sizeof(float) * ((size_t)kFT * NS * nC + 2 * (size_t)kMaxU * NK * kTT);
+         sizeof(float) * (2 * (size_t)kFT * ((NS + 1) & ~1) * nC + 2 * (size_t)kMaxU * NK * kTT);
 }
 
-template <int NS, int NK>
+template <int NS, int NK, int NCT>
 int launch_scores_tiled(const float* BT, long long ldb, int nk, int C, const long long* iC,
                         int nC, const float* weigh, int ns, int Nfilt, int L, float* As,
                         signed char* ims, int* err, cudaStream_t s) {
   const size_t smem = scores_tiled_smem(NK, NS, nC);
-  KS_CUDA(cudaFuncSetAttribute(ks_detect_scores_tiled_kernel<NS, NK>,
+  KS_CUDA(cudaFuncSetAttribute(ks_detect_scores_tiled_kernel<NS, NK, NCT>,
                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   ks::DeviceInfo dev;
   int rc = ks::device_info(&dev);
   if (rc) return rc;
   int occ = 0;
-  KS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, ks_detect_scores_tiled_kernel<NS, NK>,
+  KS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, ks_detect_scores_tiled_kernel<NS, NK, NCT>,
                                                         256, smem));
   const int ftiles = (Nfilt + kFT - 1) / kFT;
   const int n_ttiles = (L + kTT - 1) / kTT;
   // about one wave of resident blocks, each walking its share of the time tiles
   const int gy = std::max(1, std::min(n_ttiles, std::max(occ, 1) * dev.sm_count / ftiles));
   const dim3 grid((unsigned)ftiles, (unsigned)gy);
-  ks_detect_scores_tiled_kernel<NS, NK><<<grid, 256, smem, s>>>(BT, ldb, nk, C, iC, nC, weigh,
+  ks_detect_scores_tiled_kernel<NS, NK, NCT><<<grid, 256, smem, s>>>(BT, ldb, nk, C, iC, nC, weigh,
                                                                 ns, Nfilt, L, n_ttiles, As, ims,
                                                                 err);
   KS_CUDA(cudaGetLastError());
   return KS_OK;
 }
 
-// Peak test, one block per (f, tile), one thread per sample.  The reference's
-// test, pooled == As[f, t] && As[f, t] > th with pooled the max-pool over
-// +-nt0 of the neighbour maximum (0 at the batch edges), needs the neighbour
-// maximum only where As[f, t] > th: there the thread walks the nC2 neighbour
-// rows over the window, keeping the running maximum from 0 as the max-pool
-// does, and stops after the first row that lifts it above As[f, t] (the
-// sample is then no peak; most candidates stop at the first rows, the nearest
-// positions).  Maxima are exact, so the order of the walk does not matter.
-// (A warp walking one candidate at a time, a lane per row, measured 6x
-// slower: candidates are many and most stop within one row.)
-__global__ void __launch_bounds__(kTile)
+// Peak test, one block per (position f, 1024 samples).  The reference's test,
+// pooled == As[f, t] && As[f, t] > th with pooled the max-pool over +-nt0 of
+// the neighbour maximum (0 at the batch edges), needs the neighbour maximum
+// only where As[f, t] > th and, when f is one of its own neighbours (the nearest
+// position), neither sample beside it in its own row is larger.  Those
+// survivors are collected, and a warp walks the rows of one at a time, its own
+// row first, a lane per sample, stopping after the rows that lift the running
+// maximum above As[f, t].  Maxima are exact, so the order of the walk does not
+// matter.
+//
+// What bounds it: reading As once (368 MB at C=384, 1532 positions, 60122
+// samples) and the survivors' walks: 660 us; with every sample above the
+// threshold walking the rows in its own thread 1755 us, with one row of a
+// survivor in flight at a time 1290 us, with a position's tiles one after the
+// other in one block 1900 us.
+constexpr int kPeakTile = 1024;
+constexpr int kPeakHalo = 512;   // staged beside the tile; a wider window's own row is read
+                                 // from global memory
+__global__ void __launch_bounds__(256)
 ks_detect_peaks_kernel(const float* __restrict__ As, const long long* __restrict__ iC2,
                        int nC2, int Nfilt, int L, int nt, int nt0, float th,
                        unsigned* __restrict__ bits, int nwords) {
   extern __shared__ float sm[];
-  int* snb = reinterpret_cast<int*>(sm);           // [nC2]
+  const int halo = nt0 <= kPeakHalo ? nt0 : 0;
+  float* row = sm;                                           // [kPeakTile + 2 halo]
+  int* snb = reinterpret_cast<int*>(row + kPeakTile + 2 * halo);  // [nC2]
+  __shared__ int list[kPeakTile];
+  __shared__ unsigned sbits[kPeakTile / 32];
+  __shared__ int nlist, taken, self;
   const int f = blockIdx.x;
-  const int t0 = blockIdx.y * kTile;
-  for (int j = threadIdx.x; j < nC2; j += kTile) {
-    long long g = iC2[(long long)j * Nfilt + f];
-    snb[j] = (int)(g < 0 ? f : (g >= Nfilt ? f : g));
+  const int lane = threadIdx.x & 31;
+  const int t0 = blockIdx.y * kPeakTile;
+  if (threadIdx.x < kPeakTile / 32) sbits[threadIdx.x] = 0u;
+  if (threadIdx.x == 0) nlist = taken = self = 0;
+  // neighbour values exist for samples nt .. L-nt-1 only (0 elsewhere)
+  const float* own = As + (long long)f * L;
+  bool any = false;
+  for (int i = threadIdx.x; i < kPeakTile + 2 * halo; i += 256) {
+    const int t = t0 - halo + i;
+    const bool in = t >= 0 && t < L;
+    const float v = in ? own[t] : 0.f;
+    row[i] = v;
+    any |= in && i >= halo && i < halo + kPeakTile && v > th;
   }
-  __syncthreads();
-  const int t = t0 + threadIdx.x;
-  bool peak = false;
-  if (t < L) {
-    const float a = As[(long long)f * L + t];
-    if (a > th) {
-      // neighbour values exist for samples nt .. L-nt-1 only (0 elsewhere)
-      const int lo = max(t - nt0, nt), hi = min(t + nt0, L - nt - 1);
-      float m = 0.f;
-      for (int j = 0; j < nC2 && !(m > a); ++j) {
-        const float* row = As + (long long)snb[j] * L;
-        for (int u = lo; u <= hi; ++u) m = fmaxf(m, row[u]);
+  if (__syncthreads_or(any)) {
+    for (int j = threadIdx.x; j < nC2; j += 256) {
+      const long long g = iC2[(long long)j * Nfilt + f];
+      const int n = (int)(g < 0 ? f : (g >= Nfilt ? f : g));
+      snb[j] = n;
+      if (n == f) self = 1;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < kPeakTile; i += 256) {
+      const int t = t0 + i;
+      const float a = row[halo + i];
+      bool keep = t < L && a > th;
+      if (keep && self && halo > 0) {
+        const int lo = max(t - nt0, nt), hi = min(t + nt0, L - nt - 1);
+        keep = !(t - 1 >= lo && t - 1 <= hi && row[halo + i - 1] > a) &&
+               !(t + 1 <= hi && t + 1 >= lo && row[halo + i + 1] > a);
       }
-      peak = m == a;
+      const unsigned b = __ballot_sync(0xffffffffu, keep);
+      if (b) {
+        int o = 0;
+        if (lane == 0) o = atomicAdd(&nlist, __popc(b));
+        o = __shfl_sync(0xffffffffu, o, 0);
+        if (keep) list[o + __popc(b & ((1u << lane) - 1u))] = i;
+      }
+    }
+    __syncthreads();
+    while (true) {
+      int e = 0;
+      if (lane == 0) e = atomicAdd(&taken, 1);
+      e = __shfl_sync(0xffffffffu, e, 0);
+      if (e >= nlist) break;
+      const int i = list[e], t = t0 + i;
+      const float a = row[halo + i];
+      const int lo = max(t - nt0, nt), n = min(t + nt0, L - nt - 1) - lo + 1;
+      float m = 0.f;                    // the lane's maximum
+      bool over = false;
+      if (self && halo == nt0) {        // the position's own row, staged
+        const float* p = row + (lo - t0 + halo);
+        for (int u = lane; u < n; u += 32) m = fmaxf(m, p[u]);
+        over = __any_sync(0xffffffffu, m > a);
+      }
+      // four rows' windows (up to 64 samples each at a time) in flight together
+      for (int j = 0; j < nC2 && !over; j += 4) {
+        for (int u = lane; u - lane < n; u += 64) {
+          float v[8];
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            const float* p = As + (long long)snb[min(j + r, nC2 - 1)] * L + lo;
+            v[2 * r] = u < n ? p[u] : 0.f;
+            v[2 * r + 1] = u + 32 < n ? p[u + 32] : 0.f;
+          }
+#pragma unroll
+          for (int r = 0; r < 8; ++r) m = fmaxf(m, v[r]);
+        }
+        over = __any_sync(0xffffffffu, m > a);
+      }
+      const bool reached = __any_sync(0xffffffffu, m == a);
+      if (lane == 0 && !over && reached) atomicOr(&sbits[i >> 5], 1u << (i & 31));
     }
   }
-  const unsigned w = __ballot_sync(0xffffffffu, peak);
-  const int word = (t0 >> 5) + (threadIdx.x >> 5);
-  if ((threadIdx.x & 31) == 0 && word < nwords) bits[(long long)f * nwords + word] = w;
+  __syncthreads();
+  const int word = (t0 >> 5) + threadIdx.x;
+  if (threadIdx.x < kPeakTile / 32 && word < nwords)
+    bits[(long long)f * nwords + word] = sbits[threadIdx.x];
 }
 
 __global__ void ks_detect_count_kernel(const unsigned* __restrict__ bits, int Nfilt, int nwords,
@@ -361,29 +490,50 @@ __global__ void ks_detect_count_kernel(const unsigned* __restrict__ bits, int Nf
   counts[e] = n;
 }
 
-// Exclusive scan of n counts in place (one block), total in *total.
+// Exclusive scan of n counts in place (one block), total in *total: tiles of 8
+// values per thread, the next tile's loads in flight while this one is
+// scanned (97 us per 90000 counts with one contiguous run per thread).
 __global__ void __launch_bounds__(1024)
 ks_detect_scan_kernel(long long* __restrict__ counts, long long n, long long* __restrict__ total) {
-  __shared__ long long part[1024];
-  const long long per = (n + 1023) / 1024;
-  const long long a = threadIdx.x * per, b = min(n, a + per);
-  long long s = 0;
-  for (long long i = a; i < b; ++i) s += counts[i];
-  part[threadIdx.x] = s;
-  __syncthreads();
-  for (int o = 1; o < 1024; o <<= 1) {
-    const long long v = threadIdx.x >= o ? part[threadIdx.x - o] : 0;
+  __shared__ long long wsum[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  long long v[8];
+  auto load = [&](long long i) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = i + j < n ? counts[i + j] : 0;
+  };
+  long long carry = 0;
+  load(8LL * threadIdx.x);
+  for (long long base = 0; base < n; base += 8 * 1024) {
+    const long long i = base + 8LL * threadIdx.x;
+    long long e[8], run = 0;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      e[j] = run;
+      run += v[j];
+    }
+    load(i + 8 * 1024);
+    long long incl = run;
+    for (int o = 1; o < 32; o <<= 1) {
+      const long long x = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += x;
+    }
     __syncthreads();
-    part[threadIdx.x] += v;
+    if (lane == 31) wsum[warp] = incl;
     __syncthreads();
+    long long w = wsum[lane];
+    for (int o = 1; o < 32; o <<= 1) {
+      const long long x = __shfl_up_sync(0xffffffffu, w, o);
+      if (lane >= o) w += x;
+    }
+    const long long prev = __shfl_sync(0xffffffffu, w, max(warp - 1, 0));
+    const long long before = carry + incl - run + (warp ? prev : 0);
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (i + j < n) counts[i + j] = before + e[j];
+    carry += __shfl_sync(0xffffffffu, w, 31);
   }
-  long long run = part[threadIdx.x] - s;
-  for (long long i = a; i < b; ++i) {
-    const long long c = counts[i];
-    counts[i] = run;
-    run += c;
-  }
-  if (threadIdx.x == 1023) *total = part[1023];
+  if (threadIdx.x == 0) *total = carry;
 }
 
 __global__ void ks_detect_emit_kernel(const unsigned* __restrict__ bits, int Nfilt, int nwords,
@@ -585,13 +735,13 @@ extern "C" KS_API int ks_detect(const float* X, int64_t C, int64_t L, const floa
   if (rc) return rc;
   // 2. scores over sizes and waveforms
   if (C <= kMaxCBits) {
-    // the reference's defaults (5 sizes, 6 waveforms) have their own instantiation
-    rc = (nsizes == 5 && nk == 6)
-             ? launch_scores_tiled<5, 6>(BT, d.Lpad, (int)nk, (int)C, iCl, (int)nC, weigh,
-                                         (int)nsizes, (int)Nfilt, (int)L, As, ims, err, s)
-             : launch_scores_tiled<kMaxNS, kMaxNK>(BT, d.Lpad, (int)nk, (int)C, iCl, (int)nC,
-                                                   weigh, (int)nsizes, (int)Nfilt, (int)L, As,
-                                                   ims, err, s);
+    // the reference's defaults (5 sizes, 6 waveforms, 10 channels) and their sizes
+    // and waveforms with other channel counts have their own instantiations
+    const auto launch = nsizes == 5 && nk == 6 ? (nC == 10 ? launch_scores_tiled<5, 6, 10>
+                                                           : launch_scores_tiled<5, 6, 0>)
+                                               : launch_scores_tiled<kMaxNS, kMaxNK, 0>;
+    rc = launch(BT, d.Lpad, (int)nk, (int)C, iCl, (int)nC, weigh, (int)nsizes, (int)Nfilt, (int)L,
+                As, ims, err, s);
     if (rc) return rc;
   } else {
     const dim3 grid((unsigned)Nfilt, (unsigned)((L + kTile - 1) / kTile));
@@ -601,12 +751,13 @@ extern "C" KS_API int ks_detect(const float* X, int64_t C, int64_t L, const floa
   }
   // 3. neighbour maximum, max-pool, peaks
   {
-    const size_t smem = sizeof(int) * (size_t)nC2;
-    if (smem > 200 * 1024) return fail(KS_ERR_UNSUPPORTED, "ks_detect: nC2 too large");
+    const size_t smem = sizeof(int) * (size_t)nC2 +
+                        sizeof(float) * (size_t)(kPeakTile + 2 * (nt0 <= kPeakHalo ? nt0 : 0));
+    if (sizeof(int) * (size_t)nC2 > 200 * 1024) return fail(KS_ERR_UNSUPPORTED, "ks_detect: nC2 too large");
     KS_CUDA(cudaFuncSetAttribute(ks_detect_peaks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)smem));
-    const dim3 grid((unsigned)Nfilt, (unsigned)((L + kTile - 1) / kTile));
-    ks_detect_peaks_kernel<<<grid, kTile, smem, s>>>(As, iC2l, (int)nC2, (int)Nfilt, (int)L,
+    const dim3 grid((unsigned)Nfilt, (unsigned)((L + kPeakTile - 1) / kPeakTile));
+    ks_detect_peaks_kernel<<<grid, 256, smem, s>>>(As, iC2l, (int)nC2, (int)Nfilt, (int)L,
                                                      (int)nt, (int)nt0, th, bits, (int)d.nwords);
     KS_CUDA(cudaGetLastError());
   }

@@ -22,6 +22,11 @@ __device__ __forceinline__ unsigned long long f2_fma(unsigned long long a, unsig
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
   return r;
 }
+// c += a b in place.
+__device__ __forceinline__ void f2_fma_acc(unsigned long long& c, unsigned long long a,
+                                           unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b));
+}
 __device__ __forceinline__ unsigned long long f2_mul(unsigned long long a, unsigned long long b) {
   unsigned long long r;
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
