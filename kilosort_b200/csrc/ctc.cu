@@ -3,10 +3,14 @@
 //   G[(i,k), (j,m)] = sum_c U[i,k,c] * U[j,m,c]            (Gram of U rows)
 //   ctc[i, j, l] = sum_{k,m} G[(i,k), (j,m)] * WtW[k, m, l]
 // G is one FP32 contraction over channels (the TN SIMT GEMM of the
-// projection); the lag contraction is a small per-(i, j-tile) kernel.
+// projection), symmetric element by element (the same products in the same
+// order), so ctc computes its upper tiles only; the lag contraction is a
+// per-(i, j-tile) kernel.
 #include "ks_common.cuh"
 #include "project.cuh"
+#include "residual_apply.cuh"
 
+#include <algorithm>
 #include <cmath>
 
 namespace ks {
@@ -27,31 +31,83 @@ __global__ void ks_wtw_kernel(const float* __restrict__ W, int P, int nt,
 
 constexpr int kCtcJ = 16;
 
+// ctc[i, j, l] for one i and the tiles of NG * 16 templates j blockIdx.x, +
+// gridDim.x, ...: group g of 128 threads takes 16 of a tile's j, a thread one
+// lag for all of them, j in pairs through packed multiply-adds.  G is symmetric
+// and only its upper triangle is read (row <= column).
+//
+// What bounds it: the FP32 pipe (36 multiply-adds per output at P = 6) next to
+// the 4 K^2 (2nt+1) bytes written: 180 us at K = 600, where one output per
+// thread and two shared-memory reads per multiply-add took 449 us.
+// PT: the components where they are known at compile time (6), else 0.
+template <int PT>
 __global__ void __launch_bounds__(256)
 ks_ctc_lag_kernel(const float* __restrict__ G, long long ldg,
-                  const float* __restrict__ WtW, int K, int P, int nt,
+                  const float* __restrict__ WtW, int K, int P_rt, int nt, int ng,
                   float* __restrict__ ctc) {
-  extern __shared__ float sm[];
-  const int nlag = 2 * nt + 1;
-  float* sWtW = sm;                   // [P*P][nlag]
-  float* sG = sm + P * P * nlag;      // [kCtcJ][P][P]  (j, k, m)
+  extern __shared__ __align__(16) float sm[];
+  const int P = PT ? PT : P_rt;
+  const int nlag = 2 * nt + 1, P2 = P * P;
+  float* sG = sm;                          // [ng][P2][kCtcJ]
+  float* sWtW = sm + ng * P2 * kCtcJ;      // [P2][nlag]
   const int i = blockIdx.y;
-  const int j0 = blockIdx.x * kCtcJ;
-  for (int e = threadIdx.x; e < P * P * nlag; e += blockDim.x) sWtW[e] = WtW[e];
-  for (int e = threadIdx.x; e < kCtcJ * P * P; e += blockDim.x) {
-    const int jj = e / (P * P), km = e % (P * P);
-    const int k = km / P, m = km % P;
-    const int j = j0 + jj;
-    sG[e] = (j < K) ? G[(long long)(i * P + k) * ldg + (long long)j * P + m] : 0.f;
-  }
-  __syncthreads();
-  for (int e = threadIdx.x; e < kCtcJ * nlag; e += blockDim.x) {
-    const int jj = e / nlag, l = e % nlag;
-    const int j = j0 + jj;
-    if (j >= K) continue;
-    float s = 0.f;
-    for (int km = 0; km < P * P; ++km) s = fmaf(sG[jj * P * P + km], sWtW[km * nlag + l], s);
-    ctc[((long long)i * K + j) * nlag + l] = s;
+  const int grp = threadIdx.x >> 7, lt = threadIdx.x & 127;
+  const int step = ng * kCtcJ;
+  for (int e = threadIdx.x; e < P2 * nlag; e += 256) sWtW[e] = WtW[e];
+  for (int j0 = blockIdx.x * step; j0 < K; j0 += gridDim.x * step) {
+    __syncthreads();                       // the previous tile is read
+    for (int e = threadIdx.x; e < step * P2; e += 256) {
+      // consecutive threads along the row that is read: (j, m) right of the
+      // diagonal, k left of it
+      int k, jj, m;
+      if (j0 >= i) {
+        k = e / (step * P);
+        const int r = e - k * step * P;
+        jj = r / P;
+        m = r - jj * P;
+      } else {
+        const int r = e / P;
+        k = e - r * P;
+        jj = r / P;
+        m = r - jj * P;
+      }
+      const int j = j0 + jj;
+      float v = 0.f;
+      if (j < K) {
+        const long long a = (long long)i * P + k, b = (long long)j * P + m;
+        v = a <= b ? G[a * ldg + b] : G[b * ldg + a];
+      }
+      sG[((jj / kCtcJ) * P2 + k * P + m) * kCtcJ + jj % kCtcJ] = v;
+    }
+    __syncthreads();
+    if (grp >= ng) continue;
+    const int jb = j0 + grp * kCtcJ;
+    for (int l = lt; l < nlag; l += 128) {
+      unsigned long long acc[kCtcJ / 2];
+#pragma unroll
+      for (int q = 0; q < kCtcJ / 2; ++q) acc[q] = 0ull;
+      const ulonglong2* g = reinterpret_cast<const ulonglong2*>(sG + grp * P2 * kCtcJ);
+      const float* w = sWtW + l;
+#pragma unroll 4
+      for (int km = 0; km < P2; ++km) {
+        const float wv = w[km * nlag];
+        const unsigned long long w2 = f2_pack(wv, wv);
+#pragma unroll
+        for (int q = 0; q < kCtcJ / 4; ++q) {
+          const ulonglong2 v = g[km * (kCtcJ / 4) + q];
+          f2_fma_acc(acc[2 * q], v.x, w2);
+          f2_fma_acc(acc[2 * q + 1], v.y, w2);
+        }
+      }
+      float* out = ctc + ((long long)i * K + jb) * nlag + l;
+#pragma unroll
+      for (int q = 0; q < kCtcJ / 2; ++q) {
+        float lo, hi;
+        f2_unpack(acc[q], lo, hi);
+        if (jb + 2 * q < K) out[(long long)(2 * q) * nlag] = lo;
+        if (jb + 2 * q + 1 < K) out[(long long)(2 * q + 1) * nlag] = hi;
+      }
+    }
   }
 }
 
@@ -151,12 +207,22 @@ int launch_ctc(const float* U, const float* W, int64_t K, int64_t P, int64_t C,
   const int nw = (int)(P * P * (2 * nt + 1));
   ks_wtw_kernel<<<(nw + 255) / 256, 256, 0, stream>>>(W, (int)P, (int)nt, WtW);
   KS_CUDA(cudaGetLastError());
-  int rc = sgemm_tn(Upad, Upad, G, K * P, K * P, lay.cols, lay.ldg, stream, false);
+  int rc = sgemm_tn(Upad, Upad, G, K * P, K * P, lay.cols, lay.ldg, stream, false, true);
   if (rc) return rc;
-  const size_t smem = sizeof(float) * (P * P * (2 * nt + 1) + kCtcJ * P * P);
-  KS_CUDA(cudaFuncSetAttribute(ks_ctc_lag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  dim3 grid((unsigned)((K + kCtcJ - 1) / kCtcJ), (unsigned)K);
-  ks_ctc_lag_kernel<<<grid, 256, smem, stream>>>(G, lay.ldg, WtW, (int)K, (int)P, (int)nt, ctc);
+  DeviceInfo dev;
+  if ((rc = device_info(&dev))) return rc;
+  // two groups of 16 templates per block where their Gram blocks fit
+  const size_t wtw = sizeof(float) * P * P * (2 * nt + 1), per = sizeof(float) * kCtcJ * P * P;
+  const int ng = wtw + 2 * per <= dev.smem_optin ? 2 : 1;
+  const size_t smem = wtw + ng * per;
+  const auto kernel = P == 6 ? ks_ctc_lag_kernel<6> : ks_ctc_lag_kernel<0>;
+  KS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // a block keeps the basis correlations over several tiles of templates: about
+  // eight blocks per SM in all
+  const int64_t tiles = (K + ng * kCtcJ - 1) / (ng * kCtcJ);
+  const int64_t gx = std::min<int64_t>(tiles, std::max<int64_t>(1, (8LL * dev.sm_count + K - 1) / K));
+  dim3 grid((unsigned)gx, (unsigned)K);
+  kernel<<<grid, 256, smem, stream>>>(G, lay.ldg, WtW, (int)K, (int)P, (int)nt, ng, ctc);
   KS_CUDA(cudaGetLastError());
   return KS_OK;
 }

@@ -252,7 +252,8 @@ __device__ __forceinline__ unsigned long long dup2(float v) {
 // operations over q; A is [>= tiles_m*BM, Kd], Bt is [>= tiles_n*128, Kd]
 // (both zero padded), Kd % 16 == 0.  Stores m < M, n < N, row-major with
 // leading dimension ldc, or (kTiled) in 32-column blocks
-// C[((n/32)*M + m)*32 + n%32].  Tiles of BM = 16 TM rows x 128 columns, TM x 8
+// C[((n/32)*M + m)*32 + n%32]; `upper` leaves out the tiles below the diagonal.
+// Tiles of BM = 16 TM rows x 128 columns, TM x 8
 // per thread, columns two at a time through packed operations.
 //
 // What bounds it: the FP32 pipe.  A packed operation does the work of two
@@ -268,7 +269,7 @@ template <int TM, int TN, bool kTiled>
 __global__ void __launch_bounds__(256, TN == 8 ? 2 : 1)
 ks_sgemm_tn_kernel(const float* __restrict__ A, const float* __restrict__ Bt,
                    float* __restrict__ Cm, int M, int N, int Kd, long long ldc,
-                   int tiles_m) {
+                   int tiles_m, bool upper) {
   constexpr int BM = 16 * TM, BN = 16 * TN, BK = sgemm_slice(TN);
   constexpr int kP = BK / 4;                           // 16-byte pieces of a row's slice
   constexpr int kALoads = (BM * kP + 255) / 256, kBLoads = BN * kP / 256;
@@ -279,6 +280,7 @@ ks_sgemm_tn_kernel(const float* __restrict__ A, const float* __restrict__ Bt,
   const int tm = blockIdx.x % tiles_m;
   const int tn = blockIdx.x / tiles_m;
   const long long m0 = (long long)tm * BM, n0 = (long long)tn * BN;
+  if (upper && n0 + BN <= m0) return;                  // below the diagonal
   const long long last = ((N + 127LL) & ~127LL) - 1;   // the operand's last (padded) row
   const int tx = tid & 15, ty = tid >> 4;
   // a thread's pieces: row idx / kP, columns 4 (idx % kP) of the slice
@@ -411,20 +413,22 @@ static int sgemm_rows(int64_t M) {
 
 template <int TM, int TN>
 static int launch_sgemm(const float* A, const float* Bt, float* Cm, int64_t M, int64_t N,
-                        int64_t Kd, int64_t ldc, cudaStream_t stream, bool tiled) {
+                        int64_t Kd, int64_t ldc, cudaStream_t stream, bool tiled,
+                        bool upper) {
   const int tiles_m = (int)((M + 16 * TM - 1) / (16 * TM));
   const int tiles_n = (int)((N + 16 * TN - 1) / (16 * TN));
   const long long nblocks = (long long)tiles_m * tiles_n;
   if (nblocks > 0x7fffffffLL) return fail(KS_ERR_UNSUPPORTED, "sgemm_tn: too many tiles");
   const size_t smem = sizeof(float) * 2 * sgemm_slice(TN) * (16 * TM + 4 + 16 * TN + 4);
   const auto kernel = tiled ? ks_sgemm_tn_kernel<TM, TN, true> : ks_sgemm_tn_kernel<TM, TN, false>;
-  kernel<<<(unsigned)nblocks, 256, smem, stream>>>(A, Bt, Cm, (int)M, (int)N, (int)Kd, ldc, tiles_m);
+  kernel<<<(unsigned)nblocks, 256, smem, stream>>>(A, Bt, Cm, (int)M, (int)N, (int)Kd, ldc, tiles_m,
+                                               upper);
   KS_CUDA(cudaGetLastError());
   return KS_OK;
 }
 
 int sgemm_tn(const float* A, const float* Bt, float* Cm, int64_t M, int64_t N,
-             int64_t Kd, int64_t ldc, cudaStream_t stream, bool tiled) {
+             int64_t Kd, int64_t ldc, cudaStream_t stream, bool tiled, bool upper) {
   if (Kd % 16) return fail(KS_ERR_ARG, "sgemm_tn: Kd must be a multiple of 16");
   DeviceInfo dev;
   const int rc = device_info(&dev);
@@ -436,12 +440,12 @@ int sgemm_tn(const float* A, const float* Bt, float* Cm, int64_t M, int64_t N,
   // 197 and 219)
   const int64_t wide = ((M + rows - 1) / rows) * ((N + 255) / 256);
   if (2 * wide >= 5 * dev.sm_count && rows != 64)
-    return rows == 96 ? launch_sgemm<6, 16>(A, Bt, Cm, M, N, Kd, ldc, stream, tiled)
-                      : launch_sgemm<8, 16>(A, Bt, Cm, M, N, Kd, ldc, stream, tiled);
+    return rows == 96 ? launch_sgemm<6, 16>(A, Bt, Cm, M, N, Kd, ldc, stream, tiled, upper)
+                      : launch_sgemm<8, 16>(A, Bt, Cm, M, N, Kd, ldc, stream, tiled, upper);
   switch (rows) {
-    case 64: return launch_sgemm<4, 8>(A, Bt, Cm, M, N, Kd, ldc, stream, tiled);
-    case 96: return launch_sgemm<6, 8>(A, Bt, Cm, M, N, Kd, ldc, stream, tiled);
-    default: return launch_sgemm<8, 8>(A, Bt, Cm, M, N, Kd, ldc, stream, tiled);
+    case 64: return launch_sgemm<4, 8>(A, Bt, Cm, M, N, Kd, ldc, stream, tiled, upper);
+    case 96: return launch_sgemm<6, 8>(A, Bt, Cm, M, N, Kd, ldc, stream, tiled, upper);
+    default: return launch_sgemm<8, 8>(A, Bt, Cm, M, N, Kd, ldc, stream, tiled, upper);
   }
 }
 

@@ -69,7 +69,7 @@ int launch_project(const float* X, const float* U, const float* W, int64_t C,
                    float* B, int64_t ldb, bool tiled, void* ws, size_t ws_bytes,
                    int* err_out, cudaStream_t stream);
 int sgemm_tn(const float* A, const float* Bt, float* Cm, int64_t M, int64_t N,
-             int64_t Kd, int64_t ldc, cudaStream_t stream, bool tiled);
+             int64_t Kd, int64_t ldc, cudaStream_t stream, bool tiled, bool upper = false);
 // High-pass FIR as a split-BF16 tcgen05 product with the Toeplitz matrix of
 // the taps (fir_tc.cu).  P hi/lo [C][cols] is the batch padded circularly
 // (P[c][j] = x[c][(j - h) mod L]) with cols = fir_tc_cols(rows, ntaps); the
