@@ -340,9 +340,9 @@ def uneven_main(args, dev, rank, world, emit=True):
                                    "channel_samples_per_s": samples * world / (ms_loop * 1e-3)},
         "speedup_batched_vs_per_batch": ms_loop / ms,
         "clocks": sampler.summary(),
-        # per group: energy, {nm, 1/nm}, reorder per recording; temporal per
-        # batch; grouped contraction, peel, residual
-        "gpu_launches": sum(3 * len(mrecs) + len(m.items) + 3 for m in matchers),
+        # per group: set-up, group order, group bounds, reorder per recording;
+        # temporal per batch; grouped contraction and peel
+        "gpu_launches": sum(4 * len(mrecs) + len(m.items) + 2 for m in matchers),
     }
     if rank == 0 and emit:
         print(json.dumps(line), flush=True)
@@ -546,10 +546,10 @@ def stream_main(args, dev, rank, world, emit=True):
         "spikes_per_s": nsp * world / dt,
         # per batch: filter (sums, CAR, high-pass, matrix split, whitening
         # contraction, artifact zeroing), temporal projection; per group:
-        # energy, {nm, 1/nm}, reorder, contraction, peel; per refinement: loss
-        # (5), adjoint (6), ctc (3), transpose (1)
-        "gpu_launches": (7 * sm.n_batches + 5 * -(-sm.n_batches // sm.group)
-                         + 15 * (sm.refinements // (args.steps + max(1, args.warmup)))),
+        # set-up, group order, group bounds, reorder, contraction, peel; per
+        # refinement: loss and adjoint (14), ctc (3), transpose (1)
+        "gpu_launches": (7 * sm.n_batches + 6 * -(-sm.n_batches // sm.group)
+                         + 18 * (sm.refinements // (args.steps + max(1, args.warmup)))),
         "e2e": {"value": value, "unit": "channel-samples/s", "h2d_bytes_per_step": h2d,
                 "d2h_bytes_per_step": nsp * 20},
         "clocks": sampler.summary(),
@@ -1076,8 +1076,8 @@ def main():
             a = agreement(st.cpu().numpy(), st_r, amps.cpu().numpy(), amps_r)
             agr[form] = {k: a[k] for k in ("agreement", "amp_rel_max", "matched", "n_a", "n_r")}
 
-    # energy, reorder, temporal, contraction, {nm, 1/nm}, peel, residual
-    launches_per_batch = 7
+    # reorder, temporal, contraction, set-up, group order, bounds, peel, residual
+    launches_per_batch = 8
     per_step_samples = C * NT_BATCH * nb
     head_ms = results[head]["ms"]
     value = per_step_samples * world / (head_ms * 1e-3)
@@ -1121,9 +1121,9 @@ def main():
         "cpu_baseline": cpu,
         "reference_gpu": ref_gpu,
         "clocks": sampler.summary(),
-        # batched head: energy, {nm, 1/nm}, reorder, a temporal projection per
-        # batch, grouped contraction, peel, residual
-        "gpu_launches": (3 + nb + 3) if head == "bf16x3_batched" else launches_per_batch * nb,
+        # batched head: set-up, group order, bounds, reorder, a temporal projection
+        # per batch, grouped contraction, peel
+        "gpu_launches": (4 + nb + 2) if head == "bf16x3_batched" else launches_per_batch * nb,
     }
     # the other workloads, shortened (every rank takes part): the drop-in
     # extract sharded over the ranks, the uneven multi-recording batches, the

@@ -442,11 +442,12 @@ KS_API int ks_phy_templates(const float* Wall, const float* W, int64_t K, int64_
 /*
  * Stage timing of ks_run_matching, for profiling the public call as it runs
  * (no work is skipped or added).  While enabled on the calling host thread,
- * ks_run_matching records CUDA events at five points on its stream: start,
- * after the template energies, after the projection, after the peel kernel,
+ * ks_run_matching records CUDA events at five points on its stream: start
+ * (twice), after the projection and the template set-up, after the peel kernel,
  * after the residual kernel.  ks_trace_read waits for the last of the first
  * n+1 events of the thread's most recent traced call and writes n <= 4
- * intervals in ms: [energy + copy, projection, peel kernel, residual]
+ * intervals in ms: [empty (an event pair), projection and template set-up
+ * (energies included), peel kernel, residual]
  * (ks_match_batches records the same five points around its stages:
  * [per-recording set-up, projections, peel launch, residual launch]).  The
  * events are the library's, created on the current device by the first

@@ -312,10 +312,8 @@ extern "C" KS_API int ks_match_batches(const ks_rec_desc* recs, int64_t n_recs,
     const ks_rec_desc& d = recs[r];
     const RecPlan& rp = pl.rec[r];
     float* nm = reinterpret_cast<float*>(base + rp.nm);
-    if ((rc = launch_template_energy(d.U, d.K, d.P, d.C, nm, s))) return rc;
-    if ((rc = launch_nm_pairs(nm, d.K, reinterpret_cast<float2*>(base + rp.nmi), s))) return rc;
-    if ((rc = launch_group_setup(d.U, d.ctcT, reinterpret_cast<const float2*>(base + rp.nmi), d.K,
-                                 d.P, d.C, d.nt, base + rp.groups, s)))
+    if ((rc = launch_group_setup(d.U, d.ctcT, nm, true, reinterpret_cast<float2*>(base + rp.nmi),
+                                 d.K, d.P, d.C, d.nt, base + rp.groups, s)))
       return rc;
     if (precision == KS_PROJ_BF16X3)
       rc = launch_reorder_templates(d.U, d.K, d.P, d.C, rp.Kpad, rp.Q, nullptr,

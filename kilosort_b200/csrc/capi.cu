@@ -220,9 +220,10 @@ int ks_peel(float* B, int64_t ldb, int b_layout, float* Xres, const float* U, co
     rc = launch_tile_rows(B, ldb, K, L, Bt, s);
     if (rc) return rc;
   }
-  rc = launch_peel_tiled(Bt, Xres, Xres, U, W, ctcT, nm, C, L, K, P, nt, th2, max_peels, capacity,
-                         st, amps, th_amps, info, base + m.peel_off, m.bytes - m.peel_off, s,
-                         wait_limit_ns(), nullptr, true);
+  rc = launch_peel_tiled(Bt, Xres, Xres, U, W, ctcT, const_cast<float*>(nm), false, C,
+                         L, K, P, nt, th2, max_peels, capacity, st, amps, th_amps, info,
+                         base + m.peel_off, m.bytes - m.peel_off, s, wait_limit_ns(), nullptr,
+                         true);
   if (rc) return rc;
   return b_layout == KS_B_ROWS ? launch_untile_rows(Bt, K, L, B, ldb, s) : KS_OK;
 }
@@ -261,14 +262,12 @@ int ks_run_matching(const float* X, const float* U, const float* W, const float*
     ctcT = t;
   }
   trace_mark(0, s);
-  rc = launch_template_energy(U, K, P, C, nm, s);
-  if (rc) return rc;
   trace_mark(1, s);
   rc = launch_project(X, U, W, C, L, K, P, nt, precision, Bt, 0, true, base + m.proj_off,
                       m.ctc_off - m.proj_off, nullptr, s);
   if (rc) return rc;
   // the projection's error word is the first int of its workspace
-  return launch_peel_tiled(Bt, X, Xres, U, W, ctcT, nm, C, L, K, P, nt, th2, max_peels,
+  return launch_peel_tiled(Bt, X, Xres, U, W, ctcT, nm, true, C, L, K, P, nt, th2, max_peels,
                            capacity, st, amps, th_amps, info, base + m.peel_off,
                            m.bytes - m.peel_off, s, wait_limit_ns(),
                            reinterpret_cast<const int*>(base + m.proj_off), true);

@@ -13,7 +13,7 @@
 // Kernels: ks_detect_scores_tiled_kernel (a block per tile of 32 positions,
 // persistent over 32-sample time tiles: the union of the positions' nearest
 // channels is staged, double-buffered by cp.async, the (s, k) sums of one
-// position over 32 samples per warp in registers; A is never stored;
+// position per half warp, two samples per lane, in registers; A is never stored;
 // ks_detect_scores_kernel is the form for more than 8192 channels),
 // ks_detect_peaks_kernel (a block per (f, 1024-sample tile): only where the
 // score exceeds the threshold and both samples beside it, the maximum over the

@@ -47,24 +47,24 @@ static GroupTables group_tables_at(void* tables, int64_t K) {
   return t;
 }
 
-// Group order, product bounds and permuted {nm, 1/nm} of the grouped update
-// for one template set (ctcT in the transposed layout, nmi from
-// launch_nm_pairs), written into tables (group_tables_bytes(K)).
-int launch_group_setup(const float* U, const float* ctcT, const float2* nmi, int64_t K,
-                       int64_t P, int64_t C, int64_t nt, void* tables, cudaStream_t stream) {
+// Energies, group order, product bounds and permuted {nm, 1/sqrt(nm)} of the
+// grouped update for one template set (ctcT in the transposed layout), written
+// into nmi and tables (group_tables_bytes(K)).  nm is written when `energies`,
+// else read.
+int launch_group_setup(const float* U, const float* ctcT, float* nm, bool energies, float2* nmi,
+                       int64_t K, int64_t P, int64_t C, int64_t nt, void* tables,
+                       cudaStream_t stream) {
   const GroupTables t = group_tables_at(tables, K);
   const int ng = n_groups(K);
-  ks_template_key_kernel<<<(unsigned)((K * 32 + 255) / 256), 256, 0, stream>>>(U, (int)K, (int)P,
-                                                                              (int)C, t.key, t.sup);
+  ks_template_setup_kernel<<<(unsigned)K, 256, 0, stream>>>(
+      U, (int)K, (int)P, (int)C, nm, energies ? nm : nullptr, nmi, t.key, t.sup);
   KS_CUDA(cudaGetLastError());
-  ks_group_order_kernel<<<(unsigned)((K + 255) / 256), 256, 0, stream>>>(t.key, (int)K, t.rperm);
+  ks_group_order_kernel<<<(unsigned)((K + 31) / 32), 256, 0, stream>>>(t.key, (int)K, nmi, t.rperm,
+                                                                      t.nmip);
   KS_CUDA(cudaGetLastError());
   const long long items = K * (long long)ng;
   ks_group_bound_kernel<<<(unsigned)std::min<long long>(items, 1 << 20), 256, 0, stream>>>(
       ctcT, t.rperm, (int)K, (int)(2 * nt + 1), ng, t.mg);
-  KS_CUDA(cudaGetLastError());
-  ks_group_nmi_kernel<<<(unsigned)((K + 31 + 255) / 256), 256, 0, stream>>>(nmi, t.rperm, (int)K,
-                                                                      t.nmip);
   KS_CUDA(cudaGetLastError());
   return KS_OK;
 }
@@ -99,9 +99,9 @@ int launch_ctc_transpose(const float* ctc, int64_t K, int64_t nt, float* ctcT,
                          cudaStream_t stream) {
   if (!ctc || !ctcT || K < 1 || nt < 1) return fail(KS_ERR_ARG, "ks_ctc_transpose: bad args");
   if (ctc == ctcT) return fail(KS_ERR_ARG, "ks_ctc_transpose: in-place transpose is not supported");
-  const long long rows = K * K;
-  const int grid = (int)std::min<long long>(rows, 65535LL * 4);
-  ks_ctc_transpose_kernel<<<grid, 128, 0, stream>>>(ctc, (int)K, (int)(2 * nt + 1), ctcT);
+  const long long tiles = ((K + 7) / 8) * ((K + 3) / 4);
+  const int grid = (int)std::min<long long>(tiles, 65535LL * 4);
+  ks_ctc_transpose_kernel<<<grid, 256, 0, stream>>>(ctc, (int)K, (int)(2 * nt + 1), ctcT);
   KS_CUDA(cudaGetLastError());
   return KS_OK;
 }
@@ -144,7 +144,7 @@ int peel_occupancy(const DeviceInfo& dev, size_t smem, const void* kernel, int* 
 }
 
 int launch_peel_tiled(float* Bt, const float* X, float* Xres, const float* U, const float* W,
-                      const float* ctcT, const float* nm, int64_t C, int64_t L, int64_t K,
+                      const float* ctcT, float* nm, bool energies, int64_t C, int64_t L, int64_t K,
                       int64_t P, int64_t nt, float th2, int64_t max_peels,
                       int64_t capacity, int64_t* st, float* amps, float* th_amps,
                       int64_t* info, void* ws, size_t ws_bytes, cudaStream_t stream,
@@ -193,12 +193,9 @@ int launch_peel_tiled(float* Bt, const float* X, float* Xres, const float* U, co
   if (rc) return rc;
   const int grid = dev.sm_count * occ;
   KS_CUDA(cudaMemsetAsync(base, 0, 256, stream));       // barrier count and error word
-  rc = launch_nm_pairs(nm, K, nmi, stream);
+  rc = grouped ? launch_group_setup(U, ctcT, nm, energies, nmi, K, P, C, nt, tables, stream)
+               : launch_nm_pairs(nm, K, nmi, stream);
   if (rc) return rc;
-  if (grouped) {
-    rc = launch_group_setup(U, ctcT, nmi, K, P, C, nt, tables, stream);
-    if (rc) return rc;
-  }
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;

@@ -1750,15 +1750,34 @@ __global__ void ks_untile_rows_kernel(const float* __restrict__ Bt, int K, int L
   }
 }
 
-__global__ void ks_ctc_transpose_kernel(const float* __restrict__ ctc, int K, int nlag,
-                                        float* __restrict__ ctcT) {
-  // ctcT[k][j][l] = ctc[j][k][l]; one row of nlag contiguous floats per (k, j)
-  const long long rows = (long long)K * K;
-  for (long long r = blockIdx.x; r < rows; r += gridDim.x) {
-    const int k = (int)(r / K), j = (int)(r % K);
-    const float* src = ctc + ((long long)j * K + k) * nlag;
-    float* dst = ctcT + r * nlag;
-    for (int l = threadIdx.x; l < nlag; l += blockDim.x) dst[l] = src[l];
+// ctcT[k][j][l] = ctc[j][k][l]: a block moves the rows of 8 k by 4 j, a warp one
+// k with its 16 loads of 4 rows in flight, so that runs of eight rows are read
+// and of four written.  Bound by the two passes over memory (54 us at K = 600);
+// one row per block took 170 us there, now 66 (5.4 TB/s).
+__global__ void __launch_bounds__(256) ks_ctc_transpose_kernel(const float* __restrict__ ctc, int K,
+                                                               int nlag, float* __restrict__ ctcT) {
+  const int tk = (K + 7) / 8, tj = (K + 3) / 4;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (long long t = blockIdx.x; t < (long long)tk * tj; t += gridDim.x) {
+    const int k = (int)(t / tj) * 8 + warp, j0 = (int)(t % tj) * 4;
+    if (k >= K) continue;
+    for (int l0 = 0; l0 < nlag; l0 += 128) {
+      float v[4][4];
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const int j = j0 + r, l = l0 + 32 * q + lane;
+          v[r][q] = j < K && l < nlag ? ctc[((long long)j * K + k) * nlag + l] : 0.f;
+        }
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const int j = j0 + r, l = l0 + 32 * q + lane;
+          if (j < K && l < nlag) ctcT[((long long)k * K + j) * nlag + l] = v[r][q];
+        }
+    }
   }
 }
 
@@ -1767,43 +1786,84 @@ __global__ void ks_ctc_transpose_kernel(const float* __restrict__ ctc, int K, in
 // group) pairs the no-op test can leave alone; any order gives the same
 // results.
 //
-// Spatial key of each template: the channel centroid sum_c c*e_c / sum_c e_c
-// of its energy e_c = sum_p U[k,p,c]^2 (0 for a template without energy), and
-// its support mask: bit (c/16)/support_width(C) is set where some U[k,p,c] is
-// not zero.  One warp per template, fixed summation order.
-__global__ void ks_template_key_kernel(const float* __restrict__ U, int K, int P, int C,
-                                       float* __restrict__ key,
-                                       unsigned long long* __restrict__ sup) {
-  const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (w >= K) return;
+// Per template: the energy nm = sum_{p,c} U^2 (when nm_out is given; else nm_in
+// holds it), {nm, 1/nm} (NaN when nm is not a positive normal), the spatial key
+// (the channel centroid sum_c c*e_c / sum_c e_c of its energy e_c =
+// sum_p U[k,p,c]^2, 0 for a template without energy) and the support mask: bit
+// (c/16)/support_width(C) is set where some U[k,p,c] is not zero.  One block
+// of 8 warps per template, fixed summation orders: the energy a warp per
+// component, lanes over channels, then the components in turn
+// (ks_template_energy's order).  Latency-bound: 7 us at C=384, K=480, where
+// one warp per template in three kernels took 33 us.
+__global__ void __launch_bounds__(256)
+ks_template_setup_kernel(const float* __restrict__ U, int K, int P, int C,
+                         const float* __restrict__ nm_in, float* __restrict__ nm_out,
+                         float2* __restrict__ nmi, float* __restrict__ key,
+                         unsigned long long* __restrict__ sup) {
+  __shared__ float sp[8];
+  __shared__ double sse[8], ssc[8];
+  __shared__ unsigned smask[2];
+  const int k = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const float* u = U + (size_t)k * P * C;
+  if (threadIdx.x < 2) smask[threadIdx.x] = 0u;
+  if (nm_out && warp < P) {
+    float s = 0.f;
+#pragma unroll 4
+    for (int c = lane; c < C; c += 32) {
+      const float v = u[warp * C + c];
+      s = __fadd_rn(s, __fmul_rn(v, v));
+    }
+    for (int o = 16; o; o >>= 1) s = __fadd_rn(s, __shfl_xor_sync(0xffffffffu, s, o));
+    if (lane == 0) sp[warp] = s;
+  }
   const int width = support_width(C);
   double se = 0.0, sc = 0.0;
-  unsigned long long mask = 0ull;
-  for (int c0 = 0; c0 < C; c0 += 32) {
-    const int c = c0 + lane;
+  unsigned lo = 0u, hi = 0u;
+  for (int c = threadIdx.x; c < C; c += 256) {
     float e = 0.f;
     bool nz = false;
-    if (c < C) {
-      for (int p = 0; p < P; ++p) {
-        const float u = U[((size_t)w * P + p) * C + c];
-        e = fmaf(u, u, e);
-        nz |= u != 0.f;
-      }
-      se += e;
-      sc += (double)c * e;
+    for (int p = 0; p < P; ++p) {
+      const float v = u[p * C + c];
+      e = fmaf(v, v, e);
+      nz |= v != 0.f;
     }
-    const unsigned b = __ballot_sync(0xffffffffu, nz);
-    if (b & 0xffffu) mask |= 1ull << (c0 / kXCh / width);
-    if (b >> 16) mask |= 1ull << ((c0 / kXCh + 1) / width);
+    se += e;
+    sc += (double)c * e;
+    if (nz) {
+      const int bit = c / kXCh / width;
+      if (bit < 32) lo |= 1u << bit;
+      else hi |= 1u << (bit - 32);
+    }
   }
   for (int o = 16; o; o >>= 1) {
     se += __shfl_xor_sync(0xffffffffu, se, o);
     sc += __shfl_xor_sync(0xffffffffu, sc, o);
   }
+  lo = __reduce_or_sync(0xffffffffu, lo);
+  hi = __reduce_or_sync(0xffffffffu, hi);
+  __syncthreads();
   if (lane == 0) {
-    key[w] = se > 0.0 ? (float)(sc / se) : 0.f;
-    sup[w] = mask;
+    sse[warp] = se;
+    ssc[warp] = sc;
+    atomicOr(&smask[0], lo);
+    atomicOr(&smask[1], hi);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double e = 0.0, c = 0.0;
+    for (int w = 0; w < 8; ++w) {
+      e += sse[w];
+      c += ssc[w];
+    }
+    key[k] = e > 0.0 ? (float)(c / e) : 0.f;
+    sup[k] = (unsigned long long)smask[1] << 32 | smask[0];
+    float nm = nm_out ? 0.f : nm_in[k];
+    if (nm_out) {
+      for (int p = 0; p < P; ++p) nm = __fadd_rn(nm, sp[p]);
+      nm_out[k] = nm;
+    }
+    const bool normal = nm >= 1.17549435e-38f && nm <= 3.40282347e38f;
+    nmi[k] = make_float2(nm, normal ? __frcp_rn(nm) : __int_as_float(0x7fc00000));
   }
 }
 
@@ -1813,12 +1873,18 @@ __device__ __forceinline__ unsigned sortable_key(float f) {
 }
 
 // rperm[r] = the template of rank r in ascending key order (the smaller
-// template index first on equal keys): each thread counts the keys below its
-// own, staged through shared memory 1024 at a time.
+// template index first on equal keys), and {nm, 1/sqrt(nm)} of the templates in
+// that order; an nm outside [2^-30, 2^30], where the group fold's comparison of
+// scores by b/sqrt(nm) could leave the normal range, gets a NaN scale.  The
+// last template fills the positions past K up to whole groups.  Eight threads
+// count the keys below each template's, staged through shared memory 1024 at a
+// time.
 __global__ void __launch_bounds__(256) ks_group_order_kernel(const float* __restrict__ key, int K,
-                                                             int* __restrict__ rperm) {
+                                                             const float2* __restrict__ nmi,
+                                                             int* __restrict__ rperm,
+                                                             float2* __restrict__ nmip) {
   __shared__ unsigned sk[1024];
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  const int k = blockIdx.x * 32 + (threadIdx.x >> 3), part = threadIdx.x & 7;
   const unsigned mine = k < K ? sortable_key(key[k]) : 0u;
   int rank = 0;
   for (int j0 = 0; j0 < K; j0 += 1024) {
@@ -1826,22 +1892,32 @@ __global__ void __launch_bounds__(256) ks_group_order_kernel(const float* __rest
     __syncthreads();
     for (int i = threadIdx.x; i < n; i += blockDim.x) sk[i] = sortable_key(key[j0 + i]);
     __syncthreads();
-    if (k < K)
-      for (int i = 0; i < n; ++i) {
-        const unsigned v = sk[i];
-        rank += (v < mine || (v == mine && j0 + i < k)) ? 1 : 0;
-      }
+#pragma unroll 4
+    for (int i = part; i < n; i += 8) {
+      const unsigned v = sk[i];
+      rank += (v < mine || (v == mine && j0 + i < k)) ? 1 : 0;
+    }
   }
-  if (k < K) rperm[rank] = k;
-  // whole groups: the last template fills the positions past K
-  if (k < K && rank == K - 1)
-    for (int r = K; r < n_groups(K) * kGroup; ++r) rperm[r] = k;
+  for (int o = 4; o; o >>= 1) rank += __shfl_xor_sync(0xffffffffu, rank, o);
+  if (k >= K || part) return;
+  const float nm = nmi[k].x;
+  const bool ok = nm >= 9.3132257e-10f && nm <= 1.0737418e9f;
+  const float2 v = make_float2(nm, ok ? __frsqrt_rn(nm) : __int_as_float(0x7fc00000));
+  rperm[rank] = k;
+  nmip[rank] = v;
+  if (rank == K - 1)
+    for (int r = K; r < n_groups(K) * kGroup; ++r) {
+      rperm[r] = k;
+      nmip[r] = v;
+    }
 }
 
 // mg[k][g] = the largest |ctcT[k][j][l]| over the rows j of group g (rows
 // rperm[32g ..]) and all lags l, by the integer maximum of the magnitude bits
 // (so a NaN anywhere gives a NaN bound, which never passes the no-op test).
-// One block of 256 threads per (template, group).
+// One block of 256 threads per (template, group), a warp's 16 loads of its four
+// rows in flight: bound by reading ctcT once (118 MB at K = 480: 29 us; 41 with
+// one row of loads in flight).
 __global__ void __launch_bounds__(256) ks_group_bound_kernel(const float* __restrict__ ctcT,
                                                              const int* __restrict__ rperm, int K,
                                                              int nlag, int ng,
@@ -1852,11 +1928,19 @@ __global__ void __launch_bounds__(256) ks_group_bound_kernel(const float* __rest
   for (long long item = blockIdx.x; item < items; item += gridDim.x) {
     const int k = (int)(item / ng), g = (int)(item % ng);
     unsigned m = 0u;
-    for (int r = warp; r < kGroup; r += 8) {
-      const int rr = g * kGroup + r;
-      if (rr >= K) break;
-      const float* row = ctcT + ((size_t)k * K + rperm[rr]) * nlag;
-      for (int l = lane; l < nlag; l += 32) m = max(m, __float_as_uint(row[l]) & 0x7fffffffu);
+    // the warp's four rows (the positions past K repeat the last template)
+    const float* row[kGroup / 8];
+#pragma unroll
+    for (int r = 0; r < kGroup / 8; ++r)
+      row[r] = ctcT + ((size_t)k * K + rperm[g * kGroup + warp + 8 * r]) * nlag;
+    for (int l0 = 0; l0 < nlag; l0 += 128) {
+#pragma unroll
+      for (int r = 0; r < kGroup / 8; ++r)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const int l = l0 + 32 * q + lane;
+          if (l < nlag) m = max(m, __float_as_uint(row[r][l]) & 0x7fffffffu);
+        }
     }
     for (int o = 16; o; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
     __syncthreads();
@@ -1867,19 +1951,6 @@ __global__ void __launch_bounds__(256) ks_group_bound_kernel(const float* __rest
       for (int w = 0; w < 8; ++w) x = max(x, wm[w]);
       mg[item] = __uint_as_float(x);
     }
-  }
-}
-
-// {nm, 1/sqrt(nm)} of the template rows in group order; an nm outside
-// [2^-30, 2^30], where the group fold's comparison of scores by b/sqrt(nm)
-// could leave the normal range, gets a NaN scale.
-__global__ void ks_group_nmi_kernel(const float2* __restrict__ nmi, const int* __restrict__ rperm,
-                                    int K, float2* __restrict__ nmip) {
-  const int n = n_groups(K) * kGroup;     // whole groups
-  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
-    const float nm = nmi[rperm[r]].x;
-    const bool ok = nm >= 9.3132257e-10f && nm <= 1.0737418e9f;
-    nmip[r] = make_float2(nm, ok ? __frsqrt_rn(nm) : __int_as_float(0x7fc00000));
   }
 }
 

@@ -98,7 +98,8 @@ extern "C" KS_API int ks_peel_static(float* Bt, float* Xres, const float* U, con
   void* ws = nullptr;
   rc = scratch_address(dev.device, static_cast<cudaStream_t>(stream), &ws);
   if (rc) return rc;
-  return launch_peel_tiled(Bt, Xres, Xres, U, W, ctcT, nm, C, L, K, P, nt, th2, max_peels, capacity, st,
-                           amps, th_amps, info, ws, kPeelStaticBytes,
-                           static_cast<cudaStream_t>(stream), wait_limit_ns(), nullptr, false);
+  return launch_peel_tiled(Bt, Xres, Xres, U, W, ctcT, const_cast<float*>(nm), false,
+                           C, L, K, P, nt, th2, max_peels, capacity, st, amps, th_amps, info,
+                           ws, kPeelStaticBytes, static_cast<cudaStream_t>(stream),
+                           wait_limit_ns(), nullptr, false);
 }

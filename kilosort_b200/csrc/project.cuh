@@ -99,8 +99,9 @@ size_t peel_scratch_size(int64_t L, int64_t K, bool grouped);
 // Tables of the grouped update for one template set (group order, bounds,
 // {nm, 1/nm} in group order), built on the stream by launch_group_setup.
 size_t group_tables_bytes(int64_t K);
-int launch_group_setup(const float* U, const float* ctcT, const float2* nmi, int64_t K,
-                       int64_t P, int64_t C, int64_t nt, void* tables, cudaStream_t stream);
+int launch_group_setup(const float* U, const float* ctcT, float* nm, bool energies, float2* nmi,
+                       int64_t K, int64_t P, int64_t C, int64_t nt, void* tables,
+                       cudaStream_t stream);
 void group_tables(void* tables, int64_t K, const int** rperm, const float** mg,
                   const float2** nmip, const unsigned long long** sup);
 int64_t tiled_rows_floats(int64_t L, int64_t K);
@@ -113,9 +114,10 @@ int launch_ctc_transpose(const float* ctc, int64_t K, int64_t nt, float* ctcT,
 int check_peel_shape(int64_t C, int64_t L, int64_t K, int64_t P, int64_t nt, float th2,
                      int64_t max_peels, int64_t capacity);
 int launch_nm_pairs(const float* nm, int64_t K, float2* nmi, cudaStream_t stream);
-// Xres is written from X (they may be the same array).
+// Xres is written from X (they may be the same array).  The template energies nm
+// are computed here when `energies` (grouped only), else read.
 int launch_peel_tiled(float* Bt, const float* X, float* Xres, const float* U, const float* W,
-                      const float* ctcT, const float* nm, int64_t C, int64_t L, int64_t K,
+                      const float* ctcT, float* nm, bool energies, int64_t C, int64_t L, int64_t K,
                       int64_t P, int64_t nt, float th2, int64_t max_peels,
                       int64_t capacity, int64_t* st, float* amps, float* th_amps,
                       int64_t* info, void* ws, size_t ws_bytes, cudaStream_t stream,
