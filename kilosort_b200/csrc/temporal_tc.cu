@@ -39,9 +39,9 @@
 // shared-memory bandwidth (MMA operands, staging, stores): 146 us at C=384,
 // P=6, L=60122 (4.4 TB/s; 97 us at the copy rate); 261 us with tiles of 1024
 // samples of 4 channels, whose 48-byte rows split sectors and whose MMAs were
-//XX
-// own stores, hides the stores' reads (182 -> 153); copying the staged rows out
-// by the warps instead of TMA took 160.
+// issued by a producer thread.  Staging two row sets at a time, each part with
+// stores of its own, hides the reads of the stores (182 -> 153 us); copying the
+// staged rows out by the warps instead of TMA took 160.
 // Tiles of one time range are consecutive (channel groups fastest), so the
 // partial 128-byte lines at channel-group edges meet in L2.  Every mbarrier
 // wait is bounded; a wait that runs out sets the error word and the CTA
