@@ -17,8 +17,8 @@
 //
 // Kernels (C = selected channels, L = batch samples):
 //   ks_pre_sum_kernel   per-channel sums in double (int16 values: exact)
-//   ks_pre_car_kernel   32-sample tiles: centred values into shared memory,
-//                       per-sample lower median by one warp: counts in 256
+//   ks_pre_car_kernel   32-sample tiles: a warp's centred values of one sample in
+//                       registers, their lower median: counts in 256
 //                       buckets over mean -/+ 4 sd, then an exact rank among the
 //                       few values of the median's bucket (a radix select on the
 //                       order-preserving integer keys when that bucket is
@@ -41,6 +41,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cuda_bf16.h>
+#include <type_traits>
 
 namespace {
 
@@ -52,20 +53,45 @@ constexpr int kFirC = 16;             // channels per FIR tile
 constexpr int kFirThreads = 256;      // 8 samples x 1 channel per thread
 constexpr int kMaxTaps = 1023;
 
-__global__ void ks_pre_sum_kernel(const int16_t* __restrict__ raw, int L, long long ldr,
-                                  const long long* __restrict__ map, int C, int chunk,
-                                  double* __restrict__ sums, int* err) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= C) return;
-  const long long m = map ? map[c] : c;
-  if (m < 0 || m >= ldr) {
+constexpr int kSumT = 256;            // samples per block of the sums
+constexpr int kSumC = 64;             // channels per block of the sums
+
+// A thread sums every fourth sample of the block's 256, 32 loads in flight; the
+// four parts meet in shared memory.  Integer sums, so exact in any order.
+// Bound by reading the batch once (7 us at the copy rate): 18 us for 385 x 60122,
+// 47 us with one sample in flight per thread and 512-sample blocks.
+__global__ void __launch_bounds__(4 * kSumC)
+ks_pre_sum_kernel(const int16_t* __restrict__ raw, int L, long long ldr,
+                  const long long* __restrict__ map, int C, double* __restrict__ sums, int* err) {
+  __shared__ int part[4][kSumC];
+  const int lc = threadIdx.x % kSumC, ph = threadIdx.x / kSumC;
+  const int c = blockIdx.x * kSumC + lc;
+  long long m = c < C ? (map ? map[c] : c) : 0;
+  const bool bad = m < 0 || m >= ldr;
+  if (bad) {
     atomicCAS(err, 0, KS_ERR_ARG);
-    return;
+    m = 0;
   }
-  const int t0 = blockIdx.y * chunk, t1 = min(L, t0 + chunk);
-  long long s = 0;                    // |int16| * chunk fits easily
-  for (int t = t0; t < t1; ++t) s += raw[(long long)t * ldr + m];
-  atomicAdd(sums + c, (double)s);
+  const int t0 = blockIdx.y * kSumT + ph;
+  const int16_t* src = raw + (long long)t0 * ldr + m;
+  int s = 0;                          // 64 * |int16| fits easily
+  if ((int)(blockIdx.y + 1) * kSumT <= L) {
+    const long long step = 4 * ldr;
+#pragma unroll 1
+    for (int q = 0; q < kSumT / 4; q += 32, src += 32 * step) {
+      int v[32];
+#pragma unroll
+      for (int i = 0; i < 32; ++i) v[i] = src[i * step];
+#pragma unroll
+      for (int i = 0; i < 32; ++i) s += v[i];
+    }
+  } else {
+    for (int t = t0; t < L; t += 4, src += 4 * ldr) s += *src;
+  }
+  part[ph][lc] = s;
+  __syncthreads();
+  if (ph == 0 && c < C && !bad)
+    atomicAdd(sums + c, (double)(part[0][lc] + part[1][lc] + part[2][lc] + part[3][lc]));
 }
 
 __device__ __forceinline__ uint32_t order_key(float f) {
@@ -76,51 +102,68 @@ __device__ __forceinline__ float key_value(uint32_t k) {
   return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
 }
 
-// Rank-k value (0-based, ascending) of column s of the tile, by one warp:
-// four passes of an 8-bit radix select on the order keys.
-__device__ float warp_select(const float* tile, int pitch, int C, int s, int k, int* hist) {
+// The counts of a warp's histogram: which bucket holds rank k, how many values
+// are below it and how many in it (the same answer in every lane).
+__device__ __forceinline__ void find_bucket(const int* hist, int k, int& sel, int& before,
+                                            int& count) {
+  const int lane = threadIdx.x & 31;
+  const int4 a = reinterpret_cast<const int4*>(hist)[2 * lane];
+  const int4 b = reinterpret_cast<const int4*>(hist)[2 * lane + 1];
+  const int cnt[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+  int local = 0;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) local += cnt[i];
+  int incl = local;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += v;
+  }
+  const int excl = incl - local;
+  const unsigned hit = __ballot_sync(0xffffffffu, excl <= k && k < incl);
+  const int src = __ffs(hit) - 1;
+  sel = before = count = 0;
+  int acc = excl;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    if (acc <= k && k < acc + cnt[i]) {
+      sel = lane * 8 + i;
+      before = acc;
+      count = cnt[i];
+    }
+    acc += cnt[i];
+  }
+  sel = __shfl_sync(0xffffffffu, sel, src);
+  before = __shfl_sync(0xffffffffu, before, src);
+  count = __shfl_sync(0xffffffffu, count, src);
+}
+
+__device__ __forceinline__ void clear_hist(int* hist) {
+  const int lane = threadIdx.x & 31;
+  reinterpret_cast<int4*>(hist)[lane] = make_int4(0, 0, 0, 0);
+  reinterpret_cast<int4*>(hist)[lane + 32] = make_int4(0, 0, 0, 0);
+}
+
+// Rank-k value (0-based, ascending) of the warp's C values (v[j] of lane l is
+// value l + 32j): four passes of an 8-bit radix select on the order keys.
+template <int NJ>
+__device__ __noinline__ float warp_select(const float (&v)[NJ], int C, int k, int* hist) {
   const int lane = threadIdx.x & 31;
   uint32_t prefix = 0, mask = 0;
 #pragma unroll 1
   for (int shift = 24; shift >= 0; shift -= 8) {
-#pragma unroll
-    for (int b = 0; b < 8; ++b) hist[lane * 8 + b] = 0;
     __syncwarp();
-    for (int c = lane; c < C; c += 32) {
-      const uint32_t key = order_key(tile[c * pitch + s]);
-      if ((key & mask) == prefix) atomicAdd(hist + ((key >> shift) & 255u), 1);
+    clear_hist(hist);
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) {
+      const uint32_t key = order_key(v[j]);
+      if (lane + 32 * j < C && (key & mask) == prefix)
+        atomicAdd(hist + ((key >> shift) & 255u), 1);
     }
     __syncwarp();
-    int cnt[8], local = 0;
-#pragma unroll
-    for (int b = 0; b < 8; ++b) {
-      cnt[b] = hist[lane * 8 + b];
-      local += cnt[b];
-    }
-    int incl = local;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int v = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += v;
-    }
-    const int excl = incl - local;
-    const unsigned hit = __ballot_sync(0xffffffffu, excl <= k && k < incl);
-    const int src = __ffs(hit) - 1;
-    int sel = 0, before = 0;
-    if (lane == src) {
-      int acc = excl;
-#pragma unroll
-      for (int b = 0; b < 8; ++b) {
-        if (k < acc + cnt[b]) {
-          sel = lane * 8 + b;
-          before = acc;
-          break;
-        }
-        acc += cnt[b];
-      }
-    }
-    sel = __shfl_sync(0xffffffffu, sel, src);
-    before = __shfl_sync(0xffffffffu, before, src);
+    int sel, before, count;
+    find_bucket(hist, k, sel, before, count);
     k -= before;
     prefix |= (uint32_t)sel << shift;
     mask |= 255u << shift;
@@ -135,85 +178,60 @@ __device__ __forceinline__ float warp_sum(float v) {
   return v;
 }
 
-// Bucket of v among 256 over [lo, lo + 256 / inv): a non-decreasing function of
-// v (a rounded difference, a rounded product by inv > 0, truncation, clamping).
-__device__ __forceinline__ int median_bucket(float v, float lo, float inv) {
-  const float t = __fmul_rn(__fsub_rn(v, lo), inv);
-  return t < 0.f ? 0 : (t >= 255.f ? 255 : (int)t);
+// Bucket of v among 256: a non-decreasing function of v (one rounding of
+// v * inv + shift with inv > 0, truncation, clamping; +infinity is the last).
+__device__ __forceinline__ unsigned median_bucket(float v, float inv, float shift) {
+  return min(__float2uint_rz(fmaf(v, inv, shift)), 255u);
 }
 
-// Rank-k value (0-based, ascending) of column s of the tile, by one warp.
-// The values are counted into 256 buckets over mean -/+ 4 sd of the column
-// (outliers clamp to the end buckets); the bucket that holds rank k is found
-// from the counts, and since the bucket is a non-decreasing function of the
-// value, the rank-k value is the (k - values below the bucket)-th smallest of
-// that bucket's values, ranked exactly by comparisons.  Near the median the
-// buckets hold a few values each, so the shared-memory counts hardly collide.
-// A bucket of more than 32 values, or a zero or non-finite spread, goes to the
-// radix select.
-__device__ float warp_median(const float* tile, int pitch, int C, int s, int k, int* hist,
-                             float* cand, int* ncand) {
+// Rank-k value (0-based, ascending) of the warp's C values, held as above with
+// +infinity past them, 32 (NJ - 4) < C.  The values are counted into 256 buckets
+// over their mean -/+ 4 sd (outliers clamp to the end buckets); the bucket that
+// holds rank k is found from the counts, and since the bucket is a
+// non-decreasing function of the value, the rank-k value is the (k - values
+// below the bucket)-th smallest of that bucket's values, ranked exactly by
+// comparisons.  Near the median the buckets hold a few values each, so the
+// shared-memory counts hardly collide.  A bucket of more than 32 values, or a
+// zero or non-finite spread, goes to the radix select.
+template <int NJ>
+__device__ __forceinline__ float warp_median(const float (&v)[NJ], int C, float rC, int k,
+                                             int* hist, float* cand) {
   const int lane = threadIdx.x & 31;
+  clear_hist(hist);
   float sum = 0.f, sq = 0.f;
-  for (int c = lane; c < C; c += 32) {
-    const float v = tile[c * pitch + s];
-    sum += v;
-    sq = fmaf(v, v, sq);
-  }
+#pragma unroll
+  for (int j = 0; j < NJ; ++j)
+    if (j < NJ - 4 || lane + 32 * j < C) {
+      sum += v[j];
+      sq = fmaf(v[j], v[j], sq);
+    }
   sum = warp_sum(sum);
   sq = warp_sum(sq);
-  const float mean = sum / (float)C;
-  const float sd = sqrtf(fmaxf(sq / (float)C - mean * mean, 0.f));
-  const float lo = mean - 4.f * sd;
-  const float inv = 32.f / sd;                 // 256 buckets over 8 sd
-  if (!(sd > 0.f) || !isfinite(inv) || !isfinite(lo))
-    return warp_select(tile, pitch, C, s, k, hist);
-#pragma unroll
-  for (int b = 0; b < 8; ++b) hist[lane * 8 + b] = 0;
-  if (lane == 0) *ncand = 0;
+  const float mean = sum * rC;
+  const float var = fmaf(sq, rC, -mean * mean);
+  const float inv = 32.f * rsqrtf(var);        // 256 buckets over 8 sd
+  const float shift = fmaf(-mean, inv, 128.f);
+  if (!(var > 0.f) || !isfinite(inv) || !isfinite(shift)) return warp_select(v, C, k, hist);
   __syncwarp();
-  for (int c = lane; c < C; c += 32)
-    atomicAdd(hist + median_bucket(tile[c * pitch + s], lo, inv), 1);
+  unsigned b[NJ];
+#pragma unroll
+  for (int j = 0; j < NJ; ++j) {
+    b[j] = median_bucket(v[j], inv, shift);
+    atomicAdd(hist + b[j], 1);
+  }
   __syncwarp();
-  int cnt[8], local = 0;
+  int sel, before, m;
+  find_bucket(hist, k, sel, before, m);
+  if (m > 32) return warp_select(v, C, k, hist);
+  int at = 0;
 #pragma unroll
-  for (int b = 0; b < 8; ++b) {
-    cnt[b] = hist[lane * 8 + b];
-    local += cnt[b];
-  }
-  int incl = local;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int v = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += v;
-  }
-  const int excl = incl - local;
-  const unsigned hit = __ballot_sync(0xffffffffu, excl <= k && k < incl);
-  const int src = __ffs(hit) - 1;
-  int sel = 0, before = 0, m = 0;
-  if (lane == src) {
-    int acc = excl;
-#pragma unroll
-    for (int b = 0; b < 8; ++b) {
-      if (k < acc + cnt[b]) {
-        sel = lane * 8 + b;
-        before = acc;
-        m = cnt[b];
-        break;
-      }
-      acc += cnt[b];
+  for (int j = 0; j < NJ; ++j) {
+    const bool in = b[j] == (unsigned)sel;
+    const unsigned who = __ballot_sync(0xffffffffu, in);
+    if (who) {
+      if (in) cand[at + __popc(who & ((1u << lane) - 1u))] = v[j];
+      at += __popc(who);
     }
-  }
-  sel = __shfl_sync(0xffffffffu, sel, src);
-  before = __shfl_sync(0xffffffffu, before, src);
-  m = __shfl_sync(0xffffffffu, m, src);
-  if (m > 32) {
-    __syncwarp();
-    return warp_select(tile, pitch, C, s, k, hist);
-  }
-  for (int c = lane; c < C; c += 32) {
-    const float v = tile[c * pitch + s];
-    if (median_bucket(v, lo, inv) == sel) cand[atomicAdd(ncand, 1)] = v;
   }
   __syncwarp();
   const int kk = k - before;
@@ -233,8 +251,16 @@ __device__ float warp_median(const float* tile, int pitch, int C, int s, int k, 
 // Centred (and common-average-referenced) samples: Xc[c][t], t < L; with kPad
 // instead the bf16 hi/lo planes of the circularly padded batch
 // P[c][j] = x[c][(j - h) mod L], j < cols (sample t at every j = t + h mod L).
-template <bool kCar, bool kPad>
-__global__ void __launch_bounds__(kCarThreads)
+//
+// A block takes 32 samples, a warp four of them in turn: lane l holds the
+// channels l + 32j (32 NJ of them at a time; with kCar all), the next sample's
+// loads in flight while this one's median is found in registers; the results
+// meet in shared memory as rows of 32 samples per channel.  Bound by issue slots
+// (about 700 instructions per sample of 384 channels, 300 of them the median's
+// counts and ranks): 75 us at C=384, L=60122, where a median re-reading the tile
+// from shared memory three times took 142.
+template <bool kCar, bool kPad, int NJ>
+__global__ void __launch_bounds__(kCarThreads, NJ <= 12 ? 3 : 1)
 ks_pre_car_kernel(const int16_t* __restrict__ raw, int L, long long ldr,
                   const long long* __restrict__ map, int C, float sign,
                   const double* __restrict__ sums, float* __restrict__ Xc,
@@ -242,56 +268,77 @@ ks_pre_car_kernel(const int16_t* __restrict__ raw, int L, long long ldr,
                   long long cols, int* err) {
   extern __shared__ __align__(16) float sm[];
   constexpr int pitch = kCarTile + 1;
-  float* tile = sm;                                        // [C][pitch]
-  int* hist = reinterpret_cast<int*>(tile + (size_t)C * pitch);   // [8 warps][256]
-  float* med = reinterpret_cast<float*>(hist + 8 * 256);   // [kCarTile]
-  float* cand = med + kCarTile;                            // [8 warps][32]
-  int* ncand = reinterpret_cast<int*>(cand + 8 * 32);      // [8 warps]
+  constexpr int kWarps = kCarThreads / 32, kPer = kCarTile / kWarps;
+  int* hist = reinterpret_cast<int*>(sm);                  // [8 warps][256]
+  float* cand = reinterpret_cast<float*>(hist + kWarps * 256);    // [8 warps][32]
+  // column of each channel, its mean
+  const int Cr = (C + 127) / 128 * 128;                    // = 32 NJ with kCar
+  long long* off = reinterpret_cast<long long*>(cand + kWarps * 32);   // [Cr]
+  float* mean = reinterpret_cast<float*>(off + Cr);        // [Cr]
+  float* tile = mean + Cr;                                 // [C][pitch]
   const int t0 = blockIdx.x * kCarTile;
   const int nt = min(kCarTile, L - t0);
-  for (int c = threadIdx.x; c < C; c += kCarThreads) {
-    const long long m = map ? map[c] : c;
-    if (m < 0 || m >= ldr) {
-      atomicCAS(err, 0, KS_ERR_ARG);
-      for (int s = 0; s < nt; ++s) tile[c * pitch + s] = 0.f;
-      continue;
-    }
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int c = threadIdx.x; c < Cr; c += kCarThreads) {
+    const long long m = c >= C ? 0 : map ? map[c] : c;
+    const bool bad = m < 0 || m >= ldr;
+    if (bad) atomicCAS(err, 0, KS_ERR_ARG);
+    off[c] = bad ? 0 : m;
     // the mean of the (sign-inverted) samples: negation commutes with the
-    // rounded mean and difference, so this is fl(sign * raw - mean(sign * raw))
-    const float mean = sign * (float)(sums[c] / (double)L);
-    const int16_t* src = raw + (long long)t0 * ldr + m;
-    for (int s = 0; s < nt; ++s)
-      tile[c * pitch + s] = __fsub_rn(sign * (float)src[(long long)s * ldr], mean);
+    // rounded mean and difference, so this is fl(sign * raw - mean(sign * raw));
+    // past the last channel every value is +infinity
+    mean[c] = c < C ? sign * (float)(sums[c] / (double)L) : -INFINITY;
   }
   __syncthreads();
-  if (kCar) {
-    const int warp = threadIdx.x >> 5;
-    for (int s = warp; s < nt; s += kCarThreads / 32) {
-      const float m = warp_median(tile, pitch, C, s, (C - 1) / 2, hist + warp * 256,
-                                  cand + warp * 32, ncand + warp);
-      if ((threadIdx.x & 31) == 0) med[s] = m;
-    }
-    __syncthreads();
-  }
-  for (int e = threadIdx.x; e < C * kCarTile; e += kCarThreads) {
-    const int c = e / kCarTile, s = e - c * kCarTile;
-    if (s < nt) {
-      const float v = tile[c * pitch + s];
-      const float y = kCar ? __fsub_rn(v, med[s]) : v;
-      if (kPad) {
-        const __nv_bfloat16 hv = __float2bfloat16_rn(y);
-        const __nv_bfloat16 lv = __float2bfloat16_rn(y - __bfloat162float(hv));
-        // t0 + s < L and h < L: the first position is one subtraction away
-        long long j = t0 + s + h;
-        if (j >= L) j -= L;
-        for (; j < cols; j += L) {
-          Phi[(size_t)c * cols + j] = hv;
-          Plo[(size_t)c * cols + j] = lv;
-        }
-      } else {
-        Xc[(size_t)c * L + t0 + s] = y;
+  const float rC = 1.f / (float)C;
+  for (int c0 = 0; c0 < C; c0 += 32 * NJ) {
+    unsigned x[NJ];
+    auto load = [&](int s) {
+      // past the batch the last sample again, not written
+      const int16_t* row = raw + (long long)(t0 + min(s, nt - 1)) * ldr;
+#pragma unroll
+      for (int j = 0; j < NJ; ++j) x[j] = (unsigned short)row[off[c0 + lane + 32 * j]];
+    };
+    load(warp);
+#pragma unroll 1
+    for (int i = 0; i < kPer; ++i) {
+      const int s = warp + kWarps * i;
+      float v[NJ];
+#pragma unroll
+      for (int j = 0; j < NJ; ++j) {
+        // 2^23 + 2^15 + x exactly, from the bits
+        const float f = __uint_as_float((x[j] ^ 0x8000u) | 0x4b000000u) - 8421376.f;
+        v[j] = fmaf(sign, f, -mean[c0 + lane + 32 * j]);
+      }
+      if (s >= nt) break;
+      if (i + 1 < kPer) load(s + kWarps);
+      float med = 0.f;
+      if (kCar) med = warp_median(v, C, rC, (C - 1) / 2, hist + warp * 256, cand + warp * 32);
+#pragma unroll
+      for (int j = 0; j < NJ; ++j) {
+        const int c = c0 + lane + 32 * j;
+        if ((kCar && j < NJ - 4) || c < C)
+          tile[c * pitch + s] = kCar ? __fsub_rn(v[j], med) : v[j];
       }
     }
+  }
+  __syncthreads();
+  if (lane >= nt) return;
+  if (kPad) {
+    // t0 + s < L and h < L: the first position is one subtraction away
+    long long j0 = t0 + lane + h;
+    if (j0 >= L) j0 -= L;
+    for (long long j = j0; j < cols; j += L) {
+      for (int c = warp; c < C; c += kWarps) {
+        const float y = tile[c * pitch + lane];
+        const __nv_bfloat16 hv = __float2bfloat16_rn(y);
+        Phi[(size_t)c * cols + j] = hv;
+        Plo[(size_t)c * cols + j] = __float2bfloat16_rn(y - __bfloat162float(hv));
+      }
+    }
+  } else {
+    for (int c = warp; c < C; c += kWarps)
+      Xc[(size_t)c * L + t0 + lane] = tile[c * pitch + lane];
   }
 }
 
@@ -481,9 +528,8 @@ extern "C" KS_API int ks_preprocess_int16(const int16_t* raw, int64_t L, int64_t
 
   // 1. per-channel sums
   {
-    const int chunk = 512;
-    const dim3 grid((unsigned)((C + 255) / 256), (unsigned)((L + chunk - 1) / chunk));
-    ks_pre_sum_kernel<<<grid, 256, 0, s>>>(raw, (int)L, ld_raw, map, (int)C, chunk, sums, err);
+    const dim3 grid((unsigned)((C + kSumC - 1) / kSumC), (unsigned)((L + kSumT - 1) / kSumT));
+    ks_pre_sum_kernel<<<grid, 4 * kSumC, 0, s>>>(raw, (int)L, ld_raw, map, (int)C, sums, err);
     KS_CUDA(cudaGetLastError());
   }
   // 2. centring and common average reference (with a high-pass: into the
@@ -494,8 +540,9 @@ extern "C" KS_API int ks_preprocess_int16(const int16_t* raw, int64_t L, int64_t
   __nv_bfloat16* phi = reinterpret_cast<__nv_bfloat16*>(base + p.phi);
   __nv_bfloat16* plo = reinterpret_cast<__nv_bfloat16*>(base + p.plo);
   {
-    const size_t smem = sizeof(float) * (size_t)C * (kCarTile + 1) + sizeof(int) * 8 * 256 +
-                        sizeof(float) * kCarTile + sizeof(float) * 8 * 32 + sizeof(int) * 8;
+    const size_t smem = (sizeof(float) + sizeof(long long)) * (size_t)ks::round_up(C, 128) +
+                        sizeof(float) * (kCarTile + 1) * (size_t)C +
+                        (kCarThreads / 32) * (sizeof(int) * 256 + sizeof(float) * 32);
     const unsigned grid = (unsigned)((L + kCarTile - 1) / kCarTile);
     const float sign = invert_sign ? -1.f : 1.f;
     auto run = [&](auto kernel) -> int {
@@ -505,11 +552,21 @@ extern "C" KS_API int ks_preprocess_int16(const int16_t* raw, int64_t L, int64_t
       KS_CUDA(cudaGetLastError());
       return KS_OK;
     };
-    int rc;
-    if (hp_taps)
-      rc = do_car ? run(ks_pre_car_kernel<true, true>) : run(ks_pre_car_kernel<false, true>);
-    else
-      rc = do_car ? run(ks_pre_car_kernel<true, false>) : run(ks_pre_car_kernel<false, false>);
+    // with the median a warp holds every channel of a sample, 32 a register, and
+    // the last four registers may be partly or wholly empty
+    auto pick = [&](auto pad) -> int {
+      constexpr bool kPad = decltype(pad)::value;
+      if (!do_car) return run(ks_pre_car_kernel<false, kPad, 4>);
+      if (C <= 128) return run(ks_pre_car_kernel<true, kPad, 4>);
+      if (C <= 256) return run(ks_pre_car_kernel<true, kPad, 8>);
+      if (C <= 384) return run(ks_pre_car_kernel<true, kPad, 12>);
+      if (C <= 512) return run(ks_pre_car_kernel<true, kPad, 16>);
+      if (C <= 640) return run(ks_pre_car_kernel<true, kPad, 20>);
+      if (C <= 768) return run(ks_pre_car_kernel<true, kPad, 24>);
+      if (C <= 896) return run(ks_pre_car_kernel<true, kPad, 28>);
+      return run(ks_pre_car_kernel<true, kPad, kMaxC / 32>);
+    };
+    const int rc = hp_taps ? pick(std::true_type{}) : pick(std::false_type{});
     if (rc) return rc;
   }
   // 3. high-pass (the identity when there is no filter), artifact flag
@@ -559,7 +616,8 @@ extern "C" KS_API int ks_preprocess_int16(const int16_t* raw, int64_t L, int64_t
   }
   // 5. artifact: the whole batch becomes zeros
   {
-    const int blocks = (int)std::min<long long>(4096, ((long long)C * L + 255) / 256);
+    // few blocks: without an artifact they only read the flag
+    const int blocks = (int)std::min<long long>(592, ((long long)C * L + 255) / 256);
     ks_pre_zero_kernel<<<blocks, 256, 0, s>>>(X, (int)C, (int)L, ldx, art);
     KS_CUDA(cudaGetLastError());
   }
