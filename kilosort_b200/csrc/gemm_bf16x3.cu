@@ -14,9 +14,12 @@
 //              buffered 128x256 FP32 accumulator and commits stage releases and
 //              accumulator hand-offs to mbarriers
 //   warps 2-5  epilogue: tcgen05.ld 32 columns at a time (one template row per
-//              thread) and store 128-byte rows of the output (row-major B, or
-//              the 32-column tiled layout of the peel, where a warp's 32 rows
-//              are one contiguous 4 KB run)
+//              thread) and store 128-byte rows of the output: the 32-column
+//              tiled layout of the peel, where a warp's 32 rows are one
+//              contiguous 4 KB run, or row-major B by one row per store (a
+//              row's 32 columns from the 32 lanes, turned in shared memory: with a
+//              row per lane, 32 lines a store, the epilogue bound short
+//              contractions; whitening 384 x 384 x 60122 111 us, now 56)
 // Tiles are (128 templates) x (256 samples), template tiles of one sample tile
 // consecutive so concurrent CTAs share the Y tile through L2.  No TMA multicast.
 // One launch can cover many batches of up to kGroupRecs recordings: the tile
@@ -44,6 +47,8 @@ constexpr int kTileA = kBM * kBK * 2;             // 16 KB
 constexpr int kTileB = kBN * kBK * 2;             // 32 KB
 constexpr int kStageBytes = 2 * kTileA + 2 * kTileB;
 constexpr int kThreads = 192;
+constexpr int kBarBytes = 128;        // mbarriers and the TMEM address
+constexpr int kTurn = 32 * 33;        // floats of an epilogue warp's turned block
 constexpr int kTmemCols = 512;
 constexpr unsigned long long kLimitNs = 2000000000ull;
 
@@ -208,6 +213,7 @@ ks_bf16x3_kernel(const __grid_constant__ GemmGroup g) {
   } else {
     // ---------------------------------------------------------- epilogue
     const int q = warp & 3;                  // TMEM lane quadrant of this warp
+    float* turn = reinterpret_cast<float*>(gbase + kStages * kStageBytes + kBarBytes) + q * kTurn;
     int acc = 0;
     uint32_t acc_ph = 0;
     for (int t = blockIdx.x; t < g.n_tiles; t += gridDim.x) {
@@ -225,27 +231,40 @@ ks_bf16x3_kernel(const __grid_constant__ GemmGroup g) {
         uint32_t r[32];
         tmem_ld32(tl + (uint32_t)(c * 32), r);
         const int n = n0 + c * 32;
-        if (row < bt.K && n < bt.L) {
-          float* dst = g.tiled ? bt.B + ((size_t)(n >> 5) * bt.K + row) * 32
-                               : bt.B + (size_t)row * bt.ldb + n;
-          // the tiled layout's last block is written whole (zeros past L)
-          const bool full = (g.tiled || n + 32 <= bt.L) &&
-                            ((reinterpret_cast<uintptr_t>(dst) & 15) == 0);
-          if (full) {
+        if (n >= bt.L) continue;             // the same for the whole warp
+        if (g.tiled) {
+          if (row < bt.K) {
+            // the last block is written whole (zeros past L)
+            float* dst = bt.B + ((size_t)(n >> 5) * bt.K + row) * 32;
             const int nv = bt.L - n;   // valid columns of this block (>= 1)
 #pragma unroll
             for (int e = 0; e < 32; ++e)
               if (e >= nv) r[e] = 0u;
+            if ((reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
 #pragma unroll
-            for (int v = 0; v < 8; ++v)
-              reinterpret_cast<float4*>(dst)[v] =
-                  make_float4(__uint_as_float(r[4 * v]), __uint_as_float(r[4 * v + 1]),
-                              __uint_as_float(r[4 * v + 2]), __uint_as_float(r[4 * v + 3]));
-          } else {
+              for (int v = 0; v < 8; ++v)
+                reinterpret_cast<float4*>(dst)[v] =
+                    make_float4(__uint_as_float(r[4 * v]), __uint_as_float(r[4 * v + 1]),
+                                __uint_as_float(r[4 * v + 2]), __uint_as_float(r[4 * v + 3]));
+            } else {
 #pragma unroll
-            for (int e = 0; e < 32; ++e)
-              if (n + e < bt.L) dst[e] = __uint_as_float(r[e]);
+              for (int e = 0; e < 32; ++e)
+                if (e < nv) dst[e] = __uint_as_float(r[e]);
+            }
           }
+        } else {
+          // rows of any alignment: a lane a column of the warp's 32 x 32 block,
+          // turned in shared memory
+#pragma unroll
+          for (int e = 0; e < 32; ++e) turn[lane * 33 + e] = __uint_as_float(r[e]);
+          __syncwarp();
+          const int rows = min(32, bt.K - m0 - q * 32);
+          float* dst = bt.B + (size_t)(m0 + q * 32) * bt.ldb + n + lane;
+          if (n + lane < bt.L) {
+#pragma unroll 8
+            for (int i = 0; i < rows; ++i) dst[(size_t)i * bt.ldb] = turn[i * 33 + lane];
+          }
+          __syncwarp();
         }
       }
       fence_before();
@@ -336,7 +355,7 @@ int launch_gemm_group(GemmGroup& g, cudaStream_t stream) {
   DeviceInfo dev;
   int rc = device_info(&dev);
   if (rc) return rc;
-  const size_t smem = (size_t)kStages * kStageBytes + 1024 + 256;
+  const size_t smem = (size_t)kStages * kStageBytes + 1024 + kBarBytes + 4 * kTurn * sizeof(float);
   static thread_local int attr_device = -1;
   if (attr_device != dev.device) {
     KS_CUDA(cudaFuncSetAttribute(ks_bf16x3_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
