@@ -22,8 +22,10 @@
 //                      once
 #include "ks_common.cuh"
 #include "project.cuh"
+#include "residual_apply.cuh"
 
 #include <cuda_bf16.h>
+#include <type_traits>
 
 namespace ks {
 
@@ -76,6 +78,10 @@ constexpr int kPMax = 8;
 // every row starts on a 16-byte boundary.
 __host__ __device__ inline int temporal_xw(int nt) { return (kTT + nt + 8 + 3) & ~3; }
 
+// Floats of a warp's turned results: half of the components of 16 channels by 16
+// samples (pitch 20), or half of the samples by 16 channels.
+__host__ __device__ constexpr int temporal_turn(int P) { return kCG * 20 * ((P + 1) / 2); }
+
 // Asynchronous 4-byte global -> shared copy; src_bytes 0 fills zeros.
 __device__ __forceinline__ void cp_async4(float* dst, const float* src, int src_bytes) {
   const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
@@ -94,8 +100,12 @@ __device__ __forceinline__ void cp_async_wait_prev() {
 // register window (every operand index a compile-time constant) and each
 // tap's components come from the transposed basis Wt[t][8] as two broadcast
 // 16-byte loads.  acc[i][p] accumulates taps t = 0 .. nt-1 in increasing
-// order.  Results go straight from registers to Y: the PP values of one
-// (sample, channel) are contiguous there.
+// order, pairs of components packed.  Whole groups of taps run without a branch,
+// so that the next tap's basis is loaded ahead; f32 results are turned in shared
+// memory so that a store writes whole sectors.  Bound by FMA issue (235 us at
+// C=384, P=6, nt=61, L=60122): 434 us there; 526 with a branch per tap, bounds
+// checked per copied sample and 8-byte stores (519 with the stores alone
+// so, 489 with the checks alone so).
 template <int PP>
 __global__ void __launch_bounds__(kTemporalThreads)
 ks_temporal_kernel(const float* __restrict__ X, const float* __restrict__ W,
@@ -108,6 +118,8 @@ ks_temporal_kernel(const float* __restrict__ X, const float* __restrict__ W,
   const int ntr = (nt + 7) & ~7;            // taps rounded to the group of 8
   float* sW = sm;                           // Wt[ntr][8] (zero past nt and PP)
   float* sX[2] = {sW + 8 * ntr, sW + 8 * ntr + kCG * xw};   // [kCG][xw] each
+  float* sT = sX[1] + kCG * xw;             // [8 warps][kTurn]
+  constexpr int kTurn = temporal_turn(PP);
   const int half = nt / 2;
   for (int i = threadIdx.x; i < 8 * ntr; i += kTemporalThreads) {
     const int t = i >> 3, p = i & 7;
@@ -115,13 +127,23 @@ ks_temporal_kernel(const float* __restrict__ X, const float* __restrict__ W,
   }
   auto fetch = [&](int tile, float* dst) {
     const int tau0 = (tile % tiles_t) * kTT, cg0 = (tile / tiles_t) * kCG;
-    for (int cl = 0; cl < kCG; ++cl) {
-      const int c = cg0 + cl;
-      const float* xrow = X + (long long)(c < C ? c : 0) * L;
-      for (int u = threadIdx.x; u < xw; u += kTemporalThreads) {
-        const int t = tau0 - half + u;
-        const bool ok = c < C && t >= 0 && t < L;
-        cp_async4(dst + cl * xw + u, ok ? xrow + t : X, ok ? 4 : 0);
+    // a warp copies two channels, a lane every 32nd sample
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int w = 2 * (threadIdx.x >> 5) + h, c = cg0 + w;
+      const float* src = X + (long long)(c < C ? c : 0) * L + (tau0 - half) + lane;
+      float* d = dst + w * xw + lane;
+      if (c < C && tau0 >= half && tau0 - half + xw <= L) {
+        int u = lane;
+#pragma unroll 4
+        for (; u < xw; u += 32, src += 32, d += 32) cp_async4(d, src, 4);
+      } else {
+        for (int u = lane; u < xw; u += 32, src += 32, d += 32) {
+          const int t = tau0 - half + u;
+          const bool ok = c < C && t >= 0 && t < L;
+          cp_async4(d, ok ? src : X, ok ? 4 : 0);
+        }
       }
     }
     cp_async_commit();
@@ -138,71 +160,129 @@ ks_temporal_kernel(const float* __restrict__ X, const float* __restrict__ W,
     __syncthreads();
     const int tau0 = (tile % tiles_t) * kTT, cg0 = (tile / tiles_t) * kCG;
     const float4* xs4 = reinterpret_cast<const float4*>(sX[buf] + cl * xw + g * kS);
-    float acc[kS][PP];
+    // packed over pairs of components (the basis is zero past PP)
+    constexpr int HP = (PP + 1) / 2;
+    unsigned long long a2[kS][HP];
 #pragma unroll
     for (int i = 0; i < kS; ++i)
 #pragma unroll
-      for (int p = 0; p < PP; ++p) acc[i][p] = 0.f;
-    float win[kS + 8];
+      for (int p = 0; p < HP; ++p) a2[i][p] = 0ull;
+    unsigned long long win[kS + 8];         // every sample twice
 #pragma unroll
     for (int k = 0; k < kS / 4; ++k) {
       const float4 a = xs4[k];
-      win[4 * k] = a.x; win[4 * k + 1] = a.y; win[4 * k + 2] = a.z; win[4 * k + 3] = a.w;
+      win[4 * k] = f2_pack(a.x, a.x);
+      win[4 * k + 1] = f2_pack(a.y, a.y);
+      win[4 * k + 2] = f2_pack(a.z, a.z);
+      win[4 * k + 3] = f2_pack(a.w, a.w);
     }
-    const float4* w4 = reinterpret_cast<const float4*>(sW);
-    for (int t0 = 0; t0 < nt; t0 += 8) {
-      {
-        const float4 a = xs4[(t0 + kS) / 4], b = xs4[(t0 + kS) / 4 + 1];
-        win[kS + 0] = a.x; win[kS + 1] = a.y; win[kS + 2] = a.z; win[kS + 3] = a.w;
-        win[kS + 4] = b.x; win[kS + 5] = b.y; win[kS + 6] = b.z; win[kS + 7] = b.w;
+    // eight taps from t0 (kTail: those below nt, a branch each)
+    auto taps = [&](int t0, auto tail) {
+      constexpr bool kTail = decltype(tail)::value;
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const float4 a = xs4[(t0 + kS) / 4 + k];
+        win[kS + 4 * k] = f2_pack(a.x, a.x);
+        win[kS + 4 * k + 1] = f2_pack(a.y, a.y);
+        win[kS + 4 * k + 2] = f2_pack(a.z, a.z);
+        win[kS + 4 * k + 3] = f2_pack(a.w, a.w);
       }
 #pragma unroll
       for (int tt = 0; tt < 8; ++tt) {
-        if (t0 + tt < nt) {
-          const float4 wa = w4[2 * (t0 + tt)], wb = w4[2 * (t0 + tt) + 1];
-          const float w[8] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
+        if (!kTail || t0 + tt < nt) {
+          const ulonglong2* wt = reinterpret_cast<const ulonglong2*>(sW + 8 * (t0 + tt));
+          const ulonglong2 wa = wt[0], wb = HP > 2 ? wt[1] : wa;
+          const unsigned long long w[4] = {wa.x, wa.y, wb.x, wb.y};
 #pragma unroll
           for (int i = 0; i < kS; ++i)
 #pragma unroll
-            for (int p = 0; p < PP; ++p) acc[i][p] = fmaf(w[p], win[i + tt], acc[i][p]);
+            for (int p = 0; p < HP; ++p) a2[i][p] = f2_fma(w[p], win[i + tt], a2[i][p]);
         }
       }
 #pragma unroll
       for (int i = 0; i < kS; ++i) win[i] = win[i + 8];
-    }
+    };
+    int t0 = 0;
+#pragma unroll 1
+    for (; t0 + 8 <= nt; t0 += 8) taps(t0, std::false_type{});
+    if (t0 < nt) taps(t0, std::true_type{});
+    float acc[kS][2 * HP];
+#pragma unroll
+    for (int i = 0; i < kS; ++i)
+#pragma unroll
+      for (int p = 0; p < HP; ++p) f2_unpack(a2[i][p], acc[i][2 * p], acc[i][2 * p + 1]);
     // the window is no longer read: the next fetch may overwrite this buffer
     __syncthreads();
     const long long q0 = (long long)(cg0 + cl) * PP;
+    // f32 results: a warp holds 16 samples of all 16 channels, whose rows it turns
+    // in shared memory so that a store writes whole sectors
+    float* turn = sT + (threadIdx.x >> 5) * kTurn;
+    const int lane = threadIdx.x & 31, gw = (threadIdx.x >> 5) * 2, gl = lane >> 4;
     if (YT) {
-      // rows (channel, component), samples contiguous: 8 samples per store pair
-      if (cg0 + cl < C) {
+      // rows (channel, component), samples contiguous: 16 samples a row, half of
+      // the components at a time
+      constexpr int H = (PP + 1) / 2;
 #pragma unroll
-        for (int p = 0; p < PP; ++p) {
-          float4* dst = reinterpret_cast<float4*>(YT + (q0 + p) * ldyt + tau0 + g * kS);
-          dst[0] = make_float4(acc[0][p], acc[1][p], acc[2][p], acc[3][p]);
-          dst[1] = make_float4(acc[4][p], acc[5][p], acc[6][p], acc[7][p]);
+      for (int h = 0; h < 2; ++h) {
+        const int np = h ? PP - H : H;
+        __syncwarp();
+#pragma unroll
+        for (int p = 0; p < H; ++p)
+          if (h * H + p < PP) {
+            float4* d = reinterpret_cast<float4*>(turn + (p * kCG + cl) * 20 + gl * kS);
+            const int pp = h * H + p < PP ? h * H + p : 0;
+            d[0] = make_float4(acc[0][pp], acc[1][pp], acc[2][pp], acc[3][pp]);
+            d[1] = make_float4(acc[4][pp], acc[5][pp], acc[6][pp], acc[7][pp]);
+          }
+        __syncwarp();
+        // four lanes a row, eight rows at once
+        for (int r = lane >> 2; r < np * kCG; r += 8) {
+          const int c = cg0 + (r & (kCG - 1)), p = h * H + r / kCG;
+          if (c < C)
+            *reinterpret_cast<float4*>(YT + ((long long)c * PP + p) * ldyt + tau0 + gw * kS +
+                                       4 * (lane & 3)) =
+                *reinterpret_cast<const float4*>(turn + r * 20 + 4 * (lane & 3));
         }
       }
       buf ^= 1;
       continue;
     }
+    if (Yf) {
+      // rows (sample), channels and components contiguous: half of a thread's
+      // samples at a time
+      constexpr int R = kCG * PP;            // floats of a row
 #pragma unroll
-    for (int i = 0; i < kS; ++i) {
-      const long long o = (long long)(tau0 + g * kS + i) * Q + q0;
-      // pairs of components as one 8-byte (f32) or 4-byte (bf16) store: with
-      // PP even, o + p is even for even p
-      if (Yf) {
+      for (int h = 0; h < 2; ++h) {
+        __syncwarp();
 #pragma unroll
-        for (int p = 0; p < PP; p += 2) {
-          if (PP % 2 == 0)
-            *reinterpret_cast<float2*>(Yf + o + p) = make_float2(acc[i][p], acc[i][p + 1]);
-          else {
-            Yf[o + p] = acc[i][p];
-            if (p + 1 < PP) Yf[o + p + 1] = acc[i][p + 1];
+        for (int i = 0; i < kS / 2; ++i)
+#pragma unroll
+          for (int p = 0; p < PP; p += 2) {
+            float* d = turn + (gl * (kS / 2) + i) * R + cl * PP + p;
+            if (PP % 2 == 0)
+              *reinterpret_cast<float2*>(d) =
+                  make_float2(acc[h * kS / 2 + i][p], acc[h * kS / 2 + i][p + 1]);
+            else {
+              d[0] = acc[h * kS / 2 + i][p];
+              if (p + 1 < PP) d[1] = acc[h * kS / 2 + i][p + 1];
+            }
           }
+        __syncwarp();
+#pragma unroll
+        for (int e = lane; e < kS * R / 4; e += 32) {
+          const int r = e / (R / 4), q = e - r * (R / 4);
+          const int tau = tau0 + (gw + r / (kS / 2)) * kS + h * (kS / 2) + r % (kS / 2);
+          *reinterpret_cast<float4*>(Yf + (long long)tau * Q + (long long)cg0 * PP + 4 * q) =
+              *reinterpret_cast<const float4*>(turn + r * R + 4 * q);
         }
       }
-      if (Yhi) {
+    }
+    if (Yhi) {
+#pragma unroll
+      for (int i = 0; i < kS; ++i) {
+        const long long o = (long long)(tau0 + g * kS + i) * Q + q0;
+        // pairs of components as one 4-byte store: with PP even, o + p is even
+        // for even p
 #pragma unroll
         for (int p = 0; p < PP; p += 2) {
           const float v0 = acc[i][p], v1 = p + 1 < PP ? acc[i][p + 1] : 0.f;
@@ -229,9 +309,9 @@ ks_temporal_kernel(const float* __restrict__ X, const float* __restrict__ W,
 }
 
 size_t temporal_smem(int nt, int P) {
-  (void)P;
   const int ntr = (nt + 7) & ~7;
-  return sizeof(float) * (8 * (size_t)ntr + 2 * (size_t)kCG * temporal_xw(nt));
+  return sizeof(float) * (8 * (size_t)ntr + 2 * (size_t)kCG * temporal_xw(nt) +
+                          kTemporalThreads / 32 * (size_t)temporal_turn(P));
 }
 
 // ------------------------------------------------------------------ FP32 GEMM
