@@ -1356,7 +1356,7 @@ __device__ PeelOutcome run_peel(const PeelArgs& a, const Smem& s, int rank, unsi
     for (long long i = t0; i < a.nblk; i += ts) a.xcount[i] = 0;
     if (t0 < 6) a.wctr[t0] = 0u;
   }
-  if (!ks_grid_sync(a.bar, G, epoch, a.err, a.limit_ns)) {
+  if (!ks_grid_sync(a.bar, G, epoch, a.limit_ns)) {
     const int e = ks_ld_volatile(a.err);
     if (rank == 0 && tid == 0) {
       a.info[0] = 0;
@@ -1392,7 +1392,7 @@ __device__ PeelOutcome run_peel(const PeelArgs& a, const Smem& s, int rank, unsi
   int it = 0;
   int status = KS_OK;
   KS_TRACE(199, 0, ks_globaltimer());
-  bool ok = ks_grid_sync(a.bar, G, epoch, a.err, a.limit_ns);
+  bool ok = ks_grid_sync(a.bar, G, epoch, a.limit_ns);
   for (; ok && it < a.max_peels; ++it) {
     const int p = it & 1, q = p ^ 1;
     KS_TRACE(it, 0, ks_globaltimer());
@@ -1403,7 +1403,7 @@ __device__ PeelOutcome run_peel(const PeelArgs& a, const Smem& s, int rank, unsi
       for (int ch = rank; ch < a.nchunks; ch += (int)G) detect_chunk(a, s, ch, it);
     }
     KS_TRACE(it, 1, ks_globaltimer());
-    if (!ks_grid_sync(a.bar, G, epoch, a.err, a.limit_ns)) break;
+    if (!ks_grid_sync(a.bar, G, epoch, a.limit_ns)) break;
     KS_TRACE(it, 2, ks_globaltimer());
 
     const unsigned* bits = a.dbits + (size_t)p * a.nwords;
@@ -1421,7 +1421,7 @@ __device__ PeelOutcome run_peel(const PeelArgs& a, const Smem& s, int rank, unsi
       // phase A: one warp per dirty block, dealt round-robin (metadata only,
       // about the same work per block)
       group_scan(a, s, p, gwarp, nwarps, ndirty, pcur, lane, warp);
-      if (!ks_grid_sync(a.bar, G, epoch, a.err, a.limit_ns)) break;
+      if (!ks_grid_sync(a.bar, G, epoch, a.limit_ns)) break;
       // phase B: the units.  Up to kStaticUnits per warp are dealt round-robin
       // (neighbouring warps run one block's groups at the same time; a counter
       // taken one unit at a time by thousands of warps would be their queue);
@@ -1535,7 +1535,7 @@ __device__ PeelOutcome run_peel(const PeelArgs& a, const Smem& s, int rank, unsi
     KS_TRACE(it, 5, total);
     KS_TRACE(it, 6, ndirty);
     n_out += total;
-    ok = ks_grid_sync(a.bar, G, epoch, a.err, a.limit_ns);
+    ok = ks_grid_sync(a.bar, G, epoch, a.limit_ns);
   }
   // one read of the error word for the whole block
   const int e = __syncthreads_or(tid == 0 && ks_ld_volatile(a.err) != 0) ? ks_ld_volatile(a.err) : 0;
@@ -2025,7 +2025,7 @@ __host__ __device__ inline void bind_scratch(PeelArgs& a, char* team, char* list
   const TeamLayout t = team_layout(a.L, grouped ? a.K : 0);
   const ListLayout l = list_layout(a.L);
   a.bar = reinterpret_cast<unsigned*>(team);
-  a.err = reinterpret_cast<int*>(team + 64);
+  a.err = reinterpret_cast<int*>(team) + 1;     // read with the count by the barrier
   a.cfmax = reinterpret_cast<float*>(team + t.cfmax);
   a.imax = reinterpret_cast<int*>(team + t.imax);
   a.pack = reinterpret_cast<unsigned long long*>(team + t.pack);
