@@ -33,8 +33,10 @@
 //           and clears its pack[p] entries.
 //   UPDATE  every block computes the exclusive prefix of the chunk counts (a
 //           peak's global index in the iteration) and of the dirty bitmap.
-//           Records are written in (iteration, tau) order.  Warps scan the dirty
-//           blocks and work through the units found (grouped update), or take
+//           Records are written in (iteration, tau) order, after the updates.
+//           Warps scan the dirty blocks and, past a barrier, work through the
+//           units found (grouped update; with few dirty blocks a warp updates a
+//           (block, group) pair as it looks at it, without the barrier), or take
 //           work items (dirty block in column order, row range) from a counter
 //           (ungrouped; large teams: round-robin, the last round from the
 //           counter): B[j,c] -= amp*ctc[j,k,c-tau+nt] for the peaks touching column c,
@@ -1110,8 +1112,7 @@ __device__ __forceinline__ unsigned long long unit_fold(const PeelArgs& a, const
 // inputs fetched.
 template <bool kInit>
 __device__ void run_units(const PeelArgs& a, const Smem& s, long long first, long long step,
-                          int nu, unsigned long long* pack_out, int lane, int warp) {
-  uint2 rec = make_uint2(0u, 0u);
+                          int nu, uint2 rec, unsigned long long* pack_out, int lane, int warp) {
   auto record = [&](int i) {
     if (kInit) {
       const unsigned w = (unsigned)first + (unsigned)i * (unsigned)step, ng = (unsigned)a.ng;
@@ -1122,7 +1123,6 @@ __device__ void run_units(const PeelArgs& a, const Smem& s, long long first, lon
     return make_uint2(__shfl_sync(0xffffffffu, rec.x, i), __shfl_sync(0xffffffffu, rec.y, i));
   };
   if (nu <= 0) return;
-  if (!kInit && lane < nu) rec = a.units[first + lane * step];
   uint2 u = record(0);
   float* Cs = unit_tile(s, warp);
   __syncwarp();                       // the tile's and the slots' earlier readers are done
@@ -1316,6 +1316,62 @@ __device__ void group_scan(const PeelArgs& a, const Smem& s, int p, long long w,
   flush();
 }
 
+// (dirty block, group) pairs per warp up to which pairs are updated as they are
+// looked at: peel at C=96, K=80, L=60122 173 us with the list alone, 164 with one
+// pair per warp, 154 with two or four (more pairs are better dealt as the units
+// that the list leaves of them).
+constexpr long long kFusedItems = 2;
+
+// The records of nu units from `first` in steps of `step`: one per lane.
+__device__ __forceinline__ uint2 unit_records(const PeelArgs& a, long long first, long long step,
+                                              int nu, int lane) {
+  return lane < nu ? a.units[first + lane * step] : make_uint2(0u, 0u);
+}
+
+// One (dirty block, group) pair w: what group_scan does for one group (the warp
+// of group 0 also folds the untouched columns), then the unit if there is one.
+__device__ __forceinline__ void scan_and_update(const PeelArgs& a, const Smem& s, int p, int w,
+                                                unsigned long long* pack_out, int lane, int warp) {
+  const int nt = a.nt, ng = a.ng;
+  const int blk = dirty_block(s, a.nwords, w / ng), g = w % ng;
+  const int c = blk * kCol + lane;
+  const bool colok = c < a.L;
+  const size_t at = ((size_t)blk * ng + g) * 32 + lane;
+  const unsigned long long best = a.gbest[at];
+  const int expo = a.gexp[at];
+  const TouchList tl = order_touch_warp(s, touch_word(a, p, blk, lane), lane, warp);
+  // exponent field of the lane's peak's product bound plus 26
+  int x = 255;
+  if (lane < tl.n)
+    x = min(255, 26 + bound_expo(__fmul_rn(fabsf(tl.amp[lane]),
+                                           __ldg(a.mg + (size_t)tl.k[lane] * ng + g))));
+  bool touched = false, need = false;
+  for (int e = 0; e < tl.n; ++e) {
+    const int d = c - tl.tau[e];
+    const int xe = __shfl_sync(0xffffffffu, x, e);
+    if (colok && d >= -nt && d <= nt) {
+      touched = true;
+      need |= xe > expo;
+    }
+  }
+  if (touched) {
+    if (!need && best) atomicMax(&pack_out[c], best);
+  } else if (colok && g == 0) {
+    atomicMax(&pack_out[c], pack_score(a.cfmax[c], a.imax[c]));
+  }
+  const unsigned cols = __ballot_sync(0xffffffffu, need);
+  if (!cols) return;
+  int* bl = a.blist + (size_t)blk * 32;
+  if (lane == 0) bl[0] = tl.n;
+  if (lane < tl.n) {
+    bl[1 + lane] = tl.tau[lane];
+    bl[1 + kTouch + lane] = tl.k[lane];
+    bl[1 + 2 * kTouch + lane] = __float_as_int(tl.amp[lane]);
+  }
+  run_units<false>(a, s, 0, 1, 1, make_uint2(((unsigned)blk << 11) | (unsigned)g, cols), pack_out,
+                   lane, warp);
+}
+
 // Outcome of one batch's peel, the same in every block of the team.
 struct PeelOutcome {
   long long n_out;
@@ -1374,8 +1430,8 @@ __device__ PeelOutcome run_peel(const PeelArgs& a, const Smem& s, int rank, unsi
       // every (block, group) tile: the group metadata of every column too
       const long long n_items = (long long)a.nblk * a.ng;
       if (gwarp < n_items)
-        run_units<true>(a, s, gwarp, nwarps, (int)((n_items - gwarp + nwarps - 1) / nwarps), pinit,
-                        lane, warp);
+        run_units<true>(a, s, gwarp, nwarps, (int)((n_items - gwarp + nwarps - 1) / nwarps),
+                        make_uint2(0u, 0u), pinit, lane, warp);
     } else {
       const int rg = (a.K + kItemRows - 1) / kItemRows;
       const TouchList none{0, nullptr, nullptr, nullptr};
@@ -1418,33 +1474,45 @@ __device__ PeelOutcome run_peel(const PeelArgs& a, const Smem& s, int rank, unsi
     unsigned long long* pcur = a.pack + (size_t)p * a.L;
     KS_TRACE(it, 3, ks_globaltimer());
     if (kGrouped) {
-      // phase A: one warp per dirty block, dealt round-robin (metadata only,
-      // about the same work per block)
-      group_scan(a, s, p, gwarp, nwarps, ndirty, pcur, lane, warp);
-      if (!ks_grid_sync(a.bar, G, epoch, a.limit_ns)) break;
-      // phase B: the units.  Up to kStaticUnits per warp are dealt round-robin
-      // (neighbouring warps run one block's groups at the same time; a counter
-      // taken one unit at a time by thousands of warps would be their queue);
-      // more are taken from a counter in claims of about a quarter of a warp's
-      // share (at most 32).  A warp reads its records at once and fetches each
-      // unit's inputs while it runs the one before.
-      KS_TRACE(it, 7, ks_globaltimer());
-      const unsigned n_units = ks_ld_acquire(a.wctr + 2 + p);
-      const bool dealt = (long long)n_units <= kStaticUnits * nwarps;
-      const unsigned claim =
-          (unsigned)min(32LL, max(1LL, (long long)n_units / (nwarps * 4)));
-      if (dealt) {
-        if (gwarp < n_units)
-          run_units<false>(a, s, gwarp, nwarps, (int)((n_units - gwarp + nwarps - 1) / nwarps), pcur,
-                           lane, warp);
+      if ((long long)ndirty * a.ng <= kFusedItems * nwarps) {
+        // few (dirty block, group) pairs (a small batch, or the last iterations
+        // of a larger one): each pair is looked at and updated by one warp, without
+        // a list and its barrier (109 -> 91 us of peel at C=32, K=24, L=4122; 1423
+        // -> 1385 at C=384, K=480, L=60122)
+        for (long long w = gwarp; w < (long long)ndirty * a.ng; w += nwarps)
+          scan_and_update(a, s, p, (int)w, pcur, lane, warp);
       } else {
-        while (true) {
-          unsigned first = 0;
-          if (lane == 0) first = atomicAdd(&a.wctr[4 + p], claim);
-          first = __shfl_sync(0xffffffffu, first, 0);
-          if (first >= n_units) break;
-          run_units<false>(a, s, first, 1, (int)(min(n_units, first + claim) - first), pcur, lane,
-                           warp);
+        // phase A: one warp per dirty block, dealt round-robin (metadata only,
+        // about the same work per block)
+        group_scan(a, s, p, gwarp, nwarps, ndirty, pcur, lane, warp);
+        if (!ks_grid_sync(a.bar, G, epoch, a.limit_ns)) break;
+        // phase B: the units.  Up to kStaticUnits per warp are dealt round-robin
+        // (neighbouring warps run one block's groups at the same time; a counter
+        // taken one unit at a time by thousands of warps would be their queue);
+        // more are taken from a counter in claims of about a quarter of a warp's
+        // share (at most 32).  A warp reads its records at once and fetches each
+        // unit's inputs while it runs the one before.
+        KS_TRACE(it, 7, ks_globaltimer());
+        const unsigned n_units = ks_ld_acquire(a.wctr + 2 + p);
+        const bool dealt = (long long)n_units <= kStaticUnits * nwarps;
+        const unsigned claim =
+            (unsigned)min(32LL, max(1LL, (long long)n_units / (nwarps * 4)));
+        if (dealt) {
+          if (gwarp < n_units) {
+            const int nu = (int)((n_units - gwarp + nwarps - 1) / nwarps);
+            run_units<false>(a, s, gwarp, nwarps, nu, unit_records(a, gwarp, nwarps, nu, lane), pcur,
+                             lane, warp);
+          }
+        } else {
+          while (true) {
+            unsigned first = 0;
+            if (lane == 0) first = atomicAdd(&a.wctr[4 + p], claim);
+            first = __shfl_sync(0xffffffffu, first, 0);
+            if (first >= n_units) break;
+            const int nu = (int)(min(n_units, first + claim) - first);
+            run_units<false>(a, s, first, 1, nu, unit_records(a, first, 1, nu, lane), pcur, lane,
+                             warp);
+          }
         }
       }
     } else {
