@@ -404,9 +404,9 @@ def adjoint_main(args, dev, rank, world):
         "spikes_per_s": N * world / (ms * 1e-3),
         "window_gbs": win_bytes / (ms * 1e-3) / 1e9,
         "clocks": sampler.summary(),
-        # forward: count, scan, fill, reconstruct, sum; backward: count, scan,
-        # group, adjoint, dW, damps
-        "gpu_launches": 11,
+        # forward: count, scan, fill, order, support, reconstruct, sum; backward:
+        # count, scan, group, adjoint, dW (parts, sum), damps
+        "gpu_launches": 14,
     }
     if rank == 0:
         print(json.dumps(line), flush=True)
@@ -760,9 +760,10 @@ def extract_main(args, dev, rank, world):
         "spikes_per_step": len(st),
         "stages_ms": {"batch_source_alone": t_src * 1e3, "matching_alone": t_match * 1e3},
         "fp32_projection": {"value": C * nb * NT_BATCH * world / dt32, "ms_per_step": dt32 * 1e3},
-        # per batch: filter 6, matching 7, features 1; per call: template
+        # per batch: filter 7, temporal 1, features 1; per group (1, 2, then 4
+        # batches): set-up 3, reorder, contraction, peel; per call: template
         # channels, ctc (2), transpose
-        "gpu_launches": 14 * nb + 4,
+        "gpu_launches": 9 * nb + 6 * (min(nb, 2) + max(0, -(-(nb - 3) // 4))) + 4,
         "e2e": {"value": value, "unit": "channel-samples/s",
                 "h2d_bytes_per_step": nb * L * n_bin * 2,
                 "d2h_bytes_per_step": int(st.nbytes + tF.numel() * 4)},

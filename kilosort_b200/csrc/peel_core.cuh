@@ -1478,7 +1478,7 @@ __device__ PeelOutcome run_peel(const PeelArgs& a, const Smem& s, int rank, unsi
         // few (dirty block, group) pairs (a small batch, or the last iterations
         // of a larger one): each pair is looked at and updated by one warp, without
         // a list and its barrier (109 -> 91 us of peel at C=32, K=24, L=4122; 1423
-        // -> 1385 at C=384, K=480, L=60122)
+        // -> 1385 at C=384, K=600, L=60122)
         for (long long w = gwarp; w < (long long)ndirty * a.ng; w += nwarps)
           scan_and_update(a, s, p, (int)w, pcur, lane, warp);
       } else {
@@ -1567,7 +1567,7 @@ __device__ PeelOutcome run_peel(const PeelArgs& a, const Smem& s, int rank, unsi
     // the warps that were dealt the fewest: one warp per chunk (the chunks' peak
     // counts are independent loads).  Ahead of the scan they held up every
     // iteration by a chain of three loads and an atomic: 1566 -> 1519 us of peel at
-    // C=384, K=480, L=60122, 125 -> 118 us at C=32, K=24, L=4122.
+    // C=384, K=600, L=60122, 125 -> 118 us at C=32, K=24, L=4122.
     for (long long ch = nwarps - 1 - gwarp; ch < a.nchunks; ch += nwarps) {
       const int c_n = a.chunk_cnt[ch];
       for (int i = lane; i < c_n; i += 32) {
@@ -1866,7 +1866,7 @@ __global__ void __launch_bounds__(256) ks_ctc_transpose_kernel(const float* __re
 // (c/16)/support_width(C) is set where some U[k,p,c] is not zero.  One block
 // of 8 warps per template, fixed summation orders: the energy a warp per
 // component, lanes over channels, then the components in turn
-// (ks_template_energy's order).  Latency-bound: 7 us at C=384, K=480, where
+// (ks_template_energy's order).  Latency-bound: 7 us at C=371, K=533, where
 // one warp per template in three kernels took 33 us.
 __global__ void __launch_bounds__(256)
 ks_template_setup_kernel(const float* __restrict__ U, int K, int P, int C,
@@ -1989,7 +1989,7 @@ __global__ void __launch_bounds__(256) ks_group_order_kernel(const float* __rest
 // rperm[32g ..]) and all lags l, by the integer maximum of the magnitude bits
 // (so a NaN anywhere gives a NaN bound, which never passes the no-op test).
 // One block of 256 threads per (template, group), a warp's 16 loads of its four
-// rows in flight: bound by reading ctcT once (118 MB at K = 480: 29 us; 41 with
+// rows in flight: bound by reading ctcT once (140 MB at K = 533: 29 us; 41 with
 // one row of loads in flight).
 __global__ void __launch_bounds__(256) ks_group_bound_kernel(const float* __restrict__ ctcT,
                                                              const int* __restrict__ rperm, int K,
