@@ -88,7 +88,7 @@ __device__ __forceinline__ int ks_ld_volatile(const int* p) {
 // barriers.  A wait is round trips to L2, whatever the number of blocks (20 to
 // 296 the same): one release and one 8-byte acquire that reads the count and the
 // error together, so that no fence and no second load follow the last arrival: a
-// peel of 45 iterations at C=384, K=600, L=60122 1519 -> 1423 us against fences on
+// peel of 46 iterations at C=384, K=600, L=60122 1519 -> 1423 us against fences on
 // both sides, a sleep before every poll and the error read at the end.
 __device__ __forceinline__ bool ks_grid_sync(unsigned* ctl, unsigned nblocks, unsigned& epoch,
                                              unsigned long long limit_ns) {
