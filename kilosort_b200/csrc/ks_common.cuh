@@ -75,40 +75,64 @@ __device__ __forceinline__ int ks_ld_volatile(const int* p) {
   return *reinterpret_cast<const volatile int*>(p);
 }
 
-// Device-wide barrier for a cooperative (co-resident) grid.  ctl[0] (8-byte
-// aligned) is the arrival count, ctl[1] the error word.  The count starts at zero
-// and only grows: barrier number `epoch` (1, 2, ...) completes when it reaches
-// epoch * nblocks, so arriving is a single atomic and there is no reset to order.
-// Every block passes the same sequence of barriers and keeps its own epoch.  A
-// wait that exceeds limit_ns records KS_ERR_TIMEOUT in the error word and
-// returns; every caller then sees the error and leaves its loop, so no block
+// Control word of a team of co-resident blocks: arrivals at its barriers in the
+// low 56 bits, the first error's code above them.  Every access while the team
+// runs is 64 bits wide (memory-model ordering holds between accesses of one width
+// to one word, not between a word and its halves).
+constexpr int kCtlErrShift = 56;
+
+__device__ __forceinline__ unsigned long long ks_ctl_load(const unsigned long long* ctl) {
+  unsigned long long v;
+  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(ctl) : "memory");
+  return v;
+}
+__device__ __forceinline__ int ks_ctl_error(const unsigned long long* ctl) {
+  return (int)(ks_ctl_load(ctl) >> kCtlErrShift);
+}
+// Record an error; the first one stays.  A lost exchange means that another
+// block arrived or failed in between, so the loop ends after as many rounds as
+// there are blocks.
+__device__ __forceinline__ void ks_ctl_fail(unsigned long long* ctl, int code) {
+  unsigned long long v = ks_ctl_load(ctl);
+  while (!(v >> kCtlErrShift)) {
+    const unsigned long long seen = atomicCAS(ctl, v, v | (unsigned long long)code << kCtlErrShift);
+    if (seen == v) break;
+    v = seen;
+  }
+}
+
+// Device-wide barrier for a cooperative (co-resident) grid over a control word
+// that starts at zero.  The count only grows: barrier number `epoch` (1, 2, ...)
+// completes when it reaches epoch * nblocks, so arriving is a single atomic and
+// there is no reset to order.  Every block passes the same sequence of barriers
+// and keeps its own epoch.  A wait that exceeds limit_ns records KS_ERR_TIMEOUT
+// and returns; every caller then sees the error and leaves its loop, so no block
 // waits without bound.  Returns true when no error is recorded; the answer is the
-// same for every thread of the block (thread 0 reads the flag and the closing
+// same for every thread of the block (thread 0 reads the word and the closing
 // barrier broadcasts it), so callers may branch on it around further block
 // barriers.  A wait is round trips to L2, whatever the number of blocks (20 to
-// 296 the same): one release and one 8-byte acquire that reads the count and the
-// error together, so that no fence and no second load follow the last arrival: a
-// peel of 46 iterations at C=384, K=600, L=60122 1519 -> 1423 us against fences on
+// 296 the same): one release and one acquire that reads the count and the error
+// together, so that no fence and no second load follow the last arrival: a peel
+// of 46 iterations at C=384, K=600, L=60122 1519 -> 1423 us against fences on
 // both sides, a sleep before every poll and the error read at the end.
-__device__ __forceinline__ bool ks_grid_sync(unsigned* ctl, unsigned nblocks, unsigned& epoch,
-                                             unsigned long long limit_ns) {
+__device__ __forceinline__ bool ks_grid_sync(unsigned long long* ctl, unsigned nblocks,
+                                             unsigned& epoch, unsigned long long limit_ns) {
   __syncthreads();
   ++epoch;
   int bad = 0;
   if (threadIdx.x == 0) {
-    const unsigned target = epoch * nblocks;
-    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(ctl) : "memory");
+    const unsigned long long target = (unsigned long long)epoch * nblocks;
+    asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(ctl), "l"(1ull) : "memory");
     unsigned long long t0 = 0;
     for (unsigned spin = 0;; ++spin) {
-      unsigned long long v;
-      asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(ctl) : "memory");
-      bad = (int)(v >> 32) != 0;
-      if ((unsigned)v >= target) break;
+      const unsigned long long v = ks_ctl_load(ctl);
+      bad = (v >> kCtlErrShift) != 0;
+      if ((v & ((1ull << kCtlErrShift) - 1)) >= target) break;
       if (spin >= 16) {
         __nanosleep(20);
         if (t0 == 0) t0 = ks_globaltimer();
         if (ks_globaltimer() - t0 > limit_ns) {
-          atomicCAS(reinterpret_cast<int*>(ctl) + 1, 0, KS_ERR_TIMEOUT);
+          ks_ctl_fail(ctl, KS_ERR_TIMEOUT);
           bad = 1;
           break;
         }

@@ -192,7 +192,7 @@ int launch_peel_tiled(float* Bt, const float* X, float* Xres, const float* U, co
   rc = peel_occupancy(dev, smem, (const void*)kernel, &occ);
   if (rc) return rc;
   const int grid = dev.sm_count * occ;
-  KS_CUDA(cudaMemsetAsync(base, 0, 256, stream));       // barrier count and error word
+  KS_CUDA(cudaMemsetAsync(base, 0, 256, stream));       // control word
   rc = grouped ? launch_group_setup(U, ctcT, nm, energies, nmi, K, P, C, nt, tables, stream)
                : launch_nm_pairs(nm, K, nmi, stream);
   if (rc) return rc;

@@ -157,8 +157,7 @@ struct PeelArgs {
   int* itoff;                 // [kMaxIters] first record of each iteration
   int* xcount;                // [nblk] spikes whose residual window meets the block
   int* xlist;                 // [nblk * kXCap] their record indices (unordered)
-  unsigned* bar;              // barrier arrival count (monotonic)
-  int* err;
+  unsigned long long* ctl;    // the team's control word (barrier count, error)
   const int* upstream_err;    // error word of the producer of Bt (may be null)
   // grouped update (null rperm: every row of a touched column is rewritten)
   const int* rperm;           // [K] template rows in group order (group g: rows
@@ -396,7 +395,7 @@ __device__ void detect_chunk(const PeelArgs& a, const Smem& s, int ch, int it) {
           for (int c = b * kCol; c < c_hi; ++c) pcur[c] = 0ull;
         }
         if (pos[i] < kTouch) tch[(size_t)b * kTouch + pos[i]] = Touch{tau, k, amp, slot};
-        else atomicCAS(a.err, 0, KS_ERR_DEGENERATE);
+        else ks_ctl_fail(a.ctl, KS_ERR_DEGENERATE);
       }
     }
   }
@@ -526,7 +525,7 @@ __device__ void detect_chunk_warp(const PeelArgs& a, float* tile, int ch, int it
         if (pos[i] == 0) atomicOr(&bits[b >> 5], 1u << (b & 31));
         if (pos[i] >= 0) {
           if (pos[i] < kTouch) tch[(size_t)b * kTouch + pos[i]] = Touch{tau, k, amp, slot};
-          else atomicCAS(a.err, 0, KS_ERR_DEGENERATE);
+          else ks_ctl_fail(a.ctl, KS_ERR_DEGENERATE);
         }
         // a block's first registration clears its rescoring slots
         for (unsigned f = __ballot_sync(0xffffffffu, pos[i] == 0); f; f &= f - 1u) {
@@ -1399,7 +1398,7 @@ __device__ PeelOutcome run_peel(const PeelArgs& a, const Smem& s, int rank, unsi
   // a failed producer of the score matrix fails the peel
   if (rank == 0 && tid == 0 && a.upstream_err) {
     const int ue = ks_ld_volatile(a.upstream_err);
-    if (ue) atomicCAS(a.err, 0, ue);
+    if (ue) ks_ctl_fail(a.ctl, ue);
   }
   // per-batch state starts empty: registration counts, dirty bitmaps, both
   // rescoring buffers (pack[1] receives the initial scores), work counters and
@@ -1412,8 +1411,8 @@ __device__ PeelOutcome run_peel(const PeelArgs& a, const Smem& s, int rank, unsi
     for (long long i = t0; i < a.nblk; i += ts) a.xcount[i] = 0;
     if (t0 < 6) a.wctr[t0] = 0u;
   }
-  if (!ks_grid_sync(a.bar, G, epoch, a.limit_ns)) {
-    const int e = ks_ld_volatile(a.err);
+  if (!ks_grid_sync(a.ctl, G, epoch, a.limit_ns)) {
+    const int e = ks_ctl_error(a.ctl);
     if (rank == 0 && tid == 0) {
       a.info[0] = 0;
       a.info[1] = e;
@@ -1448,7 +1447,7 @@ __device__ PeelOutcome run_peel(const PeelArgs& a, const Smem& s, int rank, unsi
   int it = 0;
   int status = KS_OK;
   KS_TRACE(199, 0, ks_globaltimer());
-  bool ok = ks_grid_sync(a.bar, G, epoch, a.limit_ns);
+  bool ok = ks_grid_sync(a.ctl, G, epoch, a.limit_ns);
   for (; ok && it < a.max_peels; ++it) {
     const int p = it & 1, q = p ^ 1;
     KS_TRACE(it, 0, ks_globaltimer());
@@ -1459,7 +1458,7 @@ __device__ PeelOutcome run_peel(const PeelArgs& a, const Smem& s, int rank, unsi
       for (int ch = rank; ch < a.nchunks; ch += (int)G) detect_chunk(a, s, ch, it);
     }
     KS_TRACE(it, 1, ks_globaltimer());
-    if (!ks_grid_sync(a.bar, G, epoch, a.limit_ns)) break;
+    if (!ks_grid_sync(a.ctl, G, epoch, a.limit_ns)) break;
     KS_TRACE(it, 2, ks_globaltimer());
 
     const unsigned* bits = a.dbits + (size_t)p * a.nwords;
@@ -1485,7 +1484,7 @@ __device__ PeelOutcome run_peel(const PeelArgs& a, const Smem& s, int rank, unsi
         // phase A: one warp per dirty block, dealt round-robin (metadata only,
         // about the same work per block)
         group_scan(a, s, p, gwarp, nwarps, ndirty, pcur, lane, warp);
-        if (!ks_grid_sync(a.bar, G, epoch, a.limit_ns)) break;
+        if (!ks_grid_sync(a.ctl, G, epoch, a.limit_ns)) break;
         // phase B: the units.  Up to kStaticUnits per warp are dealt round-robin
         // (neighbouring warps run one block's groups at the same time; a counter
         // taken one unit at a time by thousands of warps would be their queue);
@@ -1603,10 +1602,10 @@ __device__ PeelOutcome run_peel(const PeelArgs& a, const Smem& s, int rank, unsi
     KS_TRACE(it, 5, total);
     KS_TRACE(it, 6, ndirty);
     n_out += total;
-    ok = ks_grid_sync(a.bar, G, epoch, a.limit_ns);
+    ok = ks_grid_sync(a.ctl, G, epoch, a.limit_ns);
   }
-  // one read of the error word for the whole block
-  const int e = __syncthreads_or(tid == 0 && ks_ld_volatile(a.err) != 0) ? ks_ld_volatile(a.err) : 0;
+  // one decision on the error for the whole block
+  const int e = __syncthreads_or(tid == 0 && ks_ctl_error(a.ctl) != 0) ? ks_ctl_error(a.ctl) : 0;
   if (rank == 0 && tid == 0) {
     a.info[0] = n_out;
     a.info[1] = e ? e : status;
@@ -2028,12 +2027,11 @@ __global__ void __launch_bounds__(256) ks_group_bound_kernel(const float* __rest
 }
 
 // Scratch of one team (reused for every batch it processes), for batches of
-// up to L padded samples and K templates: [ctl 256 B: barrier count, error
-// word] [cfmax L] [imax L] [pack 2L] [chunk counts] [chunk buffers 4 x
+// up to L padded samples and K templates: [ctl 256 B: control word] [cfmax L] [imax L] [pack 2L] [chunk counts] [chunk buffers 4 x
 // nchunks*kChunk] [tcount 2 nblk] [touch 2 nblk*kTouch] [dbits 2 nwords]
 // [work counters 6], and for the grouped update [gbest nblk*ng*32 u64]
 // [gexp nblk*ng*32 u8] [blist nblk*32 int] [units nblk*ng uint2] (K = 0:
-// none).  Only the control words need zeroing before a launch; the team
+// none).  Only the control word needs zeroing before a launch; the team
 // clears the rest per batch (the initial scoring writes every gbest and gexp
 // entry).
 struct TeamLayout {
@@ -2092,8 +2090,7 @@ __host__ __device__ inline void bind_scratch(PeelArgs& a, char* team, char* list
                                              bool grouped) {
   const TeamLayout t = team_layout(a.L, grouped ? a.K : 0);
   const ListLayout l = list_layout(a.L);
-  a.bar = reinterpret_cast<unsigned*>(team);
-  a.err = reinterpret_cast<int*>(team) + 1;     // read with the count by the barrier
+  a.ctl = reinterpret_cast<unsigned long long*>(team);
   a.cfmax = reinterpret_cast<float*>(team + t.cfmax);
   a.imax = reinterpret_cast<int*>(team + t.imax);
   a.pack = reinterpret_cast<unsigned long long*>(team + t.pack);

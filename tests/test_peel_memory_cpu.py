@@ -1,0 +1,44 @@
+"""Rules of the peel's cross-block memory traffic, read from its source.
+
+Blocks of a team hand data to one another under the GPU's memory model, whose
+ordering only holds between accesses of the same width to the same word.  A
+breach shows in no output of the hardware at hand, so the source is checked.
+"""
+import os
+import re
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
+                    "kilosort_b200", "csrc")
+
+
+def source(name):
+    with open(os.path.join(CSRC, name)) as f:
+        return re.sub(r"//[^\n]*", "", f.read())
+
+
+def body(text, name):
+    """Text of the definition of function `name`, from its name to its last brace."""
+    start = re.search(r"\b%s\s*\([^;{]*\)\s*{" % re.escape(name), text)
+    assert start, name
+    depth, i = 1, start.end()
+    while depth:
+        depth += {"{": 1, "}": -1}.get(text[i], 0)
+        i += 1
+    return text[start.start():i]
+
+
+def test_barrier_accesses_have_one_width():
+    common = source("ks_common.cuh")
+    names = re.findall(r"\b(ks_grid_sync|ks_ctl_\w+)\s*\([^;{]*\)\s*{", common)
+    assert "ks_grid_sync" in names
+    widths = set()
+    for n in names:
+        text = body(common, n)
+        widths |= {int(w) for w in re.findall(r'"(?:ld|st|red|atom)\.[\w.]*?\.[bus](\d+) ', text)}
+        # the C++ atomics take their width from the word's type
+        assert not re.search(r"reinterpret_cast<|\((?:unsigned|int)\s*\*\)", text), n
+        if re.search(r"\batomic\w+\(", text):
+            assert re.search(r"unsigned long long\s*\*\s*ctl", text), n
+    assert widths == {64}
+    # and the peel keeps no narrower pointer to the word
+    assert not re.search(r"reinterpret_cast<(?:unsigned|int)\s*\*>\(team\)", source("peel_core.cuh"))
