@@ -823,14 +823,18 @@ __device__ __forceinline__ UnitIn* unit_in(const Smem& s, int warp, int i) {
   return s.unit + warp * kUnitSlots + i % kUnitSlots;
 }
 
+// Where a unit's touch list comes from: none (initial scores), the list that the
+// scan published, or the unit's slot, where the warp itself has put it (kPair).
+enum UnitKind { kInit, kListed, kPair };
+
 // Request unit u's inputs (cp.async, a 16-byte piece per lane).
-template <bool kInit>
+template <UnitKind kKind>
 __device__ __forceinline__ void unit_fetch(const PeelArgs& a, uint2 u, UnitIn* in, int lane) {
   const char* src;
   if (lane < 8) src = reinterpret_cast<const char*>(a.blist + (size_t)(u.x >> 11) * 32) + lane * 16;
   else if (lane < 16) src = reinterpret_cast<const char*>(a.rperm + (u.x & 2047u) * kGroup) + (lane - 8) * 16;
   else src = reinterpret_cast<const char*>(a.nmip + (u.x & 2047u) * kGroup) + (lane - 16) * 16;
-  if (!kInit || lane >= 8) cp_async16(reinterpret_cast<char*>(in) + lane * 16, src);
+  if (kKind == kListed || lane >= 8) cp_async16(reinterpret_cast<char*>(in) + lane * 16, src);
   cp_async_commit();
 }
 
@@ -1100,20 +1104,18 @@ __device__ __forceinline__ unsigned long long unit_fold(const PeelArgs& a, const
   return gb;
 }
 
-// The units first, first + step, ... (nu of them) of the iteration's list, or
-// (kInit) of all nblk * ng tiles, whose initial scores are folded (nothing is
-// subtracted or written back).  Per unit: its rows and staged
-// cross-correlations are waited for, the columns subtract their touching
-// peaks in application order (further peaks stage theirs in the slot's tile),
-// the rows are written back and scored.  The next unit's cross-correlations
-// are staged in the other slot once this unit's are applied, its rows are
-// requested once this unit's registers are free, and the one after it has its
-// inputs fetched.
-template <bool kInit>
+// The units first, first + step, ... (nu of them) of the iteration's list (one
+// unit with kPair), or (kInit) of all nblk * ng tiles, whose initial scores are
+// folded (nothing is subtracted or written back).  Per unit: its rows and staged
+// cross-correlations are waited for, the columns subtract their touching peaks
+// in application order (further peaks stage theirs in the tile once it is
+// read), the rows are written back and scored.  The next unit's inputs are
+// fetched once this one's peaks are applied.
+template <UnitKind kKind>
 __device__ void run_units(const PeelArgs& a, const Smem& s, long long first, long long step,
                           int nu, uint2 rec, unsigned long long* pack_out, int lane, int warp) {
   auto record = [&](int i) {
-    if (kInit) {
+    if (kKind == kInit) {
       const unsigned w = (unsigned)first + (unsigned)i * (unsigned)step, ng = (unsigned)a.ng;
       const int blk = (int)(w / ng), left = a.L - blk * kCol;
       return make_uint2(((unsigned)blk << 11) | (w % ng),
@@ -1125,7 +1127,7 @@ __device__ void run_units(const PeelArgs& a, const Smem& s, long long first, lon
   uint2 u = record(0);
   float* Cs = unit_tile(s, warp);
   __syncwarp();                       // the tile's and the slots' earlier readers are done
-  unit_fetch<kInit>(a, u, unit_in(s, warp, 0), lane);
+  unit_fetch<kKind>(a, u, unit_in(s, warp, 0), lane);
 #pragma unroll 1
   for (int i = 0; i < nu; ++i) {
     const UnitIn* in = unit_in(s, warp, i);
@@ -1133,11 +1135,11 @@ __device__ void run_units(const PeelArgs& a, const Smem& s, long long first, lon
     __syncwarp();                     // the unit's inputs have landed
     unsigned long long b[8][2];
     LaneEntries le{-1, 0u};
-    if (!kInit) le = unit_begin(a, in, u, Cs, lane);
+    if (kKind != kInit) le = unit_begin(a, in, u, Cs, lane);
     unit_rows(a, in, u, b, lane);
     uint2 un = u;
     if (i + 1 < nu) un = record(i + 1);
-    if (!kInit) {
+    if (kKind != kInit) {
       const unsigned long long one2 = f2_pack(a.one, a.one);
       unsigned long long n01, n23;
       column_pairs(le.e0 >= 0 ? -__int_as_float(in->list[1 + 2 * kTouch + le.e0]) : -0.f, lane, n01,
@@ -1158,7 +1160,7 @@ __device__ void run_units(const PeelArgs& a, const Smem& s, long long first, lon
         apply_ctc(Cs, n01, n23, one2, b, lane);
       }
     }
-    if (i + 1 < nu) unit_fetch<kInit>(a, un, unit_in(s, warp, i + 1), lane);
+    if (i + 1 < nu) unit_fetch<kKind>(a, un, unit_in(s, warp, i + 1), lane);
     // write back; the tile keeps the scores for the quotients
     {
       const int rq = lane >> 3;
@@ -1167,7 +1169,7 @@ __device__ void run_units(const PeelArgs& a, const Smem& s, long long first, lon
 #pragma unroll
       for (int r = 0; r < 8; ++r) {
         const ulonglong2 v = make_ulonglong2(b[r][0], b[r][1]);
-        if (!kInit)
+        if (kKind != kInit)
           *reinterpret_cast<ulonglong2*>(brow + (unsigned)in->row[4 * r + rq] * kCol) = v;
         *reinterpret_cast<ulonglong2*>(cs + r * 128) = v;
       }
@@ -1360,14 +1362,17 @@ __device__ __forceinline__ void scan_and_update(const PeelArgs& a, const Smem& s
   }
   const unsigned cols = __ballot_sync(0xffffffffu, need);
   if (!cols) return;
-  int* bl = a.blist + (size_t)blk * 32;
-  if (lane == 0) bl[0] = tl.n;
+  // the list goes to the warp's own slot: the warps of this block's other groups
+  // have theirs at the same time
+  int* list = unit_in(s, warp, 0)->list;
+  __syncwarp();                         // the slot's earlier readers are done
+  if (lane == 0) list[0] = tl.n;
   if (lane < tl.n) {
-    bl[1 + lane] = tl.tau[lane];
-    bl[1 + kTouch + lane] = tl.k[lane];
-    bl[1 + 2 * kTouch + lane] = __float_as_int(tl.amp[lane]);
+    list[1 + lane] = tl.tau[lane];
+    list[1 + kTouch + lane] = tl.k[lane];
+    list[1 + 2 * kTouch + lane] = __float_as_int(tl.amp[lane]);
   }
-  run_units<false>(a, s, 0, 1, 1, make_uint2(((unsigned)blk << 11) | (unsigned)g, cols), pack_out,
+  run_units<kPair>(a, s, 0, 1, 1, make_uint2(((unsigned)blk << 11) | (unsigned)g, cols), pack_out,
                    lane, warp);
 }
 
@@ -1429,7 +1434,7 @@ __device__ PeelOutcome run_peel(const PeelArgs& a, const Smem& s, int rank, unsi
       // every (block, group) tile: the group metadata of every column too
       const long long n_items = (long long)a.nblk * a.ng;
       if (gwarp < n_items)
-        run_units<true>(a, s, gwarp, nwarps, (int)((n_items - gwarp + nwarps - 1) / nwarps),
+        run_units<kInit>(a, s, gwarp, nwarps, (int)((n_items - gwarp + nwarps - 1) / nwarps),
                         make_uint2(0u, 0u), pinit, lane, warp);
     } else {
       const int rg = (a.K + kItemRows - 1) / kItemRows;
@@ -1499,8 +1504,8 @@ __device__ PeelOutcome run_peel(const PeelArgs& a, const Smem& s, int rank, unsi
         if (dealt) {
           if (gwarp < n_units) {
             const int nu = (int)((n_units - gwarp + nwarps - 1) / nwarps);
-            run_units<false>(a, s, gwarp, nwarps, nu, unit_records(a, gwarp, nwarps, nu, lane), pcur,
-                             lane, warp);
+            run_units<kListed>(a, s, gwarp, nwarps, nu, unit_records(a, gwarp, nwarps, nu, lane),
+                               pcur, lane, warp);
           }
         } else {
           while (true) {
@@ -1509,8 +1514,8 @@ __device__ PeelOutcome run_peel(const PeelArgs& a, const Smem& s, int rank, unsi
             first = __shfl_sync(0xffffffffu, first, 0);
             if (first >= n_units) break;
             const int nu = (int)(min(n_units, first + claim) - first);
-            run_units<false>(a, s, first, 1, nu, unit_records(a, first, 1, nu, lane), pcur, lane,
-                             warp);
+            run_units<kListed>(a, s, first, 1, nu, unit_records(a, first, 1, nu, lane), pcur,
+                               lane, warp);
           }
         }
       }
@@ -2027,13 +2032,13 @@ __global__ void __launch_bounds__(256) ks_group_bound_kernel(const float* __rest
 }
 
 // Scratch of one team (reused for every batch it processes), for batches of
-// up to L padded samples and K templates: [ctl 256 B: control word] [cfmax L] [imax L] [pack 2L] [chunk counts] [chunk buffers 4 x
-// nchunks*kChunk] [tcount 2 nblk] [touch 2 nblk*kTouch] [dbits 2 nwords]
-// [work counters 6], and for the grouped update [gbest nblk*ng*32 u64]
-// [gexp nblk*ng*32 u8] [blist nblk*32 int] [units nblk*ng uint2] (K = 0:
-// none).  Only the control word needs zeroing before a launch; the team
-// clears the rest per batch (the initial scoring writes every gbest and gexp
-// entry).
+// up to L padded samples and K templates: [ctl 256 B: control word] [cfmax L]
+// [imax L] [pack 2L] [chunk counts] [chunk buffers 4 x nchunks*kChunk]
+// [tcount 2 nblk] [touch 2 nblk*kTouch] [dbits 2 nwords] [work counters 6], and
+// for the grouped update [gbest nblk*ng*32 u64] [gexp nblk*ng*32 u8]
+// [blist nblk*32 int] [units nblk*ng uint2] (K = 0: none).  Only the control
+// word needs zeroing before a launch; the team clears the rest per batch (the
+// initial scoring writes every gbest and gexp entry).
 struct TeamLayout {
   size_t cfmax, imax, pack, chunk_cnt, chunk_tau, chunk_k, chunk_amp, chunk_th, tcount,
       touch, dbits, wctr, gbest, gexp, blist, units, bytes;

@@ -42,3 +42,15 @@ def test_barrier_accesses_have_one_width():
     assert widths == {64}
     # and the peel keeps no narrower pointer to the word
     assert not re.search(r"reinterpret_cast<(?:unsigned|int)\s*\*>\(team\)", source("peel_core.cuh"))
+
+
+def test_pairs_keep_their_touch_list_to_themselves():
+    """The warps that update a block's (block, group) pairs side by side have
+    equal lists; none may store its own where another reads."""
+    peel = source("peel_core.cuh")
+    shared = [n for n in re.findall(r"\b(\w+)\s*\([^;{}()]*\)\s*{", peel)
+              if "a.blist" in body(peel, n) and "reinterpret_cast<int*>(team" not in body(peel, n)]
+    assert sorted(set(shared)) == ["group_scan", "unit_fetch"]
+    # and a pair's inputs leave the published list out
+    assert re.search(r"if \(kKind == kListed \|\| lane >= 8\) cp_async16", body(peel, "unit_fetch"))
+    assert "run_units<kPair>" in body(peel, "scan_and_update")
