@@ -135,7 +135,8 @@ __global__ void __launch_bounds__(kThreads, kTeamBlocksPerSm) peel_multi_kernel(
     const Smem s = carve_smem(sa, smem_raw, true);
     PeelOutcome o{0, 0, KS_OK};
     if (!failed) {
-      o = run_peel<kRowsPerWarp, true>(sa, s, rank, (unsigned)p.team_size, epoch);
+      o = run_peel<kRowsPerWarp, true>(sa, s, rank, (unsigned)p.team_size, epoch,
+                                       i + n_teams < p.n_batches);
       failed = o.status != KS_OK && o.status != KS_ERR_OVERFLOW;   // overflow: that batch only
     }
     const bool good = !failed && o.status == KS_OK;

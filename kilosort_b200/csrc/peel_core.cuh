@@ -1390,9 +1390,10 @@ struct PeelOutcome {
 // (written by one thread) and is returned to every thread.  When the status
 // is KS_OK every record and residual list of the batch is complete and
 // visible to the team (the last pass ended at a team barrier).
+// `again`: another batch follows in the same scratch.
 template <int kRows, bool kGrouped>
 __device__ PeelOutcome run_peel(const PeelArgs& a, const Smem& s, int rank, unsigned G,
-                                unsigned& epoch) {
+                                unsigned& epoch, bool again) {
   const int tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5;
   // warps are numbered across the blocks, so that fewer items than warps are
@@ -1610,7 +1611,11 @@ __device__ PeelOutcome run_peel(const PeelArgs& a, const Smem& s, int rank, unsi
     ok = ks_grid_sync(a.ctl, G, epoch, a.limit_ns);
   }
   // one decision on the error for the whole block
-  const int e = __syncthreads_or(tid == 0 && ks_ctl_error(a.ctl) != 0) ? ks_ctl_error(a.ctl) : 0;
+  int e = __syncthreads_or(tid == 0 && ks_ctl_error(a.ctl) != 0) ? ks_ctl_error(a.ctl) : 0;
+  // The next batch's clearing and scores overwrite this scratch, and the blocks
+  // that left on the peak counts (no peak, too many) have passed no barrier since
+  // they read them: nobody goes on before all have.
+  if (again && !e && !ks_grid_sync(a.ctl, G, epoch, a.limit_ns)) e = ks_ctl_error(a.ctl);
   if (rank == 0 && tid == 0) {
     a.info[0] = n_out;
     a.info[1] = e ? e : status;
@@ -1627,7 +1632,7 @@ __global__ void __launch_bounds__(kThreads, kGrouped ? kBlocksPerSm : kTeamBlock
   extern __shared__ __align__(16) char smem_raw[];
   const Smem s = carve_smem(a, smem_raw, kGrouped);
   unsigned epoch = 0;
-  run_peel<kRowsPerWarp, kGrouped>(a, s, blockIdx.x, gridDim.x, epoch);
+  run_peel<kRowsPerWarp, kGrouped>(a, s, blockIdx.x, gridDim.x, epoch, false);
 }
 
 // the batched peel's residual scratch fits in the warp tiles

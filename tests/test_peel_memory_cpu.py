@@ -54,3 +54,19 @@ def test_pairs_keep_their_touch_list_to_themselves():
     # and a pair's inputs leave the published list out
     assert re.search(r"if \(kKind == kListed \|\| lane >= 8\) cp_async16", body(peel, "unit_fetch"))
     assert "run_units<kPair>" in body(peel, "scan_and_update")
+
+
+def test_scratch_is_reused_behind_a_barrier():
+    """A team's next batch overwrites the counts on which slower blocks leave the
+    last one: a barrier lies between the loop's exits and the return."""
+    peel = source("peel_core.cuh")
+    run = body(peel, "run_peel")
+    loop = run.index("++it) {")
+    depth, i = 1, loop + len("++it) {")
+    while depth:
+        depth += {"{": 1, "}": -1}.get(run[i], 0)
+        i += 1
+    tail = run[i:]
+    assert re.search(r"if \(again\b[^;]*ks_grid_sync\(a\.ctl", tail)
+    multi = body(source("batched.cu"), "peel_multi_kernel")
+    assert re.search(r"epoch,\s*i \+ n_teams < p\.n_batches\)", multi)
