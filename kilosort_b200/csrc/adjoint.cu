@@ -398,14 +398,15 @@ __global__ void __launch_bounds__(kAdjThreads) ks_adjoint_warp_kernel(
     const float* __restrict__ Xres, const long long* __restrict__ st,
     const float* __restrict__ amps, const float* __restrict__ U, const float* __restrict__ W,
     const int* __restrict__ offk, const int* __restrict__ list, const float* __restrict__ dloss,
-    int C, int L, int P, int nt, int nchunk, float* __restrict__ dU, float* __restrict__ dwpart,
-    float* __restrict__ dapart) {
+    int C, int L, int K, int P, int nt, int nchunk, float* __restrict__ dU,
+    float* __restrict__ dwpart, float* __restrict__ dapart) {
   extern __shared__ float sm[];
   float* sW = sm;                       // [P][nt]
   float* sD = sW + P * nt;              // [kAdjWarps][P][nt] partial dW of each warp
   __shared__ int sSpike[kAdjSpikes], sTau[kAdjSpikes];
   __shared__ float sAmp[kAdjSpikes], sDot[kAdjWarps][kAdjSpikes];
-  const int k = blockIdx.x, ch = blockIdx.y;
+  // one grid dimension: 16-channel chunks of a million channels exceed grid.y
+  const int k = (int)(blockIdx.x % K), ch = (int)(blockIdx.x / K);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int cw = ch * (kAdjWarps * CW) + warp * CW;     // the warp's first channel
   const int half = nt / 2;
@@ -759,7 +760,6 @@ extern "C" KS_API int ks_recon_adjoint(const float* Xres, const int64_t* st, con
     ks_group_by_template_kernel<<<(unsigned)K, 256, 0, s>>>(karr, N, offk, list);
     KS_CUDA(cudaGetLastError());
   }
-  const dim3 grid((unsigned)K, (unsigned)r.nchunk);
   const int ne = (int)((nt + 31) / 32);
   if (ne <= 4) {
     const size_t smem = sizeof(float) * (size_t)(1 + kAdjWarps) * P * nt;
@@ -767,12 +767,14 @@ extern "C" KS_API int ks_recon_adjoint(const float* Xres, const int64_t* st, con
                         : ne == 2 ? ks_adjoint_warp_kernel<2, 4>
                         : ne == 3 ? ks_adjoint_warp_kernel<3, 2> : ks_adjoint_warp_kernel<4, 2>;
     KS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kernel<<<grid, kAdjThreads, smem, s>>>(Xres, stp, amps, U, W, offk, list, dloss, (int)C, (int)L,
-                                           (int)P, (int)nt, (int)r.nchunk, dU, dwpart, dapart);
+    kernel<<<(unsigned)(K * r.nchunk), kAdjThreads, smem, s>>>(
+        Xres, stp, amps, U, W, offk, list, dloss, (int)C, (int)L, (int)K, (int)P, (int)nt,
+        (int)r.nchunk, dU, dwpart, dapart);
   } else {
     const size_t smem = sizeof(float) * ((size_t)P * nt + 2 * (size_t)kChunkC * nt + kAdjThreads / 32);
     if (smem > dev.smem_optin) return fail(KS_ERR_UNSUPPORTED, "ks_recon_adjoint: nt too long");
     KS_CUDA(cudaFuncSetAttribute(ks_adjoint_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const dim3 grid((unsigned)K, (unsigned)r.nchunk);
     ks_adjoint_kernel<<<grid, kAdjThreads, smem, s>>>(Xres, stp, amps, U, W, offk, list, dloss,
                                                       (int)C, (int)L, (int)K, (int)P, (int)nt,
                                                       (int)r.nchunk, dU, dwpart, dapart);

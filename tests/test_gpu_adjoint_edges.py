@@ -65,3 +65,20 @@ def test_non_finite_amplitude_reaches_the_loss():
     assert not np.isfinite(float(loss))
     lo, hi = max(0, int(st[0, 0]) - 15), min(300, int(st[0, 0]) + 16)
     assert not torch.isfinite(Xres[:, lo:hi]).any()
+
+
+def test_more_channel_chunks_than_grid_rows():
+    """65 to 128 taps go in chunks of 16 channels: 65537 of them here."""
+    from kilosort_b200.adjoint import reconstruction_loss
+    C, K, P, nt, L = 16 * 65536 + 5, 1, 1, 65, 6
+    g = torch.Generator().manual_seed(11)
+    X, U = torch.randn((C, L), generator=g), torch.randn((K, P, C), generator=g)
+    W = torch.randn((P, nt), generator=g) / nt ** 0.5
+    st, amps = torch.tensor([[1, 0], [4, 0]]), torch.tensor([1.5, -0.5])
+    q = [t.to(DEV).requires_grad_(True) for t in (amps, U, W)]
+    reconstruction_loss(X.to(DEV), st.to(DEV), *q).backward()
+    r = [t.double().requires_grad_(True) for t in (amps, U, W)]
+    oa.recon_loss(X.double(), st, *r).backward()
+    for got, ref in zip(q, r):
+        err = (got.grad.cpu().double() - ref.grad).abs().max()
+        assert err <= 1e-4 * ref.grad.abs().max() + 1e-6
