@@ -256,8 +256,7 @@ ks_recon_kernel(const float* __restrict__ X, ReconArgs a, const float* __restric
                 const int* __restrict__ ok, const float* __restrict__ oamp, int L, int nblk,
                 int ngrp, float* __restrict__ Xres, double* __restrict__ part) {
   extern __shared__ __align__(16) float sm[];
-  stage_basis(W, a.P, a.nt, sm, kRecThreads);
-  __syncthreads();
+  if (__syncthreads_or(stage_basis(W, a.P, a.nt, sm, kRecThreads))) a.sup = nullptr;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const long long w = (long long)blockIdx.x * (kRecThreads / 32) + warp;
   if (w >= (long long)nblk * ngrp) return;

@@ -1784,8 +1784,7 @@ __global__ void __launch_bounds__(kResThreads)
 ks_residual_kernel(PeelArgs a) {
   extern __shared__ __align__(16) char smem_raw[];
   float* sW = reinterpret_cast<float*>(smem_raw);
-  stage_basis(a.W, a.P, a.nt, sW, kResThreads);
-  __syncthreads();
+  if (__syncthreads_or(stage_basis(a.W, a.P, a.nt, sW, kResThreads))) a.sup = nullptr;
   const long long n_out = (int)a.info[1] == KS_OK ? a.info[0] : 0;
   const int n_iter = (int)a.info[2];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;

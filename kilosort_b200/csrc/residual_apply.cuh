@@ -43,10 +43,17 @@ __device__ __forceinline__ unsigned long long f2_add_prod(unsigned long long a,
   return f2_fma(one2, f2_mul(x, y), a);
 }
 
-// The basis [P][nt] in shared memory with rows P .. 7 zero.
-__device__ __forceinline__ void stage_basis(const float* W, int P, int nt, float* sW,
+// The basis [P][nt] in shared memory with rows P .. 7 zero.  Returns whether a
+// value that this thread staged is infinite or NaN.
+__device__ __forceinline__ bool stage_basis(const float* W, int P, int nt, float* sW,
                                             int nthreads) {
-  for (int i = threadIdx.x; i < 8 * nt; i += nthreads) sW[i] = i < P * nt ? W[i] : 0.f;
+  bool odd = false;
+  for (int i = threadIdx.x; i < 8 * nt; i += nthreads) {
+    const float w = i < P * nt ? W[i] : 0.f;
+    odd |= !(fabsf(w) < INFINITY);
+    sW[i] = w;
+  }
+  return odd;
 }
 
 // Per-warp scratch of the residual pass: the spike list (time, template,
@@ -88,7 +95,8 @@ __host__ __device__ inline int support_width(int C) { return ((C + kXCh - 1) / k
 // with packed FP32 operations: per element the reference's products in the
 // same order, each rounded as the scalar operation.  Spikes whose template is
 // exactly zero on the tile (a.sup) and whose amplitude is finite would subtract
-// +0 and are passed over.
+// +0 and are passed over (callers whose spikes do not come from this basis drop
+// a.sup when it is not finite: its product with a zero loading is NaN).
 //
 // What bounds it: instruction issue (about 5.5 warp instructions per channel
 // row and spike) next to the 8CL bytes of X and Xres (185 MB, 28 us).  The

@@ -82,3 +82,18 @@ def test_more_channel_chunks_than_grid_rows():
     for got, ref in zip(q, r):
         err = (got.grad.cpu().double() - ref.grad).abs().max()
         assert err <= 1e-4 * ref.grad.abs().max() + 1e-6
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_non_finite_basis_reaches_every_channel(bad):
+    """A tap that is not finite gives NaN also on channels where the template is
+    zero (0 times it), at that tap of every spike's window and nowhere else."""
+    from kilosort_b200.adjoint import reconstruct
+    X, U, W, st, amps = _case(70, 3, 2, 31, 300, 20, 6)
+    W[1, 7] = bad
+    Xres, _ = reconstruct(*(t.to(DEV) for t in (X, st, amps, U, W)))
+    hit = torch.zeros(300, dtype=torch.bool)
+    at = st[:, 0] - 15 + 7
+    hit[at[(at >= 0) & (at < 300)]] = True
+    finite = torch.isfinite(Xres.cpu())
+    assert not finite[:, hit].any() and finite[:, ~hit].all()

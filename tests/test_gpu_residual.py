@@ -89,3 +89,22 @@ def test_failed_batch_keeps_its_samples():
     info = m.info.cpu()
     assert int(info[0, 1]) == _lib.KS_ERR_OVERFLOW and int(info[1, 1]) == _lib.KS_OK
     assert torch.equal(m.outs[0].Xres, Xd) and torch.equal(m.outs[1].Xres, quiet)
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_non_finite_basis_reaches_every_channel(bad):
+    """The peel on given scores with a basis that is not finite at one tap: NaN at
+    that tap of every spike's window, also where the template is zero."""
+    import kilosort_b200 as kb
+    from kilosort_b200.template_matching import peel, project_scores, template_energy
+    X, U, W = (a.to(DEV) for a in _crowd(9, 48, 4, 6, 1500, 700))
+    ctc = kb.prepare_matching(dict(nt=NT, wPCA=W), U)
+    B = project_scores(X, U, W, NT, tiled=True)
+    W = W.clone()
+    W[2, 11] = bad
+    st = peel(B, X, U, W, ctc, template_energy(U), 9.0, NT, 200)[0].cpu()
+    assert len(st) >= 4
+    hit = torch.zeros(1500, dtype=torch.bool)
+    hit[st[:, 0] - NT // 2 + 11] = True
+    finite = torch.isfinite(X.cpu())
+    assert not finite[:, hit].any() and finite[:, ~hit].all()
