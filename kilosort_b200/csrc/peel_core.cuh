@@ -794,18 +794,6 @@ struct LaneEntries {
   unsigned rest;
 };
 
-__device__ __forceinline__ LaneEntries lane_entries(const TouchList& tl, int c, bool colok, int nt) {
-  LaneEntries le{-1, 0u};
-  for (int e = 0; e < tl.n; ++e) {
-    const int d = c - tl.tau[e];
-    if (colok && d >= -nt && d <= nt) {
-      if (le.e0 < 0) le.e0 = e;
-      else le.rest |= 1u << e;
-    }
-  }
-  return le;
-}
-
 // Inputs of a unit (a group tile that some columns of a block must process)
 // in shared memory: the block's ordered touch list as the scan published it,
 // the group's row indices and {nm, 1/sqrt(nm)}.  The tables are padded to whole

@@ -67,3 +67,50 @@ def test_peaks_and_amplitudes(C, F, nC, nC2, ns, nk, L, nt0, own):
         if near <= same and (a, b) not in found:
             missed += 1
     assert missed == 0 and (len(found) > 0 or not own)
+
+
+@pytest.mark.parametrize("C,F,nC,nC2,ns,nk,L,nt0", [
+    (24, 34, 10, 7, 5, 6, 1025, 20), (30, 64, 7, 1, 5, 6, 2100, 0), (12, 6, 4, 9, 8, 8, 700, 40),
+    (90, 66, 10, 20, 5, 6, 2049, 600)])
+def test_peaks_of_positions_without_their_own_row(C, F, nC, nC2, ns, nk, L, nt0):
+    """A position that is not its own neighbour peaks where a neighbour ties with
+    it: every position has a twin (same channels and weights, in another tile of
+    positions where there are several) as its first neighbour."""
+    from kilosort_b200 import spikedetect
+    rng = np.random.default_rng(C + 7 * F)
+    nt, th, half = 21, 3.0, F // 2
+    X = rng.standard_normal((C, L)).astype(np.float32)
+    iC = np.tile(np.stack([rng.permutation(C)[:nC] for _ in range(half)], 1), 2)
+    weigh = rng.uniform(0.1, 1, (ns, nC, half)).astype(np.float32)
+    weigh = np.tile(weigh / np.sqrt((weigh ** 2).sum(1, keepdims=True)), 2)
+    twin = (np.arange(F) + half) % F
+    others = [np.setdiff1d(np.arange(F), [f, twin[f]]) for f in range(F)]
+    iC2 = np.stack([np.concatenate([[twin[f]], rng.choice(others[f], nC2 - 1)]) for f in range(F)], 1)
+    wT = rng.standard_normal((nk, nt)).astype(np.float32)
+    wT /= np.linalg.norm(wT, axis=1, keepdims=True)
+    ops = dict(wTEMP=torch.from_numpy(wT), wPCA=torch.from_numpy(wT[:1].copy()),
+               yc=np.arange(C, dtype=np.float32), nt=nt, settings=dict(nt0min=nt0), Th_universal=th)
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(DEV)
+    xy, _, amp, _ = (a.cpu().numpy() for a in spikedetect.template_match(
+        t(X), ops, t(iC), t(iC2), t(weigh), torch.device(DEV)))
+    B = torch.nn.functional.conv1d(torch.from_numpy(X).double()[:, None],
+                                   torch.from_numpy(wT).double()[:, None], padding=nt // 2).numpy()
+    As = np.abs(np.einsum("sjf,jfkt->skft", weigh.astype(np.float64), B[iC])).reshape(-1, F, L).max(0)
+    As[half:] = As[:half]                # twins are the same numbers, not only close ones
+    tol = 1e-4                           # as above
+    f, s = xy[:, 0], xy[:, 1]
+    assert (np.abs(amp - As[f, s]) <= tol).all()
+    found, clear = set(zip(f.tolist(), s.tolist())), 0
+    for a, b in zip(*np.nonzero(As > th + tol)):
+        lo, hi = max(b - nt0, nt), min(b + nt0, L - nt - 1)
+        if not lo <= b <= hi:
+            continue
+        w = As[iC2[:, a], lo:hi + 1]
+        rest = w > As[a, b] - tol        # in the twin's column the twin alone
+        rest[iC2[:, a] == twin[a], b - lo] = False
+        if w.max() > As[a, b] + tol:
+            assert (a, b) not in found
+        elif not rest.any():
+            assert (a, b) in found
+            clear += 1
+    assert clear > 0
