@@ -4,8 +4,10 @@
  * Every entry point takes raw device pointers (row-major, contiguous unless a
  * leading dimension is given), int64 sizes, a CUDA stream (cudaStream_t passed
  * as void*) and, where scratch is needed, a caller-owned device workspace whose
- * size is returned by the matching *_workspace_size() query.  The library never
- * allocates device memory and never synchronises the stream, except where a
+ * size is returned by the matching *_workspace_size() query.  A workspace and a
+ * tiled B are 16-byte aligned (ks_match_batches' workspace 256; ks_peel with a
+ * tiled B, ks_recon_loss and ks_recon_adjoint take any 8-byte aligned workspace).
+ * The library never allocates device memory and never synchronises the stream, except where a
  * function says so.  Return value: 0 (KS_OK) or a KS_ERR_* code; a readable
  * message for the last failure on the calling thread is in ks_last_error().
  *

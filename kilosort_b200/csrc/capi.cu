@@ -178,6 +178,7 @@ int ks_project(const float* X, const float* U, const float* W, int64_t C,
   if (!X || !U || !W || !B) return fail(KS_ERR_ARG, "ks_project: null pointer");
   if (b_layout != KS_B_ROWS && b_layout != KS_B_TILED)
     return fail(KS_ERR_ARG, "ks_project: unknown B layout");
+  if (!aligned16(workspace)) return fail(KS_ERR_ARG, "ks_project: workspace must be 16-byte aligned");
   DeviceInfo d;
   int rc = device_info(&d);
   if (rc) return rc;
@@ -208,6 +209,9 @@ int ks_peel(float* B, int64_t ldb, int b_layout, float* Xres, const float* U, co
     return fail(KS_ERR_WORKSPACE, "ks_peel: workspace too small");
   char* base = static_cast<char*>(workspace);
   float* Bt = b_layout == KS_B_TILED ? B : reinterpret_cast<float*>(base + m.b_off);
+  if (!aligned16(Bt))
+    return fail(KS_ERR_ARG, b_layout == KS_B_TILED ? "ks_peel: tiled B must be 16-byte aligned"
+                                                   : "ks_peel: workspace must be 16-byte aligned");
   const float* ctcT = ctc;
   int rc;
   if (ctc_layout == KS_CTC_JKL) {
@@ -248,6 +252,8 @@ int ks_run_matching(const float* X, const float* U, const float* W, const float*
   const MatchLayout m = match_layout(C, L, K, P, nt, precision, ctc_layout);
   if (!workspace || workspace_bytes < m.bytes)
     return fail(KS_ERR_WORKSPACE, "ks_run_matching: workspace too small");
+  if (!aligned16(workspace))
+    return fail(KS_ERR_ARG, "ks_run_matching: workspace must be 16-byte aligned");
   DeviceInfo d;
   int rc = device_info(&d);
   if (rc) return rc;

@@ -197,6 +197,7 @@ int launch_ctc(const float* U, const float* W, int64_t K, int64_t P, int64_t C,
   if (P > 16 || nt > 1023) return fail(KS_ERR_UNSUPPORTED, "ks_ctc: P <= 16 and nt <= 1023");
   const CtcLayout lay = ctc_layout(K, P, C, nt);
   if (!ws || ws_bytes < lay.bytes) return fail(KS_ERR_WORKSPACE, "ks_ctc: workspace too small");
+  if (!aligned16(ws)) return fail(KS_ERR_ARG, "ks_ctc: workspace must be 16-byte aligned");
   Carve cv(ws);
   float* Upad = cv.take<float>((size_t)lay.rows * lay.cols);
   float* G = cv.take<float>((size_t)K * P * lay.ldg);

@@ -714,6 +714,8 @@ extern "C" KS_API int ks_detect(const float* X, int64_t C, int64_t L, const floa
   const DetectLayout d = detect_layout(C, L, nk, Nfilt);
   if (!workspace || workspace_bytes < d.bytes)
     return fail(KS_ERR_WORKSPACE, "ks_detect: workspace too small");
+  if (C <= kMaxCBits && !aligned16(workspace))
+    return fail(KS_ERR_ARG, "ks_detect: workspace must be 16-byte aligned");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const long long* iCl = reinterpret_cast<const long long*>(iC);
   const long long* iC2l = reinterpret_cast<const long long*>(iC2);

@@ -21,6 +21,8 @@ int cuda_fail(cudaError_t e, const char* what);
     if (_e != cudaSuccess) return ::ks::cuda_fail(_e, #call); \
   } while (0)
 
+// Arrays that the kernels read and write 16 bytes at a time.
+inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 inline int64_t round_up(int64_t x, int64_t m) { return (x + m - 1) / m * m; }
 inline size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 

@@ -137,3 +137,24 @@ def test_static_peel_limits_are_checked_before_the_device():
     assert rc == _lib.KS_ERR_UNSUPPORTED
     msg = lib.ks_last_error()
     assert b"K=56897" in msg and b"56896" in msg
+
+
+def test_arrays_read_16_bytes_at_a_time_are_checked_for_alignment():
+    """Addresses that no call gets to use: the check precedes the device."""
+    lib = _lib.load()
+    p, odd, many = 1 << 20, (1 << 20) + 8, 1 << 40
+    peel = lambda B, layout, ws: lib.ks_peel(
+        B, 64, layout, p, p, p, p, _lib.KS_CTC_KJL, p, 4, 64, 2, 6, 61, 64.0, 100, 10, p, p, p, p,
+        ws, many, None)
+    calls = [
+        lambda: peel(odd, _lib.KS_B_TILED, p), lambda: peel(p, _lib.KS_B_ROWS, odd),
+        lambda: lib.ks_project(p, p, p, 4, 64, 2, 6, 61, _lib.KS_PROJ_FP32, p, 64, _lib.KS_B_ROWS,
+                               None, odd, many, None),
+        lambda: lib.ks_run_matching(p, p, p, p, _lib.KS_CTC_KJL, 4, 64, 2, 6, 61, 64.0, 100,
+                                    _lib.KS_PROJ_FP32, 10, p, p, p, p, p, odd, many, None),
+        lambda: lib.ks_ctc(p, p, 2, 6, 4, 61, p, odd, many, None),
+        lambda: lib.ks_detect(p, 4, 64, p, 6, 61, p, 4, p, 5, p, 5, 8, 20, 9.0, p, 6, p, 10, p, p,
+                              p, p, p, p, p, odd, many, None)]
+    for call in calls:
+        assert call() == _lib.KS_ERR_ARG
+        assert b"16-byte aligned" in lib.ks_last_error()
