@@ -255,74 +255,76 @@ __device__ __forceinline__ float warp_median(const float (&v)[NJ], int C, float 
 // instead the bf16 hi/lo planes of the circularly padded batch
 // P[c][j] = x[c][(j - h) mod L], j < cols (sample t at every j = t + h mod L).
 //
-// A block takes 32 samples, a warp four of them in turn: lane l holds the
-// channels l + 32j (32 NJ of them at a time; with kCar all), the next sample's
+// A block takes 32 samples of 32 NJ channels (with kCar all of them), a warp four
+// of the samples in turn: lane l holds the channels l + 32j, the next sample's
 // loads in flight while this one's median is found in registers; the results
 // meet in shared memory as rows of 32 samples per channel.  Bound by issue slots
 // (about 700 instructions per sample of 384 channels, 300 of them the median's
 // counts and ranks): 75 us at C=384, L=60122, where a median re-reading the tile
-// from shared memory three times took 142.
+// from shared memory three times took 142.  Without kCar 128 channels a block:
+// with all of them, 128 at a time, a block of C=1000 had an SM to itself (whole
+// filter without whitening 684 us, now 491).
 template <bool kCar, bool kPad, int NJ>
 __global__ void __launch_bounds__(kCarThreads, NJ <= 12 ? 3 : 1)
 ks_pre_car_kernel(const int16_t* __restrict__ raw, int L, long long ldr,
-                  const long long* __restrict__ map, int C, float sign,
+                  const long long* __restrict__ map, int C_all, float sign,
                   const double* __restrict__ sums, float* __restrict__ Xc,
                   __nv_bfloat16* __restrict__ Phi, __nv_bfloat16* __restrict__ Plo, int h,
                   long long cols, int* err) {
   extern __shared__ __align__(16) float sm[];
   constexpr int pitch = kCarTile + 1;
   constexpr int kWarps = kCarThreads / 32, kPer = kCarTile / kWarps;
-  int* hist = reinterpret_cast<int*>(sm);                  // [8 warps][256]
-  float* cand = reinterpret_cast<float*>(hist + kWarps * 256);    // [8 warps][32]
+  constexpr int Cr = 32 * NJ;                              // channels, rounded up
   // column of each channel, its mean
-  const int Cr = (C + 127) / 128 * 128;                    // = 32 NJ with kCar
-  long long* off = reinterpret_cast<long long*>(cand + kWarps * 32);   // [Cr]
+  long long* off = reinterpret_cast<long long*>(sm);       // [Cr]
   float* mean = reinterpret_cast<float*>(off + Cr);        // [Cr]
-  float* tile = mean + Cr;                                 // [C][pitch]
-  const int t0 = blockIdx.x * kCarTile;
+  int* hist = reinterpret_cast<int*>(mean + Cr);           // kCar: [8 warps][256]
+  float* cand = reinterpret_cast<float*>(hist + kWarps * 256);    // kCar: [8 warps][32]
+  float* tile = kCar ? cand + kWarps * 32 : mean + Cr;     // [C][pitch]
+  const int groups = kCar ? 1 : (C_all + Cr - 1) / Cr;     // channel groups
+  const int cb = (int)(blockIdx.x % groups) * Cr, C = min(Cr, C_all - cb);
+  const int t0 = (int)(blockIdx.x / groups) * kCarTile;
   const int nt = min(kCarTile, L - t0);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int c = threadIdx.x; c < Cr; c += kCarThreads) {
-    const long long m = c >= C ? 0 : map ? map[c] : c;
+    const long long m = c >= C ? 0 : map ? map[cb + c] : cb + c;
     const bool bad = m < 0 || m >= ldr;
     if (bad) atomicCAS(err, 0, KS_ERR_ARG);
     off[c] = bad ? 0 : m;
     // the mean of the (sign-inverted) samples: negation commutes with the
     // rounded mean and difference, so this is fl(sign * raw - mean(sign * raw));
     // past the last channel every value is +infinity
-    mean[c] = c < C ? sign * (float)(sums[c] / (double)L) : -INFINITY;
+    mean[c] = c < C ? sign * (float)(sums[cb + c] / (double)L) : -INFINITY;
   }
   __syncthreads();
   const float rC = 1.f / (float)C;
-  for (int c0 = 0; c0 < C; c0 += 32 * NJ) {
-    unsigned x[NJ];
-    auto load = [&](int s) {
-      // past the batch the last sample again, not written
-      const int16_t* row = raw + (long long)(t0 + min(s, nt - 1)) * ldr;
+  unsigned x[NJ];
+  auto load = [&](int s) {
+    // past the batch the last sample again, not written
+    const int16_t* row = raw + (long long)(t0 + min(s, nt - 1)) * ldr;
 #pragma unroll
-      for (int j = 0; j < NJ; ++j) x[j] = (unsigned short)row[off[c0 + lane + 32 * j]];
-    };
-    load(warp);
+    for (int j = 0; j < NJ; ++j) x[j] = (unsigned short)row[off[lane + 32 * j]];
+  };
+  load(warp);
 #pragma unroll 1
-    for (int i = 0; i < kPer; ++i) {
-      const int s = warp + kWarps * i;
-      float v[NJ];
+  for (int i = 0; i < kPer; ++i) {
+    const int s = warp + kWarps * i;
+    float v[NJ];
 #pragma unroll
-      for (int j = 0; j < NJ; ++j) {
-        // 2^23 + 2^15 + x exactly, from the bits
-        const float f = __uint_as_float((x[j] ^ 0x8000u) | 0x4b000000u) - 8421376.f;
-        v[j] = fmaf(sign, f, -mean[c0 + lane + 32 * j]);
-      }
-      if (s >= nt) break;
-      if (i + 1 < kPer) load(s + kWarps);
-      float med = 0.f;
-      if (kCar) med = warp_median(v, C, rC, (C - 1) / 2, hist + warp * 256, cand + warp * 32);
+    for (int j = 0; j < NJ; ++j) {
+      // 2^23 + 2^15 + x exactly, from the bits
+      const float f = __uint_as_float((x[j] ^ 0x8000u) | 0x4b000000u) - 8421376.f;
+      v[j] = fmaf(sign, f, -mean[lane + 32 * j]);
+    }
+    if (s >= nt) break;
+    if (i + 1 < kPer) load(s + kWarps);
+    float med = 0.f;
+    if (kCar) med = warp_median(v, C, rC, (C - 1) / 2, hist + warp * 256, cand + warp * 32);
 #pragma unroll
-      for (int j = 0; j < NJ; ++j) {
-        const int c = c0 + lane + 32 * j;
-        if ((kCar && j < NJ - 4) || c < C)
-          tile[c * pitch + s] = kCar ? __fsub_rn(v[j], med) : v[j];
-      }
+    for (int j = 0; j < NJ; ++j) {
+      const int c = lane + 32 * j;
+      if ((kCar && j < NJ - 4) || c < C)
+        tile[c * pitch + s] = kCar ? __fsub_rn(v[j], med) : v[j];
     }
   }
   __syncthreads();
@@ -335,13 +337,13 @@ ks_pre_car_kernel(const int16_t* __restrict__ raw, int L, long long ldr,
       for (int c = warp; c < C; c += kWarps) {
         const float y = tile[c * pitch + lane];
         const __nv_bfloat16 hv = __float2bfloat16_rn(y);
-        Phi[(size_t)c * cols + j] = hv;
-        Plo[(size_t)c * cols + j] = __float2bfloat16_rn(y - __bfloat162float(hv));
+        Phi[(size_t)(cb + c) * cols + j] = hv;
+        Plo[(size_t)(cb + c) * cols + j] = __float2bfloat16_rn(y - __bfloat162float(hv));
       }
     }
   } else {
     for (int c = warp; c < C; c += kWarps)
-      Xc[(size_t)c * L + t0 + lane] = tile[c * pitch + lane];
+      Xc[(size_t)(cb + c) * L + t0 + lane] = tile[c * pitch + lane];
   }
 }
 
@@ -543,10 +545,12 @@ extern "C" KS_API int ks_preprocess_int16(const int16_t* raw, int64_t L, int64_t
   __nv_bfloat16* phi = reinterpret_cast<__nv_bfloat16*>(base + p.phi);
   __nv_bfloat16* plo = reinterpret_cast<__nv_bfloat16*>(base + p.plo);
   {
-    const size_t smem = (sizeof(float) + sizeof(long long)) * (size_t)ks::round_up(C, 128) +
-                        sizeof(float) * (kCarTile + 1) * (size_t)C +
-                        (kCarThreads / 32) * (sizeof(int) * 256 + sizeof(float) * 32);
-    const unsigned grid = (unsigned)((L + kCarTile - 1) / kCarTile);
+    // without the median 128 channels a block
+    const int64_t Cb = do_car ? C : std::min<int64_t>(C, 128);
+    const size_t smem = (sizeof(float) + sizeof(long long)) * (size_t)ks::round_up(Cb, 128) +
+                        sizeof(float) * (kCarTile + 1) * (size_t)Cb +
+                        (do_car ? (kCarThreads / 32) * (sizeof(int) * 256 + sizeof(float) * 32) : 0);
+    const unsigned grid = (unsigned)((L + kCarTile - 1) / kCarTile * ((C + Cb - 1) / Cb));
     const float sign = invert_sign ? -1.f : 1.f;
     auto run = [&](auto kernel) -> int {
       KS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));

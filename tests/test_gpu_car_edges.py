@@ -44,3 +44,17 @@ def test_exact_values(cuda_device, n_bin, C, L, car, inv, kind):
     if car:
         ref = ref - np.sort(ref, axis=0)[(C - 1) // 2]
     assert got.dtype == np.float32 and np.array_equal(got, ref)
+
+
+@pytest.mark.parametrize("C,L,hp", [(129, 700, True), (300, 1057, False), (300, 3000, True)])
+def test_channel_groups_without_the_median(cuda_device, C, L, hp):
+    """Without the common average channels do not meet: any split of them gives the
+    same values as all together (blocks take 128)."""
+    from kilosort_b200.preprocess import Preprocessor
+    rng = np.random.default_rng(C + L)
+    raw = torch.from_numpy(_raw("normal", rng, L, C + 5)).to(DEV)
+    cmap = rng.permutation(C + 5)[:C]
+    filt = torch.from_numpy(rng.standard_normal(401).astype(np.float32)) / 20 if hp else None
+    run = lambda m: Preprocessor(C + 5, L, whiten=None, chan_map=m, hp_filter=filt, do_CAR=False,
+                                 artifact_threshold=float("inf"), device=DEV)(raw)
+    assert torch.equal(run(cmap), torch.cat([run(cmap[i:i + 77]) for i in range(0, C, 77)]))
