@@ -1,15 +1,18 @@
 // Per-spike PC features (kilosort/template_matching.py:85-86) and the
 // per-template channel selection of prepare_extract (:50-51).
 //
-// ks_features_kernel: one warp per spike.  For four at a time of the nC channels
+// ks_features_kernel: one warp per spike.  For G at a time of the nC channels
 // nearest to the template's peak channel the warp gathers the nt-sample
 // residual windows around the spike (lanes over taps), projects them on the P
 // basis rows and adds amp * Ucc, rounding the product and the sum separately as
-// the reference does.  The 4 x 8 partial sums of a lane are reduced over the
-// lanes by halves, 31 shuffles that leave one (channel, component) per lane, in
-// the butterfly's order.  Output [N, nC, P] (the layout `extract` stores, :108).
+// the reference does.  The G x 8 partial sums of a lane are reduced over the
+// lanes by halves once there are as many as lanes left to part, 31 shuffles at G
+// = 4 that leave one (channel, component) per lane, in the butterfly's order.
+// Output [N, nC, P] (the layout `extract` stores, :108).
 // Latency-bound: 28 us for a batch of C=384, K=600, 10 channels of 6 components
-// (64 us with one channel at a time and a butterfly per component).
+// at four channels a time (64 us with one channel at a time and a butterfly per
+// component).  A single channel takes G = 1: 31 us per 20000 spikes of 61 taps, 41
+// with four copies of it side by side.
 #include "ks_common.cuh"
 #include "project.cuh"
 
@@ -17,6 +20,7 @@ namespace ks {
 
 constexpr int kFeatWarps = 8;
 
+template <int G>
 __global__ void __launch_bounds__(kFeatWarps * 32)
 ks_features_kernel(const float* __restrict__ Xres, const long long* __restrict__ st,
                    const float* __restrict__ amps, const float* __restrict__ W,
@@ -45,40 +49,46 @@ ks_features_kernel(const float* __restrict__ Xres, const long long* __restrict__
   const float amp = amps[s];
   const int peak = (int)iU[k];
   const int p = lane & 7;               // the lane's component after the reduction
-  for (int i0 = 0; i0 < nC; i0 += 4) {
-    const float* x[4];
+  for (int i0 = 0; i0 < nC; i0 += G) {
+    const float* x[G];
 #pragma unroll
-    for (int g = 0; g < 4; ++g) {
+    for (int g = 0; g < G; ++g) {
       int c = (int)iCC[(long long)min(i0 + g, nC - 1) * C + peak];
       if (c < 0 || c >= C) c = 0;
       x[g] = Xres + (long long)c * L + t0;
     }
     const int i = i0 + (lane >> 3);
-    const bool out = i < nC && p < P;
+    const bool out = lane < 8 * G && i < nC && p < P;
     const float u = out ? Ucc[((long long)i * K + k) * P + p] : 0.f;
-    float part[32];                     // [channel][component]
+    float part[8 * G];                  // [channel][component]
 #pragma unroll
-    for (int q = 0; q < 32; ++q) part[q] = 0.f;
+    for (int q = 0; q < 8 * G; ++q) part[q] = 0.f;
 #pragma unroll 2
     for (int t = lane; t < nt; t += 32) {
-      float xv[4];
+      float xv[G];
 #pragma unroll
-      for (int g = 0; g < 4; ++g) xv[g] = x[g][t];
+      for (int g = 0; g < G; ++g) xv[g] = x[g][t];
 #pragma unroll
       for (int q = 0; q < 8; ++q)
         if (q < P) {
           const float w = sW[q * nt + t];
 #pragma unroll
-          for (int g = 0; g < 4; ++g) part[8 * g + q] = fmaf(xv[g], w, part[8 * g + q]);
+          for (int g = 0; g < G; ++g) part[8 * g + q] = fmaf(xv[g], w, part[8 * g + q]);
         }
     }
 #pragma unroll
     for (int o = 16; o; o >>= 1) {
-      const bool up = lane & o;
+      if (o < 8 * G) {
+        const bool up = lane & o;
 #pragma unroll
-      for (int q = 0; q < o; ++q) {
-        const float send = up ? part[q] : part[q + o];
-        part[q] = (up ? part[q + o] : part[q]) + __shfl_xor_sync(0xffffffffu, send, o);
+        for (int q = 0; q < (o < 8 * G ? o : 0); ++q) {
+          const float send = up ? part[q] : part[q + o];
+          part[q] = (up ? part[q + o] : part[q]) + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+      } else {
+#pragma unroll
+        for (int q = 0; q < 8 * G; ++q)
+          if (q < P) part[q] += __shfl_xor_sync(0xffffffffu, part[q], o);
       }
     }
     if (out) tF[(s * nC + i) * P + p] = __fadd_rn(part[0], __fmul_rn(amp, u));
@@ -134,7 +144,8 @@ int launch_features(const float* Xres, const int64_t* st, const float* amps,
     return fail(KS_ERR_ARG, "ks_features: bad sizes (need 1 <= P <= 8, 1 <= nC <= C)");
   const long long blocks = (N + kFeatWarps - 1) / kFeatWarps;
   const size_t smem = sizeof(float) * P * nt;
-  ks_features_kernel<<<(unsigned)blocks, kFeatWarps * 32, smem, stream>>>(
+  const auto kernel = nC == 1 ? ks_features_kernel<1> : ks_features_kernel<4>;
+  kernel<<<(unsigned)blocks, kFeatWarps * 32, smem, stream>>>(
       Xres, reinterpret_cast<const long long*>(st), amps, W,
       reinterpret_cast<const long long*>(iCC), reinterpret_cast<const long long*>(iU), Ucc,
       (int)C, (int)L, (int)K, (int)P, (int)nt, (int)nC, N,

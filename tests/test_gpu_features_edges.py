@@ -31,3 +31,21 @@ def test_against_double(cuda_device, P, nt, nC, N):
         u = Ucc[:, k].astype(np.float64) * float(amps[s])
         ref, mag = win @ Wd.T + u, np.abs(win) @ np.abs(Wd).T + np.abs(u)
         assert (np.abs(got[s] - ref) <= (nt / 32 + 8) * 2.0 ** -24 * mag).all()
+
+
+@pytest.mark.parametrize("P,nt,N", [(1, 31, 5), (6, 61, 300), (5, 95, 20), (8, 129, 9)])
+def test_one_channel_alone(cuda_device, P, nt, N):
+    """A single channel has its own form: the same bits as beside others."""
+    import kilosort_b200 as kb
+    g = torch.Generator(device=DEV).manual_seed(P)
+    rnd = lambda *s: torch.randn(s, generator=g, device=DEV)
+    C, L, K, nC = 9, 1500, 5, 6
+    st = torch.stack([torch.randint(nt, L - nt, (N,), generator=g, device=DEV),
+                      torch.randint(0, K, (N,), generator=g, device=DEV)], 1)
+    iCC = torch.randint(0, C, (nC, C), generator=g, device=DEV)
+    args = rnd(C, L), st, rnd(N), rnd(P, nt)
+    iU, Ucc = torch.randint(0, C, (K,), generator=g, device=DEV), rnd(nC, K, P)
+    want = kb.spike_features(*args, iCC, iU, Ucc)
+    for i in range(nC):
+        got = kb.spike_features(*args, iCC[i:i + 1].contiguous(), iU, Ucc[i:i + 1].contiguous())
+        assert torch.equal(got, want[:, i:i + 1])
