@@ -12,12 +12,13 @@
 // Kernels
 //   ks_prep_templates  nm[k] and Uq (both precisions)
 //   ks_temporal        X -> Yt: each thread owns 8 consecutive samples of one
-//                      channel and all P components (8*P FMA per tap, one
-//                      shared-memory load of X per tap); output staged in
-//                      shared memory and written as contiguous rows
+//                      channel and all P components, in pairs through packed
+//                      multiply-adds, its samples in a register window that
+//                      moves on 8 taps at a time; f32 rows turned in shared
+//                      memory and written as whole sectors
 //   ks_sgemm_tn        FP32 SIMT contraction with packed multiply-adds, tiles of
-//                      64 to 128 rows x 128 or 256 columns, register double
-//                      buffering; tile order puts the template tiles of one time
+//                      64 to 128 rows x 128 columns or of 128 x 256, register
+//                      double buffering; tile order puts the template tiles of one time
 //                      tile next to each other so each Yt tile is read from HBM
 //                      once
 #include "ks_common.cuh"
@@ -333,8 +334,8 @@ __device__ __forceinline__ unsigned long long dup2(float v) {
 // (both zero padded), Kd % 16 == 0.  Stores m < M, n < N, row-major with
 // leading dimension ldc, or (kTiled) in 32-column blocks
 // C[((n/32)*M + m)*32 + n%32]; `upper` leaves out the tiles below the diagonal.
-// Tiles of BM = 16 TM rows x 128 columns, TM x 8
-// per thread, columns two at a time through packed operations.
+// Tiles of BM = 16 TM rows x 16 TN columns, TM x TN per thread, columns two at a
+// time through packed operations.
 //
 // What bounds it: the FP32 pipe.  A packed operation does the work of two
 // issue slots, so loads and moves no longer compete with the multiply-adds:
@@ -514,14 +515,14 @@ int sgemm_tn(const float* A, const float* Bt, float* Cm, int64_t M, int64_t N,
   const int rc = device_info(&dev);
   if (rc) return rc;
   const int rows = sgemm_rows(M);
-  // 256 columns need fewer shared-memory reads per multiply-add, one block per
-  // SM; with fewer than 2.5 tiles per SM their last wave costs more than that
-  // (80 x 60122 x 576: 249 us with 256 columns, 192 with 128; 3600 x 3600 x 384:
-  // 197 and 219)
-  const int64_t wide = ((M + rows - 1) / rows) * ((N + 255) / 256);
+  // 256 columns by 128 rows need fewer shared-memory reads per multiply-add, one
+  // block per SM; with fewer than 2.5 tiles per SM their last wave costs more than
+  // that (80 x 60122 x 576: 249 us with 256 columns, 192 with 128; 3600 x 3600 x
+  // 384: 197 and 219).  96 rows by 256 columns took longer for a wave than 128 rows
+  // (464 and 400 us at a depth of 2304), so that height is for 128 columns only.
+  const int64_t wide = ((M + 127) / 128) * ((N + 255) / 256);
   if (2 * wide >= 5 * dev.sm_count && rows != 64)
-    return rows == 96 ? launch_sgemm<6, 16>(A, Bt, Cm, M, N, Kd, ldc, stream, tiled, upper)
-                      : launch_sgemm<8, 16>(A, Bt, Cm, M, N, Kd, ldc, stream, tiled, upper);
+    return launch_sgemm<8, 16>(A, Bt, Cm, M, N, Kd, ldc, stream, tiled, upper);
   switch (rows) {
     case 64: return launch_sgemm<4, 8>(A, Bt, Cm, M, N, Kd, ldc, stream, tiled, upper);
     case 96: return launch_sgemm<6, 8>(A, Bt, Cm, M, N, Kd, ldc, stream, tiled, upper);

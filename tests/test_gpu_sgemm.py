@@ -33,3 +33,18 @@ def test_scores_within_the_chain_bound(K, L, tiled):
 
     want, size = scores(X, U, W), scores(X.abs(), U.abs(), W.abs())
     assert ((B.double() - want).abs() <= (C * P + nt + 2) * 2.0 ** -24 * size).all()
+
+
+@pytest.mark.parametrize("K,L", [(130, 60122), (160, 40000), (192, 47500), (385, 60122), (400, 25000)])
+def test_tile_shape_does_not_change_a_score(K, L):
+    """96-row heights and 256-column tiles on both sides of the line between them:
+    a template's scores are those of the call with 64 templates, bit for bit."""
+    from kilosort_b200.template_matching import project_scores
+    g = torch.Generator(device=DEV).manual_seed(K)
+    X = torch.randn((5, L), generator=g, device=DEV)
+    U = torch.randn((K, 6, 5), generator=g, device=DEV)
+    W = torch.randn((6, 21), generator=g, device=DEV)
+    B = project_scores(X, U, W, 21, projection="fp32")
+    for k in range(0, K, 64):
+        part = project_scores(X, U[k:k + 64].contiguous(), W, 21, projection="fp32")
+        assert torch.equal(part, B[k:k + 64])
