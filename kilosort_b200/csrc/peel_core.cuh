@@ -942,8 +942,9 @@ __device__ __forceinline__ void unit_rows(const PeelArgs& a, const UnitIn* in, u
 //
 // The best over the group's rows is found without a division per row.  With
 // t = fl(b * fl(1/sqrt(nm))), nm in [2^-30, 2^30], t is within a relative
-// 2^-23 of b/sqrt(nm), so for t in [2^-45, 2^60] (b^2 and the quotient then
-// normal) the exactly rounded scores cf = fl(fl(b^2) / nm) of two rows are
+// 2^-23 of b/sqrt(nm), so for a largest t in [2^-45, 2^48] (its b is then in
+// [2^-60, 2^63], its square and quotient normal, and no row's square infinite)
+// the exactly rounded scores cf = fl(fl(b^2) / nm) of two rows are
 // ordered as their t wherever those differ by more than a relative 2^-21: only
 // rows with t >= (1 - 2^-20) max t can hold the best, and only their quotients
 // are computed and folded (larger score, then the smaller template index).
@@ -1048,7 +1049,7 @@ __device__ __forceinline__ unsigned long long unit_fold(const PeelArgs& a, const
   const float mo = us.mo;
   float best = 0.f;
   int arg = __reduce_min_sync(0xffffffffu, in->row[lane]);
-  const bool all = odd_nm || !(mo <= 0.f || (mo >= 2.8421709e-14f && mo <= 1.1529215e18f));
+  const bool all = odd_nm || !(mo <= 0.f || (mo >= 2.8421709e-14f && mo <= 2.8147498e14f));
   unsigned rows = us.rows;
   if (!ond || all || !(mo > 0.f)) rows = 0u;
   if (rows) best = -1.f;

@@ -70,3 +70,41 @@ def test_teams_equal_single_batches(teams):
     for x, got in zip(Xs, out):
         want = kb.run_matching(ops, x, U, ctc, device=x.device)
         assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("e", [30, 44, 47, 50, 53, 56, 58, 60, 62, 64])
+@pytest.mark.parametrize("spread", [False, True])
+def test_scores_at_the_end_of_the_range(e, spread):
+    """Scores whose squares pass through the end of FP32's range (some rows' are
+    infinite, others' are not, whatever their order by b/sqrt(nm)), with template
+    energies close together and spread over most of 2^-30 .. 2^30."""
+    from kilosort_b200 import _lib
+    from kilosort_b200.template_matching import peel, project_scores, template_energy, transpose_ctc
+    import kilosort_b200 as kb
+    K, NT, nt, P = 70, 1500, 61, 6
+    X, U, W, _, _, _ = _inputs(K, NT, nt, P, False, 4000 + e)
+    if spread:
+        g = torch.Generator(device=DEV).manual_seed(e + 100)
+        U = U * torch.exp2(19 * torch.rand((K, 1, 1), generator=g, device=DEV) - 11)
+    X = torch.ldexp(X, torch.tensor(e, device=DEV)).contiguous()
+    ctc, nm = kb.prepare_matching(dict(nt=nt, wPCA=W), U), template_energy(U)
+    assert 2.0 ** -30 <= nm.min() and nm.max() <= 2.0 ** 30
+    B = project_scores(X, U, W, nt, tiled=True)
+    (C, L), cap, th = X.shape, 60000, 2.0 ** e
+    Bs, Xs = B.clone(), X.clone()
+    st = torch.zeros((cap, 2), dtype=torch.int64, device=DEV)
+    amps, tha = torch.zeros((cap, 1), device=DEV), torch.zeros((cap, 1), device=DEV)
+    info = torch.zeros(4, dtype=torch.int64, device=DEV)
+    th2 = min(th * th, 1e38)
+    lib = _lib.load()
+    _lib.check(lib.ks_peel_static(Bs.data_ptr(), Xs.data_ptr(), U.data_ptr(), W.data_ptr(),
+                                  transpose_ctc(ctc, nt).data_ptr(), nm.data_ptr(), C, L, K, P, nt,
+                                  th2, 6, cap, st.data_ptr(), amps.data_ptr(), tha.data_ptr(),
+                                  info.data_ptr(), torch.cuda.current_stream().cuda_stream),
+               "ks_peel_static")
+    n, status = int(info[0]), int(info[1])
+    assert status == 0
+    got = peel(B, X, U, W, ctc, nm, th2 ** 0.5, nt, 6, capacity=cap)
+    same = lambda a, b: torch.equal(torch.nan_to_num(a), torch.nan_to_num(b))
+    assert torch.equal(got[0], st[:n]) and same(got[1], amps[:n]) and same(got[2], tha[:n])
+    assert same(B, Bs) and same(X, Xs)
