@@ -8,7 +8,7 @@ over all 20 batches with X resident in HBM (1.85 GB per step, larger than L2).
 Three forms are timed: `run_matching` per batch with the plain-FP32 and with
 the split-BF16 projection, and the batched split form (every batch in one
 captured graph: grouped tensor-core contraction, one cooperative peel launch
-split into autotuned teams, one residual launch).  `value` is channel-samples/s
+split into autotuned teams that also apply the residuals).  `value` is channel-samples/s
 of the batched split form.  `e2e` runs that form from pinned host memory, with
 the host->device copy of X and the device->host copy of the spikes inside the
 timed region, through the pipelined front end (batched.HostPipeline: groups
@@ -259,8 +259,8 @@ def uneven_main(args, dev, rank, world, emit=True):
     """Batched form: every batch of three recordings through ks_match_batches.
 
     A step is one pass over all batches: groups of --group batches (grouped
-    projection, one cooperative peel launch split into autotuned teams, one
-    residual launch each), all captured in one CUDA graph, so a step is one
+    projection, one cooperative peel launch split into autotuned teams, which
+    apply the residuals, each), all captured in one CUDA graph, so a step is one
     graph launch.  The same batches through one run_matching call each are
     timed beside it.  X resident in HBM.
     """
@@ -894,7 +894,7 @@ def main():
 
     # the batched split form: all batches in one captured graph (grouped
     # tensor-core contraction, one cooperative peel launch split into teams,
-    # one residual launch), teams autotuned; inputs resident as above
+    # residuals included), teams autotuned; inputs resident as above
     matcher, teams, groups = None, None, None
     if batched:
         from kilosort_b200.batched import BatchedMatcher, Recording, autotune_schedule
@@ -971,13 +971,14 @@ def main():
     e2e_ms, _ = timed(e2e_batched if matcher is not None else e2e_step, head)
 
     # per-kernel breakdown of one pass through the public run_matching, timed
-    # by events the library records inside the call (ks_trace_stages): energy
-    # + copy, projection, peel kernel, residual kernel; one warm-up pass first
+    # by events the library records inside the call (ks_trace_stages): (empty),
+    # projection with the template set-up, peel kernel, residual kernel; one
+    # warm-up pass first
     lib = _lib.load()
     _lib.check(lib.ks_trace_stages(1), "ks_trace_stages")
     import ctypes
     ms4 = (ctypes.c_float * 4)()
-    stage = {"energy": 0.0, "project": 0.0, "peel": 0.0, "residual": 0.0}
+    stage = {"project": 0.0, "peel": 0.0, "residual": 0.0}
     stage_batches = {k: [] for k in stage}
     kused, nsp_total = 0, 0
     proj_head = "bf16x3" if "bf16x3" in results else "fp32"
@@ -988,7 +989,7 @@ def main():
             _lib.check(lib.ks_trace_read(ms4, 4), "ks_trace_read")
             if pass_ == 0:
                 continue
-            for key, v in zip(stage, ms4):
+            for key, v in zip(stage, list(ms4)[1:]):
                 stage[key] += v
                 stage_batches[key].append(round(v, 3))
             kused += len(torch.unique(st[:, 1]))

@@ -206,20 +206,21 @@ KS_API int ks_peel_static(float* Bt, float* Xres, const float* U, const float* W
  * per call; batch lengths may differ.  Each batch gets exactly the outputs
  * ks_run_matching gives it (st, amps, th_amps, Xres, info), computed in this
  * order on the stream: per recording the template energies and the reordered
- * templates; per batch Xres = X and the temporal projection; the score
- * contraction of every batch (split-BF16: one grouped tensor-core launch;
- * FP32: one launch per batch); one cooperative peel launch whose grid is split
- * into `teams` groups of co-resident blocks, each peeling its share of the
- * batches (longest first) and then applying that batch's residual, with no
- * host round trip.  teams <= 0 picks a default.  With an aux_stream other
- * than stream and groups > 1 the batches (longest first) are split into
- * `groups` consecutive groups: the projections of group g+1 run on
- * aux_stream while group g is peeled on stream (the peel then runs one block
- * per SM, leaving room for the projection kernels); stream waits for
- * aux_stream before returning control of the work to the caller's later
- * launches.  info[1] of a batch that no team reached (after an error) stays
- * -1.  Nothing is copied from host memory and the host is not synchronised,
- * so the call can be captured in a CUDA graph (the descriptors are read at
+ * templates; per batch the temporal projection; the score contraction of every
+ * batch (split-BF16: one grouped tensor-core launch; FP32: one launch per
+ * batch); one cooperative peel launch whose grid is split into `teams` groups
+ * of co-resident blocks, each peeling its share of the batches (longest first)
+ * and then applying that batch's residual, with no host round trip.  teams <=
+ * 0 picks a default.  With an aux_stream other than stream and groups > 1 the
+ * batches (longest first) are split into `groups` consecutive groups: the
+ * projections of group g+1 run on aux_stream while group g is peeled on stream
+ * (the peel then runs one block per SM, beside which a block of the FP32
+ * temporal projection fits, but none of the other projection kernels'); stream
+ * waits for aux_stream before returning control of the work to the caller's
+ * later launches.  info[1] of a batch that no team reached (after an error)
+ * stays -1.  Nothing is copied from host memory and the host is not
+ * synchronised, so the call can be captured in a CUDA graph (the descriptors
+ * are read at
  * call time).  ctcT is the transposed layout (KS_CTC_KJL).  Xres may equal X
  * (in place); otherwise they must not overlap.
  */

@@ -4,8 +4,8 @@ The reference matches one padded batch per ``run_matching`` call
 (kilosort/template_matching.py:79-84, the loop of ``extract``).  Here a whole
 group of batches -- up to 256, of up to 8 recordings (template sets), of any
 lengths -- goes through one grouped tensor-core contraction, one cooperative
-peel launch whose grid is split into teams of co-resident blocks, and one
-residual launch.  Each batch gets exactly what ``run_matching`` returns for it.
+peel launch whose grid is split into teams of co-resident blocks, which also
+apply their batches' residuals.  Each batch gets exactly what ``run_matching`` returns for it.
 
 * ``Recording``      one template set: U, wPCA, ctc (transposed once), Th, nt,
                      max_peels, spike capacity per batch

@@ -246,7 +246,8 @@ struct ReconArgs {
 
 // One warp per (32-column block, 32 channels), two tiles of 16 channels: lanes
 // own columns; the spikes whose window meets the block are a run of the
-// (time, index) order.  Bound by instruction issue: 211 us at C=384, K=600,
+// (time, index) order.  Bound by issue (half of the slots, with few warps) and the
+// shared-memory round trips between: 211 us at C=384, K=600,
 // 25200 spikes, where the form with lanes over channels, each lane touching its
 // own row of X, took 1173 us.
 template <int PP>
@@ -389,9 +390,10 @@ __global__ void __launch_bounds__(256) ks_group_by_template_kernel(const int* __
 // and the four dot products are reduced by one exchange; 32 spikes' dot
 // products are then added over the warps.
 //
-// What bounds it: the window reads, C*nt residual values per spike from L2 (2.4
-// GB at C=384 and 25200 spikes: 434 us).  With H and the waveform in shared
-// memory, one spike at a time between two block barriers, it took 1246 us.
+// What bounds it: instruction issue (70 % of the slots) around the window reads,
+// C*nt residual values per spike (2.9 GB through L2 at C=384 and 25200 spikes, a
+// quarter of its rate): 434 us.  With H and the waveform in shared memory, one
+// spike at a time between two block barriers, it took 1246 us.
 template <int NE, int CW>
 __global__ void __launch_bounds__(kAdjThreads) ks_adjoint_warp_kernel(
     const float* __restrict__ Xres, const long long* __restrict__ st,

@@ -275,8 +275,11 @@ cudaEvent_t pipeline_event(int i) {
 }
 
 // Resident blocks per SM of the peel: alone on the device kTeamBlocksPerSm;
-// pipelined 1, which leaves room on every SM for a block of the projection
-// kernels of the next group.
+// pipelined 1, which leaves room on every SM for a block of the FP32 temporal
+// projection of the next group.  The other projection kernels do not fit beside
+// even one (the split contraction holds 210 KB of shared memory, the split
+// temporal projection and the FP32 contraction's wide tiles 52224 registers) and
+// run before or after it.
 int peel_blocks_per_sm(bool pipelined) { return pipelined ? 1 : kTeamBlocksPerSm; }
 
 }  // namespace

@@ -36,8 +36,9 @@ constexpr int kCtcJ = 16;
 // lag for all of them, j in pairs through packed multiply-adds.  G is symmetric
 // and only its upper triangle is read (row <= column).
 //
-// What bounds it: the FP32 pipe (36 multiply-adds per output at P = 6) next to
-// the 4 K^2 (2nt+1) bytes written: 180 us at K = 600, where one output per
+// What bounds it: shared memory (80 % of its rate: the Gram block once per lag
+// and component pair), then issue; the 4 K^2 (2nt+1) bytes written are a seventh
+// of what DRAM takes in the time: 180 us at K = 600, where one output per
 // thread and two shared-memory reads per multiply-add took 449 us.
 // PT: the components where they are known at compile time (6), else 0.
 template <int PT>

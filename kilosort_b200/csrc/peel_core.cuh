@@ -953,8 +953,9 @@ __device__ __forceinline__ void unit_rows(const PeelArgs& a, const UnitIn* in, u
 // largest t outside that interval, or a group with an nm outside its range
 // (marked by a NaN scale), folds every row's quotient.
 //
-// What bounds it: the L1 and L2 traffic of the unit's rows (about 14 KB) and
-// the instructions around it.  Four columns per lane make one 16-byte access, one
+// What bounds it: latency (a launch of teams uses 37 % of the issue slots, 45 % of
+// L1's rate, 21 % of L2's): the unit's loads (about 14 KB), then the phase's
+// barrier.  Four columns per lane make one 16-byte access, one
 // row index and one scale serve four elements, and the products, differences
 // and scores run two per packed FP32 instruction; the form with one column per
 // lane and a division-free fold of larger state took about three times the

@@ -259,9 +259,9 @@ __device__ __forceinline__ float warp_median(const float (&v)[NJ], int C, float 
 // of the samples in turn: lane l holds the channels l + 32j, the next sample's
 // loads in flight while this one's median is found in registers; the results
 // meet in shared memory as rows of 32 samples per channel.  Bound by issue slots
-// (about 700 instructions per sample of 384 channels, 300 of them the median's
-// counts and ranks): 75 us at C=384, L=60122, where a median re-reading the tile
-// from shared memory three times took 142.  Without kCar 128 channels a block:
+// (63 % used: about 700 instructions per sample of 384 channels, 300 of them the
+// median's counts and ranks) and shared memory (69 %): 75 us at C=384, L=60122, where a
+// median re-reading the tile from shared memory three times took 142.  Without kCar 128 channels a block:
 // with all of them, 128 at a time, a block of C=1000 had an SM to itself (whole
 // filter without whitening 684 us, now 491).
 template <bool kCar, bool kPad, int NJ>

@@ -98,8 +98,9 @@ __host__ __device__ inline int support_width(int C) { return ((C + kXCh - 1) / k
 // +0 and are passed over (callers whose spikes do not come from this basis drop
 // a.sup when it is not finite: its product with a zero loading is NaN).
 //
-// What bounds it: instruction issue (about 5.5 warp instructions per channel
-// row and spike) next to the 8CL bytes of X and Xres (185 MB, 28 us).  The
+// What bounds it: issue (52 % of the slots at 29 % of the warps: about 5.5 warp
+// instructions per channel row and spike) and the shared-memory round trips
+// between, next to the 8CL bytes of X and Xres (185 MB, 28 us).  The
 // form with lanes over channels, which applied every listed spike to an Xres
 // copied from X beforehand, took 493 us + 38 us for the copy on a C=384, K=600
 // batch of 60122 samples; this one takes 159 us without a copy, and the
